@@ -153,14 +153,6 @@ void cache_give(hj_ctx* ctx, bool host, void* p, size_t cap) {
 // Frees the kept blocks (carved ones stay for reuse unless `slabs` is set,
 // which also frees the slabs: only when no bunch or batch holds a block).
 void cache_clear(hj_ctx* ctx, bool slabs) {
-  for (auto it = ctx->wake_sets.begin(); it != ctx->wake_sets.end();) {
-    if (it->second.refs > 0 && !slabs) {
-      ++it;
-      continue;
-    }
-    cache_give(ctx, false, it->second.dev, it->second.cap);
-    it = ctx->wake_sets.erase(it);
-  }
   std::multimap<size_t, void*> keep;
   for (auto& kv : ctx->dev_free) {
     if (ctx->carved.count(kv.second)) keep.insert(kv);
@@ -309,6 +301,7 @@ void fill_result(hj_bunch* b, const double m[4], hj_result* res) {
 cudaError_t set_kernel_attributes(hj_ctx* ctx) {
   cudaError_t e = prepare_track_kernels(ctx->max_smem_optin);
   if (e == cudaSuccess) e = prepare_wake_kernels(ctx->max_smem_optin);
+  if (e == cudaSuccess) e = prepare_scan_kernels(ctx->max_smem_optin);
   return e;
 }
 
@@ -418,7 +411,6 @@ extern "C" void hj_bunch_destroy(hj_bunch* b) {
   cudaStreamSynchronize(b->stream);       // nothing queued still uses the blocks
   cache_give(b->ctx, false, b->arena, b->arena_cap);
   cache_give(b->ctx, true, b->harena, b->harena_cap);
-  if (b->wset) b->wset->refs -= 1;
   cache_give(b->ctx, false, b->tables, b->tables_cap);
   if (b->d_sums) cudaFree(b->d_sums);
   if (b->d_log) cudaFree(b->d_log);
@@ -556,38 +548,25 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
 
   if (b->use_wake) {
     const int B = b->B;
-    b->centers.resize(B);
-    hj_grid g{};
-    hj_ctx::WakeSet* cached = nullptr;
-    std::array<uint64_t, 8> key{};
     if (grid) {
-      std::memcpy(b->centers.data(), grid->centers, sizeof(double) * B);
-      g = *grid;
-    } else {
-      const double kv[7] = {b->sigma_z0_initial, b->w.half_width_sigmas, b->w.wake_factor,
-                            b->w.wake_sqrt, b->w.ctau, b->w.sin_coef, b->w.delta_std};
-      key[0] = (uint64_t)B;
-      std::memcpy(key.data() + 1, kv, sizeof(kv));
-      auto it = ctx->wake_sets.find(key);
-      if (it != ctx->wake_sets.end()) {
-        cached = &it->second;
-        cached->used = ++ctx->wake_clock;
-        b->centers = cached->centers;
-        g.nbins = B;
-        g.edge_first = cached->e0;
-        g.edge_last = cached->eN;
-        g.edge_step = cached->estep;
-      } else {
-        HJ_TRY(hj_make_grid(b->sigma_z0_initial, b->w.half_width_sigmas, B, b->centers.data(),
-                            &g));
-      }
+      b->e0 = grid->edge_first;
+      b->eN = grid->edge_last;
+      b->estep = grid->edge_step;
+      b->c1 = grid->centers[0];
+      b->cB = grid->centers[B - 1];
+      b->uniform = host_uniform_centers(grid->centers, B, &b->J, &b->cstep);
+      if (b->uniform) b->cJ = grid->centers[b->J];
+    } else {                                             // src/evolution.jl:270-274
+      const double w = host_half_width(b->sigma_z0_initial, b->w.half_width_sigmas);
+      b->e0 = -w;
+      b->eN = w;
+      b->estep = b->cstep = host_edge_step(w, B);
+      b->c1 = host_center(w, 0, B);
+      b->cB = host_center(w, B - 1, B);
+      b->J = (B - 1) / 2;
+      b->cJ = host_center(w, b->J, B);
     }
-    b->e0 = g.edge_first;
-    b->eN = g.edge_last;
-    b->estep = g.edge_step;
-    b->inv_e = 1.0 / g.edge_step;                        // src/utils.jl:378
-    b->c1 = b->centers[0];
-    b->cB = b->centers[B - 1];
+    b->inv_e = 1.0 / b->estep;                           // src/utils.jl:378
     if (B >= 2) {
       const double step = (b->cB - b->c1) / (double)(B - 1);  // src/wakefield.jl:41-42
       b->inv_c = 1.0 / step;
@@ -597,75 +576,35 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
       b->hi_idx = (int)(idx1 - 1);
       b->hi_w = u - fl;
     }
-    HJ_TRY(shared_twiddles(ctx, b->P, &b->twP));
-    const size_t wbytes = sizeof(double) * B, fbytes = sizeof(double2) * ((size_t)b->M + 1);
-    void* blk = nullptr;
-    if (cached) {
-      blk = cached->dev;
+    if (b->uniform) {
+      host_wake_powers(b->w, b->cJ, b->cstep, b->J, &b->wake_A.x, &b->wake_tau.x,
+                       reinterpret_cast<double(*)[2]>(b->wake_pw), kScanPowers);
     } else {
-      // W, λ and FFT(W) of this grid in one block of the cache, read-only for
-      // every bunch; kept in wake_sets for the next bunch when the grid was
-      // built here, else private to this bunch
-      size_t cap = 0;
-      HJ_TRY(cache_take(ctx, false, 2 * wbytes + fbytes, &blk, &cap));
-      double* W = (double*)blk;
+      // W, λ and FFT(W) of the caller's centres in one block of the cache
+      HJ_TRY(shared_twiddles(ctx, b->P, &b->twP));
+      const size_t wbytes = sizeof(double) * B, fbytes = sizeof(double2) * ((size_t)b->M + 1);
+      HJ_TRY(cache_take(ctx, false, 2 * wbytes + fbytes, &b->tables, &b->tables_cap));
+      b->W = (double*)b->tables;
+      b->lam = b->W + B;
+      b->Wf = (double2*)((char*)b->tables + 2 * wbytes);
       std::vector<double> hW(B), hl(B);
-      host_wake_tables(b->centers.data(), B, b->w, hW.data(), hl.data());
-      cudaError_t e = cudaMemcpyAsync(W, hW.data(), wbytes, cudaMemcpyHostToDevice, b->stream);
+      host_wake_tables(grid->centers, B, b->w, hW.data(), hl.data());
+      cudaError_t e = cudaMemcpyAsync(b->W, hW.data(), wbytes, cudaMemcpyHostToDevice, b->stream);
       if (e == cudaSuccess)
-        e = cudaMemcpyAsync(W + B, hl.data(), wbytes, cudaMemcpyHostToDevice, b->stream);
+        e = cudaMemcpyAsync(b->lam, hl.data(), wbytes, cudaMemcpyHostToDevice, b->stream);
       void* xg = nullptr;
       hj_status s = HJ_OK;
       if (e == cudaSuccess && b->H >= 4) {
         s = scratch(ctx, sizeof(double2) * (size_t)b->M, &xg);
         if (s == HJ_OK)
-          e = launch_wake_spectrum(W, B, b->P, b->M, b->H, b->logH, b->twP, (double2*)xg,
-                                   (double2*)((char*)blk + 2 * wbytes), b->stream);
+          e = launch_wake_spectrum(b->W, B, b->P, b->M, b->H, b->logH, b->twP, (double2*)xg, b->Wf,
+                                   b->stream);
       }
       cudaError_t e2 = cudaStreamSynchronize(b->stream);   // host vectors, scratch
-      if (s == HJ_OK && (e != cudaSuccess || e2 != cudaSuccess))
-        s = set_err(ctx, HJ_ERR_CUDA, "wake tables: %s",
-                    cudaGetErrorString(e != cudaSuccess ? e : e2));
-      if (s != HJ_OK) {
-        cache_give(ctx, false, blk, cap);
-        return s;
-      }
-      if (!grid) {
-        constexpr size_t kWakeSets = 8;
-        if (ctx->wake_sets.size() >= kWakeSets) {   // the least recently used free set goes
-          auto lru = ctx->wake_sets.end();
-          for (auto it = ctx->wake_sets.begin(); it != ctx->wake_sets.end(); ++it)
-            if (it->second.refs == 0 && (lru == ctx->wake_sets.end() || it->second.used < lru->second.used))
-              lru = it;
-          if (lru != ctx->wake_sets.end()) {
-            cache_give(ctx, false, lru->second.dev, lru->second.cap);
-            ctx->wake_sets.erase(lru);
-          }
-        }
-        if (ctx->wake_sets.size() < kWakeSets) {
-          hj_ctx::WakeSet ws;
-          ws.centers = b->centers;
-          ws.e0 = g.edge_first;
-          ws.eN = g.edge_last;
-          ws.estep = g.edge_step;
-          ws.used = ++ctx->wake_clock;
-          ws.dev = blk;
-          ws.cap = cap;
-          cached = &ctx->wake_sets.insert({key, std::move(ws)}).first->second;
-        }
-      }
-      if (!cached) {
-        b->tables = blk;
-        b->tables_cap = cap;
-      }
+      if (s != HJ_OK) return s;
+      HJ_CUDA(ctx, e);
+      HJ_CUDA(ctx, e2);
     }
-    if (cached) {
-      cached->refs += 1;
-      b->wset = cached;
-    }
-    b->W = (double*)blk;
-    b->lam = b->W + B;
-    b->Wf = (double2*)((char*)blk + 2 * wbytes);
     HJ_CUDA(ctx, cudaMemsetAsync(b->pot, 0, b->zero_bytes, b->stream));   // pot potd hist ovf
   }
 
@@ -739,8 +678,8 @@ extern "C" hj_status hj_bunch_set_draws(hj_bunch* b, const double* d_draws, int6
   return HJ_OK;
 }
 
-// Arguments of the fused pass and of the bins step of bunch b.
-void hj_impl::fill_turn_args(const hj_bunch* b, PassArgs& a, BinsArgs& g) {
+// Arguments of the fused pass of bunch b.
+void hj_impl::fill_pass_args(const hj_bunch* b, PassArgs& a) {
   a = PassArgs{};
   a.z = b->z;
   a.dE = b->dE;
@@ -790,15 +729,53 @@ void hj_impl::fill_turn_args(const hj_bunch* b, PassArgs& a, BinsArgs& g) {
   a.part_sum = b->part_sum;
   a.hist_out = b->hist;
   a.hist_spill = b->hist_spill;
+  a.n_parts = b->nblk;
+  a.pair_offset = b->first_particle / 2;
+  a.defer_q = b->defer_q;
+}
 
-  g = BinsArgs{};
+// Arguments of the bins step on uniform centres.
+void hj_impl::fill_scan_args(const hj_bunch* b, ScanArgs& g) {
+  g = ScanArgs{};
+  g.ts = b->ts;
+  g.part_sum = b->shard ? b->d_sums : b->part_sum;
+  g.nblk = b->shard ? 1 : b->nblk;
+  g.n = b->shard ? b->n_global : b->n;
+  g.use_wake = b->use_wake;
+  g.params = b->p;
+  g.sigma_E0_initial = b->sigma_E0_initial;
+  if (!b->use_wake) return;
+  g.particle_factor = host_particle_factor(g.n, b->w.population);
+  g.B = b->B;
+  g.J = (int)b->J;
+  g.hist = b->hist;
+  g.pot = b->pot;
+  g.potd = b->potd;
+  g.hi_idx = b->hi_idx;
+  g.hi_w = b->hi_w;
+  g.cJ = b->cJ;
+  g.cstep = b->cstep;
+  g.lam_pref = 1.0 / (std::sqrt(kTwoPi) * b->w.delta_std);       // src/utils.jl:58-66
+  g.lam_f = -0.5 / (b->w.delta_std * b->w.delta_std);
+  g.A = b->wake_A;
+  g.tau = b->wake_tau;
+  std::copy(b->wake_pw, b->wake_pw + kScanPowers, g.pw);
+}
+
+cudaError_t hj_impl::launch_bunch_bins(const hj_bunch* b) {
+  if (b->uniform) {
+    ScanArgs g;
+    fill_scan_args(b, g);
+    return launch_scan(g, b->stream);
+  }
+  BinsArgs g{};
   g.ts = b->ts;
   g.part_sum = b->shard ? b->d_sums : b->part_sum;
   g.nblk = b->shard ? 1 : b->nblk;
   g.n = b->shard ? b->n_global : b->n;
   g.params = b->p;
   g.sigma_E0_initial = b->sigma_E0_initial;
-  g.population = b->w.population;
+  g.particle_factor = host_particle_factor(g.n, b->w.population);
   g.use_wake = b->use_wake;
   g.B = b->B;
   g.P = b->P;
@@ -806,7 +783,7 @@ void hj_impl::fill_turn_args(const hj_bunch* b, PassArgs& a, BinsArgs& g) {
   g.H = b->H;
   g.logH = b->logH;
   g.cnt = b->hist;
-  g.cic = b->hist ? b->hist + b->B : nullptr;
+  g.cic = b->hist + b->B;
   g.lam = b->lam;
   g.Wf = b->Wf;
   g.twP = b->twP;
@@ -815,11 +792,7 @@ void hj_impl::fill_turn_args(const hj_bunch* b, PassArgs& a, BinsArgs& g) {
   g.hi_idx = b->hi_idx;
   g.hi_w = b->hi_w;
   g.W = b->W;
-  g.conv_only = 0;
-
-  a.n_parts = b->nblk;
-  a.pair_offset = b->first_particle / 2;
-  a.defer_q = b->defer_q;
+  return launch_bins(g, b->stream);
 }
 
 extern "C" hj_status hj_bunch_advance(hj_bunch* b, int64_t turns) {
@@ -828,8 +801,9 @@ extern "C" hj_status hj_bunch_advance(hj_bunch* b, int64_t turns) {
   HJ_TRY(ctx_ok(ctx));
   if (turns < 0) return set_err(ctx, HJ_ERR_ARG, "turns must be >= 0");
   PassArgs a;
-  BinsArgs g;
-  fill_turn_args(b, a, g);
+  fill_pass_args(b, a);
+  ScanArgs g;
+  if (b->uniform) fill_scan_args(b, g);
 
   for (int64_t t = 0; t < turns; ++t) {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -848,7 +822,7 @@ extern "C" hj_status hj_bunch_advance(hj_bunch* b, int64_t turns) {
     if (b->use_wake)
       HJ_CUDA(ctx, launch_hist_reduce(b->part_cnt, b->part_cic, b->nblk, b->B, b->hist, false,
                                       b->stream, b->hist_spill));
-    HJ_CUDA(ctx, launch_bins(g, b->stream));
+    HJ_CUDA(ctx, b->uniform ? launch_scan(g, b->stream) : launch_bunch_bins(b));
     if (b->profiling) {
       HJ_CUDA(ctx, cudaEventRecord(ev[2], b->stream));
       b->profiled_turns += 1;

@@ -10,7 +10,7 @@
 // A batch holds hj_bunch objects whose particles live in one pool and whose
 // turn state lives in one device array (slot per bunch), so a poll is one
 // copy.  Per turn: k_batch_pass over the chunk table, k_batch_reduce, and
-// k_batch_bins (one 2-CTA cluster per bunch); the kernels read the bunch
+// k_batch_scan (one cluster per bunch); the kernels read the bunch
 // tables and the live counts from device memory and are launched over the
 // batch's capacity, so a captured graph stays valid as bunches come and go.
 // A bunch's chunking depends only on its own size and the batch's chunk size,
@@ -30,7 +30,7 @@ struct hj_batch {
   cudaStream_t stream = nullptr;
   int cfg = 0;
   int64_t chunk = 65536;
-  int max_bunches = 0, max_B = 0, max_H = 0, max_chunks = 0;
+  int max_bunches = 0, max_B = 0, max_chunks = 0;
   // launch widths: the live counts rounded up to a power of two (a captured
   // graph is re-captured only when the live counts outgrow them)
   int grid_chunks = 0, grid_bunches = 0, grid_items = 0;
@@ -45,7 +45,7 @@ struct hj_batch {
   TurnState* d_ts = nullptr;                   // [max_bunches]
   TurnState* h_ts = nullptr;                   // pinned copy for polls
   PassArgs* d_pass = nullptr;
-  BinsArgs* d_bins = nullptr;
+  ScanArgs* d_bins = nullptr;
   BatchChunk* d_chunks = nullptr;
   BatchChunk* d_items = nullptr;               // merge table: groups of a bunch's partial slots
   int32_t* d_counts = nullptr;                 // [0] chunks, [1] bunches, [2] merge items,
@@ -53,7 +53,7 @@ struct hj_batch {
   bool resident = false;                       // the pass: resident blocks on a chunk queue
   int resident_blocks = 0;                     // their number (SMs x blocks per SM)
   PassArgs* h_pass = nullptr;                  // pinned staging
-  BinsArgs* h_bins = nullptr;
+  ScanArgs* h_bins = nullptr;
   BatchChunk* h_chunks = nullptr;
   BatchChunk* h_items = nullptr;
   int32_t* h_counts = nullptr;
@@ -63,7 +63,6 @@ struct hj_batch {
   void* harena = nullptr;
   size_t harena_cap = 0;
   bool dirty = true;
-  int bins_ctas = 2;                           // CTAs per bunch in the bins step
   int graph_turns = 16;
   cudaGraphExec_t graph = nullptr;
   int64_t turns_enqueued = 0;
@@ -89,7 +88,8 @@ hj_status batch_upload(hj_batch* bt) {
   const int nb = (int)bt->members.size();
   for (int k = 0; k < nb; ++k) {
     hj_bunch* b = bt->members[k].b;
-    fill_turn_args(b, bt->h_pass[k], bt->h_bins[k]);
+    fill_pass_args(b, bt->h_pass[k]);
+    fill_scan_args(b, bt->h_bins[k]);
     for (int c = 0; c < b->nblk; ++c) {
       BatchChunk ch;
       ch.first = (int64_t)c * bt->chunk;
@@ -134,7 +134,7 @@ hj_status batch_upload(hj_batch* bt) {
   if (nb > 0) {
     HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_pass, bt->h_pass, sizeof(PassArgs) * nb,
                                  cudaMemcpyHostToDevice, bt->stream));
-    HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_bins, bt->h_bins, sizeof(BinsArgs) * nb,
+    HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_bins, bt->h_bins, sizeof(ScanArgs) * nb,
                                  cudaMemcpyHostToDevice, bt->stream));
   }
   if (nch > 0)
@@ -158,8 +158,8 @@ hj_status batch_launch_turn(hj_batch* bt) {
   if (bt->wake)
     HJ_CUDA(ctx, launch_batch_reduce(bt->d_pass, bt->d_items, bt->d_counts + 2, bt->grid_items,
                                      bt->max_B, bt->stream));
-  HJ_CUDA(ctx, launch_batch_bins(bt->d_bins, bt->d_counts + 1, bt->grid_bunches, bt->max_H,
-                                 bt->bins_ctas, bt->stream));
+  HJ_CUDA(ctx, launch_batch_scan(bt->d_bins, bt->d_counts + 1, bt->grid_bunches, bt->max_B,
+                                 bt->stream));
   return HJ_OK;
 }
 
@@ -222,9 +222,6 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->chunk = chunk;
   bt->max_bunches = max_bunches;
   bt->max_B = max_nbins;
-  const int64_t P = next_pow2(2 * (int64_t)max_nbins);
-  bt->max_H = (int)std::max<int64_t>(P / 4, 4);
-  bt->bins_ctas = batch_bins_ctas(bt->max_H, max_bunches, ctx->num_sms);
   bt->cfg = auto_pass_layout(layout, max_nbins, pool_particles);
   bt->pool_n = (pool_particles + 3) / 4 * 4;
   bt->max_chunks = (int)std::min<int64_t>(bt->pool_n / chunk + max_bunches + 1, INT32_MAX);
@@ -234,7 +231,7 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   Carve c;
   const size_t o_z = c.add<double>((size_t)bt->pool_n), o_e = c.add<double>((size_t)bt->pool_n);
   const size_t o_ts = c.add<TurnState>(nb), o_pass = c.add<PassArgs>(nb);
-  const size_t o_bins = c.add<BinsArgs>(nb), o_ch = c.add<BatchChunk>(nc);
+  const size_t o_bins = c.add<ScanArgs>(nb), o_ch = c.add<BatchChunk>(nc);
   const size_t o_it = c.add<BatchChunk>(nc), o_cnt = c.add<int32_t>(4);
   HJ_TRY(cache_take(ctx, false, c.off, &bt->arena, &bt->arena_cap));
   char* a = (char*)bt->arena;
@@ -242,19 +239,19 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->pool_dE = (double*)(a + o_e);
   bt->d_ts = (TurnState*)(a + o_ts);
   bt->d_pass = (PassArgs*)(a + o_pass);
-  bt->d_bins = (BinsArgs*)(a + o_bins);
+  bt->d_bins = (ScanArgs*)(a + o_bins);
   bt->d_chunks = (BatchChunk*)(a + o_ch);
   bt->d_items = (BatchChunk*)(a + o_it);
   bt->d_counts = (int32_t*)(a + o_cnt);
   Carve h;
   const size_t p_ts = h.add<TurnState>(nb), p_pass = h.add<PassArgs>(nb);
-  const size_t p_bins = h.add<BinsArgs>(nb), p_ch = h.add<BatchChunk>(nc);
+  const size_t p_bins = h.add<ScanArgs>(nb), p_ch = h.add<BatchChunk>(nc);
   const size_t p_it = h.add<BatchChunk>(nc), p_cnt = h.add<int32_t>(3);
   HJ_TRY(cache_take(ctx, true, h.off, &bt->harena, &bt->harena_cap));
   char* q = (char*)bt->harena;
   bt->h_ts = (TurnState*)(q + p_ts);
   bt->h_pass = (PassArgs*)(q + p_pass);
-  bt->h_bins = (BinsArgs*)(q + p_bins);
+  bt->h_bins = (ScanArgs*)(q + p_bins);
   bt->h_chunks = (BatchChunk*)(q + p_ch);
   bt->h_items = (BatchChunk*)(q + p_it);
   bt->h_counts = (int32_t*)(q + p_cnt);

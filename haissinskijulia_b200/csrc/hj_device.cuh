@@ -60,16 +60,18 @@ struct TurnState {
                          // shared-memory window of the kick table)
 };
 
+// sin_phis, cos_phis: of p.phi_s, constant over a run (a turn's update keeps them).
 __host__ __device__ inline TurnScalars make_turn_scalars(double E0, const hj_params& p,
-                                                         double sigma_E0_initial) {
+                                                         double sigma_E0_initial, double sin_phis,
+                                                         double cos_phis) {
   TurnScalars s;
   s.E0 = E0;
   s.gamma0 = E0 / p.mass;
   double b2 = 1.0 - 1.0 / (s.gamma0 * s.gamma0);
   s.beta0 = sqrt(b2 > 0.0 ? b2 : 0.0);
   s.eta0 = p.alpha_c - (1.0 / (s.gamma0 * s.gamma0));
-  s.sin_phis = sin(p.phi_s);
-  s.cos_phis = cos(p.phi_s);
+  s.sin_phis = sin_phis;
+  s.cos_phis = cos_phis;
   s.k = (s.beta0 <= 0.0) ? (1.0 / 0.0) : p.freq_rf * kTwoPi / (s.beta0 * kSpeedLight);
   s.inv_k = 1.0 / s.k;
   double t = E0 / 1e9;
@@ -85,6 +87,43 @@ __host__ __device__ inline TurnScalars make_turn_scalars(double E0, const hj_par
   s.drift_ok = !(s.beta0 <= 0 || E0 == 0 || s.k == 0);
   s._pad = 0;
   return s;
+}
+
+inline TurnScalars make_turn_scalars(double E0, const hj_params& p, double sigma_E0_initial) {
+  return make_turn_scalars(E0, p, sigma_E0_initial, sin(p.phi_s), cos(p.phi_s));
+}
+
+// What a turn's bins step hands to the E0 update.
+struct TurnSums {
+  double sum_z, sum_d, n_in;    // of the pass: Σz, Σ(ΔE - ΔE_start), particles in the bins
+  double sigma_z, current;      // of the wake
+  double sum_kick;              // Σ_i lerp(pot, z_i)
+  bool conv;                    // the bunch took the wake potential
+};
+
+// The end of a turn (one thread): E0 update and the next turn's scalars
+// (src/evolution.jl:401-451, :300-304).
+__device__ __forceinline__ void finish_turn(TurnState* ts, const hj_params& p, int64_t n,
+                                            double sigma_E0_initial, bool use_wake,
+                                            const TurnSums& u) {
+  const double E0 = ts->cur.E0;
+  double mean = 0.0;
+  if (p.update_E0) mean = (u.sum_d - u.sum_kick) / (double)n;
+  ts->pending = 1;
+  ts->pending_mean = mean;
+  ts->last_sigma_z = u.sigma_z;
+  ts->last_current = u.current;
+  ts->last_mean = mean;
+  ts->last_sum_kick = u.sum_kick;
+  ts->last_n_in = u.n_in;
+  ts->last_mean_z = u.sum_z / (double)n;
+  ts->turn = ts->turn + 1;
+  ts->turns_left = ts->turns_left - 1;
+  ts->cur = make_turn_scalars(E0 + mean, p, sigma_E0_initial, ts->cur.sin_phis, ts->cur.cos_phis);
+  // Flag what the turn actually used: a NaN current with no particle in
+  // range never reaches the bunch (src/wakefield.jl:305-311).
+  if (!isfinite(mean) || (use_wake && !isfinite(u.sigma_z)) || (u.conv && !isfinite(u.current)))
+    ts->status |= (1 << HJ_ERR_NONFINITE);
 }
 
 // compute_global_std from single-pass sums (src/utils.jl:593-605).

@@ -76,8 +76,7 @@ extern "C" hj_status hj_bunch_pass(hj_bunch* b) {
   HJ_TRY(ctx_ok(ctx));
   if (!b->shard) return set_err(ctx, HJ_ERR_STATE, "hj_bunch_pass is for shards (use hj_bunch_advance)");
   PassArgs a;
-  BinsArgs g;
-  fill_turn_args(b, a, g);
+  fill_pass_args(b, a);
   HJ_CUDA(ctx, launch_track_pass(a, b->nblk, b->stream));
   HJ_CUDA(ctx, launch_hist_reduce(b->part_cnt, b->part_cic, b->nblk, b->B, b->hist, false,
                                   b->stream, b->hist_spill));
@@ -102,10 +101,7 @@ extern "C" hj_status hj_bunch_bins(hj_bunch* b) {
   hj_ctx* ctx = b->ctx;
   HJ_TRY(ctx_ok(ctx));
   if (!b->shard) return set_err(ctx, HJ_ERR_STATE, "hj_bunch_bins is for shards (use hj_bunch_advance)");
-  PassArgs a;
-  BinsArgs g;
-  fill_turn_args(b, a, g);
-  HJ_CUDA(ctx, launch_bins(g, b->stream));
+  HJ_CUDA(ctx, launch_bunch_bins(b));
   b->turns_done += 1;
   return HJ_OK;
 }

@@ -4,6 +4,7 @@
 // puts it (these tables are constant over a run and computed once).
 #include <cmath>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -77,25 +78,36 @@ bool rounded_ratio(double w, int64_t m, int64_t B, double* out) {
 }
 }  // namespace
 
+namespace hj {
+double host_half_width(double sigma_z0, double half_width_sigmas) {
+  const double w = half_width_sigmas * sigma_z0;             // src/evolution.jl:270
+  return w < 1e-9 ? 1e-6 : w;                                // :272
+}
+
+// Julia's range(-w, w, length=B+1) and its midpoints hold the correctly
+// rounded values of w(2k-B)/B and w(2k+1-B)/B.
+double host_center(double w, int64_t k, int64_t B) {
+  const int64_t m = 2 * k + 1 - B;
+  double c;
+  if (!rounded_ratio(w, m, B, &c)) c = (double)((__float128)w * (__float128)m / (__float128)B);
+  return c;
+}
+
+double host_edge_step(double w, int64_t B) {
+  return (double)(((__float128)w * 2) / (__float128)B);
+}
+}  // namespace hj
+
 extern "C" hj_status hj_make_grid(double sigma_z0, double half_width_sigmas, int64_t nbins,
                                   double* centers, hj_grid* out) {
   if (!centers || !out) return HJ_ERR_ARG;
   if (nbins <= 0) return HJ_ERR_NBINS;
-  double w = half_width_sigmas * sigma_z0;                   // src/evolution.jl:270
-  if (w < 1e-9) w = 1e-6;                                    // :272
-  // Julia's range(-w, w, length=B+1) and its midpoints hold the correctly
-  // rounded values of w(2k-B)/B and w(2k+1-B)/B.
-  const __float128 W = (__float128)w, Bq = (__float128)nbins;
-  for (int64_t k = 0; k < nbins; ++k) {
-    const int64_t m = 2 * k + 1 - nbins;
-    double c;
-    if (!rounded_ratio(w, m, nbins, &c)) c = (double)(W * (__float128)m / Bq);
-    centers[k] = c;
-  }
+  const double w = hj::host_half_width(sigma_z0, half_width_sigmas);
+  for (int64_t k = 0; k < nbins; ++k) centers[k] = hj::host_center(w, k, nbins);
   out->nbins = nbins;
   out->edge_first = -w;
   out->edge_last = w;
-  out->edge_step = (double)((W * 2) / Bq);
+  out->edge_step = hj::host_edge_step(w, nbins);
   out->centers = centers;
   return HJ_OK;
 }
@@ -126,7 +138,52 @@ void host_wake_tables(const double* centers, int64_t B, const hj_wake& w, double
   }
 }
 
-// tw[k] = exp(-2πi k/P) in long double, rounded once.
+void host_wake_powers(const hj_wake& w, double cJ, double step, int64_t J, double A[2],
+                      double tau[2], double (*pw)[2], int npw) {
+  const long double rate = 1.0L / (long double)w.ctau, s = (long double)w.wake_sqrt;
+  // e^{x (1/cτ + i s)}
+  auto put = [&](long double x, double out[2]) {
+    const long double m = expl(x * rate);
+    out[0] = (double)(m * cosl(x * s));
+    out[1] = (double)(m * sinl(x * s));
+  };
+  const long double d = (long double)step;
+  for (int k = 0; k < npw; ++k) put(-d * (long double)(int64_t(1) << k), pw[k]);
+  put(-d * (long double)(J + 1), tau);
+  // F e^{c_J (1/cτ + i s)} (1 - i a): its real part is F e^{c/cτ} (cos + a sin)
+  const long double m = (long double)w.wake_factor * expl((long double)cJ * rate);
+  const long double c = cosl((long double)cJ * s), q = sinl((long double)cJ * s);
+  const long double a = (long double)w.sin_coef;
+  A[0] = (double)(m * (c + a * q));
+  A[1] = (double)(m * (q - a * c));
+}
+
+bool host_uniform_centers(const double* c, int64_t B, int64_t* J, double* step) {
+  const double h = B > 1 ? (c[B - 1] - c[0]) / (double)(B - 1) : 1.0;
+  if (!(h > 0.0) || !std::isfinite(h) || !(c[0] <= 0.0)) return false;
+  const double tol = 4.0 * 0x1p-52 * std::fmax(std::fabs(c[0]), std::fabs(c[B - 1]));
+  int64_t last = 0;
+  for (int64_t k = 0; k < B; ++k) {
+    if (!(std::fabs(c[k] - (c[0] + h * (double)k)) <= tol)) return false;
+    if (k > 0 && !(c[k] > c[k - 1])) return false;
+    if (!(c[k] > 0.0)) last = k;
+  }
+  *J = last;
+  *step = h;
+  return true;
+}
+
+double host_particle_factor(int64_t n, double population) {
+  if (population > 0.0) return population;
+  int pw = -1;                                   // floor(log10 n) by digit count
+  for (int64_t m = n; m > 0; m /= 10) ++pw;
+  if (pw > 10) pw = 10;
+  double den = 1.0;                              // exact powers of ten
+  for (int i = 0; i < std::abs(pw); ++i) den *= 10.0;
+  if (pw < 0) den = 1.0 / den;
+  return (1e11 / den) * (double)n;
+}
+
 // RF kick table of the fused pass: (V sin θm, V cos θm), θm = ϕs - 2π m / M,
 // m = 0..M-1, in extended precision and rounded once.
 // The extended-precision (sin θm, cos θm) of a phase are kept per (ϕs, M):

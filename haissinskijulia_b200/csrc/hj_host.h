@@ -10,6 +10,22 @@ double host_wake_function(double c, const hj_wake& w);
 double host_delta(double x, double sigma);
 void host_wake_tables(const double* centers, int64_t B, const hj_wake& w, double* W,
                       double* lam);
+// The centre w(2k+1-B)/B of bin k, correctly rounded (hj_make_grid).
+double host_center(double w, int64_t k, int64_t B);
+// Half width of the grid of a bunch of initial length sigma_z0 and its edge step.
+double host_half_width(double sigma_z0, double half_width_sigmas);
+double host_edge_step(double w, int64_t B);
+// The wake of uniform centres as a geometric sequence: J = the last bin whose
+// centre is <= 0, W[J-d] = Re(A σ^d) with σ = exp(-step (1/cτ + i s)), and pw[k] =
+// σ^{2^k}, k < npw, tau = σ^{J+1}; complex values as (re, im) pairs, in extended
+// precision and rounded once.
+void host_wake_powers(const hj_wake& w, double cJ, double step, int64_t J, double A[2],
+                      double tau[2], double (*pw)[2], int npw);
+// Whether the B centres are uniform to rounding with a positive step and reach
+// <= 0, i.e. the wake table is that sequence; J and the step when so.
+bool host_uniform_centers(const double* centers, int64_t B, int64_t* J, double* step);
+// Particle factor of the wake current (src/evolution.jl:373-384).
+double host_particle_factor(int64_t n, double population);
 void host_twiddles(int64_t P, double* tw_interleaved);
 void host_rf_table(double V, double phi_s, int64_t M, double* tab_interleaved);
 // Tables of the device's Float64 normals: a 2048-layer ziggurat for the

@@ -98,7 +98,7 @@ struct BatchChunk {
   int32_t part;
 };
 
-// Arguments of the per-turn bins step (single CTA).
+// Arguments of the per-turn bins step by FFT (centres that are not uniform).
 struct BinsArgs {
   TurnState* ts;
   const double* part_sum;
@@ -106,7 +106,7 @@ struct BinsArgs {
   int64_t n;
   hj_params params;
   double sigma_E0_initial;
-  double population;
+  double particle_factor;          // src/evolution.jl:373-384
   int32_t use_wake;
   int32_t B, P, M, H, logH;
   const unsigned long long* cnt;   // [B] bin counts
@@ -125,6 +125,29 @@ struct BinsArgs {
   // standalone convolution (hj_wake_potential): no turn-state update
   int32_t conv_only;
   double conv_current;
+};
+
+// Arguments of the bins step on uniform centres (hj_scan.cu).
+constexpr int kScanPowers = 15;      // σ^{2^k}, k = 0..14 (2^14 = kMaxBins)
+struct ScanArgs {
+  TurnState* ts;
+  const double* part_sum;
+  int32_t nblk;
+  int32_t use_wake;
+  int64_t n;
+  hj_params params;
+  double sigma_E0_initial;
+  double particle_factor;            // src/evolution.jl:373-384
+  int32_t B, J;                      // bins; last bin whose centre is <= 0
+  const unsigned long long* hist;    // [3B+2] counts | cell counts | cell Σw·2^24
+  double* pot;                       // [B]
+  double2* potd;                     // [B+1] kick table for the next pass
+  int32_t hi_idx;                    // as in BinsArgs
+  double hi_w;
+  double cJ, cstep;                  // centre i: cJ + (i - J) cstep
+  double lam_pref, lam_f;            // delta(c) = lam_pref exp(lam_f c²)
+  double2 A, tau;                    // W[J-d] = Re(A σ^d); tau = σ^{J+1}
+  double2 pw[kScanPowers];
 };
 
 // Moments of (z, dE) per block: [Σz, Σz², ΣdE, ΣdE²], optionally after
@@ -216,10 +239,13 @@ cudaError_t launch_wake_spectrum(const double* W, int B, int P, int M, int H, in
                                  const double2* twP, double2* Xg, double2* Wf,
                                  cudaStream_t st);
 cudaError_t launch_bins(const BinsArgs& a, cudaStream_t st);
-int batch_bins_ctas(int max_H, int max_bunches, int num_sms);
-cudaError_t launch_batch_bins(const BinsArgs* d_bunches, const int32_t* d_n_bunches,
-                              int max_bunches, int max_H, int ctas, cudaStream_t st);
 size_t bins_smem_bytes(int H);
+
+// ---- launchers (hj_scan.cu) ----
+cudaError_t prepare_scan_kernels(int max_smem);    // once per device: dynamic smem limits
+cudaError_t launch_scan(const ScanArgs& a, cudaStream_t st);
+cudaError_t launch_batch_scan(const ScanArgs* d_bunches, const int32_t* d_n_bunches,
+                              int max_bunches, int max_B, cudaStream_t st);
 
 // ---- context access for entry points outside hj_api.cu ----
 int ctx_device(const hj_ctx* ctx);

@@ -5,7 +5,6 @@
 #pragma once
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -41,19 +40,6 @@ struct hj_ctx {
   std::unordered_set<void*> carved;
   // twiddle tables of the bins step by FFT length P, shared by all bunches
   std::map<int, double2*> twiddles;
-  // grids and wake tables built from an initial σ_z, by the bit patterns of
-  // (nbins, σ_z0, half width, F, s, cτ, sin coefficient, δ width): bunches
-  // of a scan start from the same particles and share them
-  struct WakeSet {
-    std::vector<double> centers;
-    double e0 = 0, eN = 0, estep = 0;
-    void* dev = nullptr;            // W[B] | λ[B] | FFT(W)[M+1], a block of the cache
-    size_t cap = 0;
-    uint64_t used = 0;
-    int refs = 0;                   // bunches reading the tables (read-only)
-  };
-  std::map<std::array<uint64_t, 8>, WakeSet> wake_sets;
-  uint64_t wake_clock = 0;
   // Bunches and batches alive on this context.  hj_destroy with some alive
   // only marks the context closing; the last of them to be destroyed frees it,
   // so objects may be destroyed in any order (e.g. by a garbage collector).
@@ -77,7 +63,12 @@ struct hj_bunch {
   // u = (cB - c1)/Δc, cell clamp(floor(u), 0, B-2), weight u - floor(u)
   int hi_idx = 0;
   double hi_w = 0;
-  std::vector<double> centers;
+  // uniform centres: the bins step by suffix scan (hj_scan.cu); J, step and the
+  // centre of bin J, else the FFT's tables
+  bool uniform = true;
+  int64_t J = 0;
+  double cJ = 0, cstep = 0;
+  double2 wake_A{}, wake_tau{}, wake_pw[kScanPowers] = {};   // see ScanArgs
   double sigma_E0_initial = 0, sigma_z0_initial = 0;
   uint64_t seed = 0;
   int qe_mode = QE_OFF;
@@ -118,11 +109,9 @@ struct hj_bunch {
   TurnState* h_ts = nullptr;  // pinned
   double* h_rf = nullptr;     // pinned staging of the RF table
   // the buffers above are carved from one device block and one pinned block
-  // of the context's cache; twP is the context's shared table; W, lam and Wf
-  // point into a wake set shared with other bunches (wset) or a private block
-  // (tables); pot, potd, hist and hist_spill are the first zero_bytes of the
+  // of the context's cache; without uniform centres twP is the context's
+  // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, hist and hist_spill are the first zero_bytes of the
   // arena's histogram part
-  hj_ctx::WakeSet* wset = nullptr;
   bool batch_member = false;
   void* tables = nullptr;
   size_t tables_cap = 0;
@@ -233,7 +222,11 @@ hj_status bunch_create_impl(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
                             const hj_grid* grid, uint64_t seed, void* stream, hj_bunch* b,
                             int64_t chunk = 0, int cfg = -1);
 // Arguments of the fused pass and of the bins step of bunch b.
-void fill_turn_args(const hj_bunch* b, PassArgs& a, BinsArgs& g);
+void fill_pass_args(const hj_bunch* b, PassArgs& a);
+void fill_scan_args(const hj_bunch* b, ScanArgs& g);
+// Enqueues the bins step of bunch b: the suffix scan, or the FFT where the
+// centres are not uniform.
+cudaError_t launch_bunch_bins(const hj_bunch* b);
 
 }  // namespace hj_impl
 

@@ -1,5 +1,8 @@
 // hj_wake.cu -- per-turn "bins" step: wake potential by FFT convolution and
-// the E0 update, in one CTA that keeps the FFT working set in shared memory.
+// the E0 update, in one cluster that keeps the FFT working set in shared memory.
+// Bunches whose bin centres are uniform (every grid the library builds) take the
+// suffix scan of hj_scan.cu instead; this file serves centres that are not,
+// and the standalone wake potential of any grid.
 //
 // Reference (MPI branch of apply_wakefield_inplace!, src/wakefield.jl:186-327):
 //   g[i]   = delta(c_i, 0.15) * counts[i] / Σcounts                 :207-221, :238
@@ -302,44 +305,6 @@ __global__ void __launch_bounds__(kBinsThreads)
   for (int k = threadIdx.x; k <= M; k += blockDim.x) Wf[k] = real_spectrum(Xg, k, M, twP);
 }
 
-// Exact 10^p for 0 <= p <= 22.
-__device__ __forceinline__ double pow10_exact(int p) {
-  double d = 1.0;
-  for (int i = 0; i < p; ++i) d *= 10.0;
-  return d;
-}
-
-// Wake current of src/evolution.jl:373-386; floor(log10 N) by digit count.
-__device__ double wake_current(int64_t n, double E0, const hj_params& p, double sigma_z,
-                               double sigma_E0_initial, double population) {
-  const double g0 = E0 / p.mass;
-  const double eta0 = p.alpha_c - (1.0 / (g0 * g0));
-  double pf;
-  if (population > 0.0) {
-    pf = population;
-  } else {
-    int digits = 0;
-    for (int64_t m = n; m > 0; m /= 10) ++digits;
-    int pw = digits - 1;
-    if (pw > 10) pw = 10;
-    if (pw < -10) pw = -10;
-    double den = pw >= 0 ? pow10_exact(pw) : 1.0 / pow10_exact(-pw);
-    pf = (1e11 / den) * (double)n;
-  }
-  return pf / E0 / (kTwoPi * p.radius) * sigma_z / (eta0 * (sigma_E0_initial * sigma_E0_initial));
-}
-
-// compute_global_std from sums, src/utils.jl:593-605.
-__device__ __forceinline__ double global_std(double s, double s2, int64_t n) {
-  if (n <= 1) return 0.0;
-  const double nd = (double)n;
-  const double mean = s / nd;
-  const double var = (s2 / nd) - (mean * mean);
-  double sv = var * nd / (double)(n - 1);
-  if (!(sv > 0.0)) sv = (sv != sv) ? sv : 0.0;
-  return sqrt(sv);
-}
-
 // The bins step as a cluster of C = 2 or 4 CTAs; CTA r owns the spectrum
 // entries k = r (mod C).  Since x[n] = 0 for n >= H = M/2,
 //   X[Cm + r] = FFT_L(y_r)[m],  y_r[n] = Σ_{t<C/2} x[n + tL] w_M^{(n + tL) r},
@@ -390,8 +355,12 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
       const double E0 = ts->cur.E0;
       double sigma_z = 0.0, current = 0.0;
       if (a.use_wake) {
-        sigma_z = global_std(sh[0], sh[1], a.n);                 // src/evolution.jl:357
-        current = wake_current(a.n, E0, a.params, sigma_z, a.sigma_E0_initial, a.population);
+        // src/evolution.jl:357, :373-386
+        const double g0 = E0 / a.params.mass;
+        const double eta0 = a.params.alpha_c - (1.0 / (g0 * g0));
+        sigma_z = global_std_of_sums(sh[0], sh[1], a.n);
+        current = a.particle_factor / E0 / (kTwoPi * a.params.radius) * sigma_z /
+                  (eta0 * (a.sigma_E0_initial * a.sigma_E0_initial));
       }
       sh[4] = current;
       sh[5] = sigma_z;
@@ -586,28 +555,10 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
   if (rank > 0 && threadIdx.x == 0) *cluster.map_shared_rank(&s_peer_sum[rank], 0) = sum_kick;
   cluster.sync();
 
-  // E0 update and next-turn scalars (src/evolution.jl:401-451, :300-304)
   if (rank == 0 && threadIdx.x == 0 && !a.conv_only) {
     for (int r = 1; r < C; ++r) sum_kick += s_peer_sum[r];
-    const double E0 = ts->cur.E0;
-    double mean = 0.0;
-    if (a.params.update_E0) mean = (sh[2] - sum_kick) / (double)a.n;
-    const double E0n = E0 + mean;
-    ts->pending = 1;
-    ts->pending_mean = mean;
-    ts->last_sigma_z = sh[5];
-    ts->last_current = current;
-    ts->last_mean = mean;
-    ts->last_sum_kick = sum_kick;
-    ts->last_n_in = sh[3];
-    ts->last_mean_z = sh[0] / (double)a.n;
-    ts->turn = ts->turn + 1;
-    ts->turns_left = ts->turns_left - 1;
-    ts->cur = make_turn_scalars(E0n, a.params, a.sigma_E0_initial);
-    // Flag what the turn actually used: a NaN current with no particle in
-    // range never reaches the bunch (src/wakefield.jl:305-311).
-    if (!isfinite(mean) || (a.use_wake && !isfinite(sh[5])) || (do_conv && !isfinite(current)))
-      ts->status |= (1 << HJ_ERR_NONFINITE);
+    const TurnSums u{sh[0], sh[2], sh[3], sh[5], current, sum_kick, do_conv};
+    finish_turn(ts, a.params, a.n, a.sigma_E0_initial, a.use_wake != 0, u);
   }
 }
 
@@ -635,40 +586,12 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kBins4Threads, 1) k_
   bins_body<kBins4Threads, kMaxFftH / 4, 8>(a);
 }
 
-// The bins step of a batch: cluster i (CTAs Ci .. Ci + C - 1) runs bunch i;
-// slots past the live count and bunches with no turns left return at once
-// (the CTAs of a cluster read the same state before any writes it, so they agree).
-template <int NT, int MAXH, int MINB, int C = 2>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT, MINB)
-    k_batch_bins(const BinsArgs* __restrict__ bunches, const int32_t* __restrict__ n_bunches) {
-  const int i = (int)(blockIdx.x / C);
-  if (i >= *n_bunches) return;
-  const BinsArgs& a = bunches[i];
-  if (a.ts->turns_left <= 0) return;
-  bins_body<NT, MAXH, C>(a);
-}
-
-// The batched bins step for H <= 2048 (up to 4096 bins): a radix-8 pass of a
-// length-2048 transform has 256 butterflies, so 256 threads per CTA keep every
-// pass busy, and four CTAs share an SM -- a batch of bunches runs in a quarter
-// of the waves of the 1024-thread kernel.
-constexpr int kBatchBinsSmallThreads = 256;
-constexpr int kBatchBinsSmallMaxH = 2048;
-
 }  // namespace
 
 cudaError_t prepare_wake_kernels(int max_smem) {
   cudaError_t e = allow_dynamic_smem((const void*)k_bins, max_smem);
   if (e == cudaSuccess) e = allow_dynamic_smem((const void*)k_bins4, max_smem);
   if (e == cudaSuccess) e = allow_dynamic_smem((const void*)k_bins8, max_smem);
-  if (e == cudaSuccess)
-    e = allow_dynamic_smem((const void*)k_batch_bins<kBinsThreads, kMaxFftH, 1>, max_smem);
-  if (e == cudaSuccess)
-    e = allow_dynamic_smem((const void*)k_batch_bins<kBinsThreads, kMaxFftH / 2, 1, 4>,
-                           max_smem);
-  if (e == cudaSuccess)
-    e = allow_dynamic_smem(
-        (const void*)k_batch_bins<kBatchBinsSmallThreads, kBatchBinsSmallMaxH, 4>, max_smem);
   if (e == cudaSuccess) e = allow_dynamic_smem((const void*)k_wake_spectrum, max_smem);
   return e;
 }
@@ -698,29 +621,6 @@ cudaError_t launch_bins(const BinsArgs& a, cudaStream_t st) {
   }
   PdlConfig l(dim3(2), dim3(kBinsThreads), bins_smem_bytes(a.H), st);
   return cudaLaunchKernelEx(&l.cfg, k_bins, a);
-}
-
-// CTAs per bunch of a batch's bins step, fixed when the batch is created so
-// that a bunch's arithmetic does not depend on which bunches share it: four
-// for large grids when every slot's cluster still fits in one wave, else two.
-int batch_bins_ctas(int max_H, int max_bunches, int num_sms) {
-  return (max_H >= kBins4MinH && 4 * max_bunches <= num_sms) ? 4 : 2;
-}
-
-cudaError_t launch_batch_bins(const BinsArgs* d_bunches, const int32_t* d_n_bunches,
-                              int max_bunches, int max_H, int ctas, cudaStream_t st) {
-  size_t smem = bins_smem_bytes(max_H);
-  const int grid = 2 * (max_bunches > 0 ? max_bunches : 1);
-  if (ctas == 4) {
-    k_batch_bins<kBinsThreads, kMaxFftH / 2, 1, 4>
-        <<<2 * grid, kBinsThreads, bins_smem_bytes(max_H / 2), st>>>(d_bunches, d_n_bunches);
-  } else if (max_H <= kBatchBinsSmallMaxH)
-    k_batch_bins<kBatchBinsSmallThreads, kBatchBinsSmallMaxH, 4>
-        <<<grid, kBatchBinsSmallThreads, smem, st>>>(d_bunches, d_n_bunches);
-  else
-    k_batch_bins<kBinsThreads, kMaxFftH, 1><<<grid, kBinsThreads, smem, st>>>(d_bunches,
-                                                                             d_n_bunches);
-  return cudaGetLastError();
 }
 
 }  // namespace hj
