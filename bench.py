@@ -609,7 +609,7 @@ def run_sharded(args, ctx, cfg, stream, rank, world, local, clocks) -> None:
                          "traffic": None, "algorithmic_bytes": BYTES_PER_PARTICLE_TURN * n,
                          "pass_ms": pass_ms, "max_over_ranks": True},
             "cpu_baseline": None, "e2e": e2e, "replicas": replicas,
-            "gpu_launches": 4 * K * tps, "clocks": clock_info,
+            "gpu_launches": 3 * K * tps, "clocks": clock_info,
             "final": {"sigma_E": res.sigma_E, "sigma_z": res.sigma_z, "E0": res.E0},
         }
         print(json.dumps(line), flush=True)

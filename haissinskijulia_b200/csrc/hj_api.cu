@@ -1,8 +1,8 @@
 // hj_api.cu -- C ABI of the tracking library (include/haissinski_gpu.h).
 //
 // Host orchestration of the device kernels.  A run is a "bunch": its state
-// z/dE stays on the device; per turn the host only enqueues three kernels
-// (particle pass, histogram reduction, bins step) whose turn-to-turn state
+// z/dE stays on the device; per turn the host only enqueues two kernels
+// (particle pass, bins step) whose turn-to-turn state
 // (E0, pending kick, turn counter) lives in device memory, so turns never
 // wait for the host.
 #include <memory>
@@ -493,16 +493,14 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     const bool defer = b->qe_mode == QE_PHILOX && !(b->cfg & kPassFastNormals);
     const size_t o_dq =
         defer ? c.add<int64_t>(nb * (size_t)(pass_cfg_threads(b->cfg) / 32) * kDeferStage) : 0;
-    size_t o[6] = {};
+    size_t o[4] = {};
     if (b->use_wake) {
-      // pot, potd, hist and hist_spill are adjacent: one memset zeroes them
+      // pot, potd, acc and hist are adjacent: one memset zeroes them
       o[0] = c.add<double>(B);                                   // pot
       o[1] = c.add<double2>(B + 1);                              // potd
-      o[2] = c.add<unsigned long long>(3 * B + 2);               // hist
-      o[3] = c.add<unsigned long long>(3 * B + 2);               // hist_spill
+      o[2] = c.add<unsigned long long>(3 * B + 2);               // acc
+      o[3] = c.add<unsigned long long>(B);                       // hist
       b->zero_bytes = c.off - o[0];
-      o[4] = c.add<uint32_t>(nb * B);                            // part_cnt
-      o[5] = c.add<unsigned long long>(nb * (B + 1));            // part_cic
     }
     HJ_TRY(cache_take(ctx, false, c.off, &b->arena, &b->arena_cap));
     char* a = (char*)b->arena;
@@ -514,10 +512,8 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     if (b->use_wake) {
       b->pot = (double*)(a + o[0]);
       b->potd = (double2*)(a + o[1]);
-      b->hist = (unsigned long long*)(a + o[2]);
-      b->hist_spill = (unsigned long long*)(a + o[3]);
-      b->part_cnt = (uint32_t*)(a + o[4]);
-      b->part_cic = (unsigned long long*)(a + o[5]);
+      b->acc = (unsigned long long*)(a + o[2]);
+      b->hist = (unsigned long long*)(a + o[3]);
     }
     Carve hc;
     const size_t h_mom = hc.add<double>(4 * (size_t)b->nblk_m);
@@ -605,7 +601,7 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
       HJ_CUDA(ctx, e);
       HJ_CUDA(ctx, e2);
     }
-    HJ_CUDA(ctx, cudaMemsetAsync(b->pot, 0, b->zero_bytes, b->stream));   // pot potd hist ovf
+    HJ_CUDA(ctx, cudaMemsetAsync(b->pot, 0, b->zero_bytes, b->stream));   // pot potd acc hist
   }
 
   // RF table, staged in the bunch's pinned block
@@ -724,12 +720,8 @@ void hj_impl::fill_pass_args(const hj_bunch* b, PassArgs& a) {
   a.draws = b->draws;
   a.draws_first_turn = b->draws_first;
   a.draws_turns = b->draws_turns;
-  a.part_cnt = b->part_cnt;
-  a.part_cic = b->part_cic;
   a.part_sum = b->part_sum;
-  a.hist_out = b->hist;
-  a.hist_spill = b->hist_spill;
-  a.n_parts = b->nblk;
+  a.acc = b->acc;
   a.pair_offset = b->first_particle / 2;
   a.defer_q = b->defer_q;
 }
@@ -748,7 +740,9 @@ void hj_impl::fill_scan_args(const hj_bunch* b, ScanArgs& g) {
   g.particle_factor = host_particle_factor(g.n, b->w.population);
   g.B = b->B;
   g.J = (int)b->J;
-  g.hist = b->hist;
+  g.acc = b->acc;
+  g.counts = b->hist;
+  g.clear = b->shard ? 0 : 1;
   g.pot = b->pot;
   g.potd = b->potd;
   g.hi_idx = b->hi_idx;
@@ -760,6 +754,15 @@ void hj_impl::fill_scan_args(const hj_bunch* b, ScanArgs& g) {
   g.A = b->wake_A;
   g.tau = b->wake_tau;
   std::copy(b->wake_pw, b->wake_pw + kScanPowers, g.pw);
+}
+
+cudaError_t hj_impl::launch_bunch_pass(const hj_bunch* b, const PassArgs& a) {
+  if (b->shard) {
+    cudaError_t e = cudaMemsetAsync(b->acc, 0, sizeof(unsigned long long) * (3 * (size_t)b->B + 2),
+                                    b->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_track_pass(a, b->nblk, b->stream);
 }
 
 cudaError_t hj_impl::launch_bunch_bins(const hj_bunch* b) {
@@ -782,8 +785,10 @@ cudaError_t hj_impl::launch_bunch_bins(const hj_bunch* b) {
   g.M = b->M;
   g.H = b->H;
   g.logH = b->logH;
-  g.cnt = b->hist;
-  g.cic = b->hist + b->B;
+  g.cnt = b->acc;
+  g.acc = b->acc;
+  g.counts = b->hist;
+  g.clear = b->shard ? 0 : 1;
   g.lam = b->lam;
   g.Wf = b->Wf;
   g.twP = b->twP;
@@ -817,16 +822,13 @@ extern "C" hj_status hj_bunch_advance(hj_bunch* b, int64_t turns) {
       b->events_used += 3;
       HJ_CUDA(ctx, cudaEventRecord(ev[0], b->stream));
     }
-    HJ_CUDA(ctx, launch_track_pass(a, b->nblk, b->stream));
+    HJ_CUDA(ctx, launch_bunch_pass(b, a));
     if (b->profiling) HJ_CUDA(ctx, cudaEventRecord(ev[1], b->stream));
-    if (b->use_wake)
-      HJ_CUDA(ctx, launch_hist_reduce(b->part_cnt, b->part_cic, b->nblk, b->B, b->hist, false,
-                                      b->stream, b->hist_spill));
     HJ_CUDA(ctx, b->uniform ? launch_scan(g, b->stream) : launch_bunch_bins(b));
     if (b->profiling) {
       HJ_CUDA(ctx, cudaEventRecord(ev[2], b->stream));
       b->profiled_turns += 1;
-      b->profiled_launches += b->use_wake ? 3 : 2;
+      b->profiled_launches += 2;
     }
     if (b->log_every > 0 && (b->turns_done + t + 1) % b->log_every == 0) {
       const int64_t rec = kLogHeader + (b->log_density ? b->B : 0);
@@ -1120,13 +1122,11 @@ extern "C" hj_status hj_normal_tables(double* out, int64_t cap) {
 }
 
 namespace {
-// Device histogram of z on `grid` into dcnt (u64 counts), using scratch after `off` bytes.
+// Device histogram of z on `grid` into dcnt (u64 counts).
 hj_status device_histogram(hj_ctx* ctx, const double* d_z, int64_t n, const hj_grid* grid,
-                           unsigned long long* dcnt, uint32_t* part, int nblk) {
-  const int B = (int)grid->nbins;
-  HJ_CUDA(ctx, launch_histogram_only(d_z, n, B, grid->edge_first, grid->edge_last,
-                                     1.0 / grid->edge_step, part, nblk, ctx->stream));
-  HJ_CUDA(ctx, launch_hist_reduce(part, nullptr, nblk, B, dcnt, true, ctx->stream));
+                           unsigned long long* dcnt, int nblk) {
+  HJ_CUDA(ctx, launch_histogram_only(d_z, n, (int)grid->nbins, grid->edge_first, grid->edge_last,
+                                     1.0 / grid->edge_step, dcnt, nblk, ctx->stream));
   return HJ_OK;
 }
 
@@ -1170,7 +1170,6 @@ hj_status device_conv(hj_ctx* ctx, const hj_grid* grid, const hj_wake* wake, dou
   g.H = H;
   g.logH = logH;
   g.cnt = cb.cnt;
-  g.cic = nullptr;
   g.lam = cb.lam;
   g.Wf = cb.Wf;
   g.twP = cb.twP;
@@ -1187,14 +1186,12 @@ hj_status device_conv(hj_ctx* ctx, const hj_grid* grid, const hj_wake* wake, dou
 
 // Carve the conv buffers (and extra doubles) out of the context scratch.
 hj_status conv_scratch(hj_ctx* ctx, int B, size_t extra_doubles, int extra_arrays,
-                       int64_t part_words, ConvBuffers& cb, double** extra,
-                       uint32_t** part) {
+                       ConvBuffers& cb, double** extra) {
   const int P = (int)next_pow2(2 * (int64_t)B), M = P / 2, H = std::max(M / 2, 1);
   size_t sizes[] = {align_up(sizeof(double) * B),     align_up(sizeof(double) * B),
                     align_up(sizeof(double2) * P),    align_up(sizeof(double2) * (M + 1)),
                     align_up(sizeof(double2) * M),    align_up(sizeof(double2) * H),
-                    align_up(sizeof(double) * B),     align_up(sizeof(uint64_t) * B),
-                    align_up(sizeof(uint32_t) * (size_t)std::max<int64_t>(part_words, 1))};
+                    align_up(sizeof(double) * B),     align_up(sizeof(uint64_t) * B)};
   size_t total = 0;
   for (size_t s : sizes) total += s;
   const size_t ex = align_up(sizeof(double) * std::max<size_t>(extra_doubles, 1));
@@ -1210,7 +1207,6 @@ hj_status conv_scratch(hj_ctx* ctx, int B, size_t extra_doubles, int extra_array
   cb.zE = (double2*)p; p += sizes[5];
   cb.pot = (double*)p; p += sizes[6];
   cb.cnt = (unsigned long long*)p; p += sizes[7];
-  *part = (uint32_t*)p; p += sizes[8];
   for (int i = 0; i < extra_arrays; ++i) {
     extra[i] = (double*)p;
     p += ex;
@@ -1231,11 +1227,10 @@ extern "C" hj_status hj_histogram(hj_ctx* ctx, const double* z, int64_t n, const
   const int nblk = hist_blocks(ctx, n);
   ConvBuffers cb{};
   double* ex[1];
-  uint32_t* part = nullptr;
-  HJ_TRY(conv_scratch(ctx, B, (size_t)n, 1, (int64_t)nblk * B, cb, ex, &part));
+  HJ_TRY(conv_scratch(ctx, B, (size_t)n, 1, cb, ex));
   if (n > 0)
     HJ_CUDA(ctx, cudaMemcpyAsync(ex[0], z, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
-  HJ_TRY(device_histogram(ctx, ex[0], n, grid, cb.cnt, part, nblk));
+  HJ_TRY(device_histogram(ctx, ex[0], n, grid, cb.cnt, nblk));
   HJ_CUDA(ctx, cudaMemcpyAsync(counts, cb.cnt, sizeof(int64_t) * B, cudaMemcpyDeviceToHost, ctx->stream));
   HJ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return HJ_OK;
@@ -1254,8 +1249,7 @@ extern "C" hj_status hj_wake_potential(hj_ctx* ctx, const int64_t* counts, const
   for (int i = 0; i < B; ++i)
     if (counts[i] < 0) return set_err(ctx, HJ_ERR_ARG, "negative bin count");
   ConvBuffers cb{};
-  uint32_t* part = nullptr;
-  HJ_TRY(conv_scratch(ctx, B, 0, 0, 0, cb, nullptr, &part));
+  HJ_TRY(conv_scratch(ctx, B, 0, 0, cb, nullptr));
   HJ_CUDA(ctx, cudaMemcpyAsync(cb.cnt, counts, sizeof(int64_t) * B, cudaMemcpyHostToDevice, ctx->stream));
   HJ_TRY(device_conv(ctx, grid, wake, current, cb));
   HJ_CUDA(ctx, cudaMemcpyAsync(pot, cb.pot, sizeof(double) * B, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1278,13 +1272,12 @@ extern "C" hj_status hj_apply_wakefield(hj_ctx* ctx, const double* z, double* dE
   const int nblk = hist_blocks(ctx, n);
   ConvBuffers cb{};
   double* ex[2];
-  uint32_t* part = nullptr;
-  HJ_TRY(conv_scratch(ctx, B, (size_t)n, 2, (int64_t)nblk * B, cb, ex, &part));
+  HJ_TRY(conv_scratch(ctx, B, (size_t)n, 2, cb, ex));
   if (n > 0) {
     HJ_CUDA(ctx, cudaMemcpyAsync(ex[0], z, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     HJ_CUDA(ctx, cudaMemcpyAsync(ex[1], dE, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   }
-  HJ_TRY(device_histogram(ctx, ex[0], n, grid, cb.cnt, part, nblk));
+  HJ_TRY(device_histogram(ctx, ex[0], n, grid, cb.cnt, nblk));
   HJ_TRY(device_conv(ctx, grid, wake, current, cb));
   if (n > 0) {
     const double c1 = grid->centers[0], cB = grid->centers[B - 1];

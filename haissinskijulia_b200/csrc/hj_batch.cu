@@ -1,6 +1,6 @@
 // hj_batch.cu -- batches of independent bunches (hj_batch_*): one particle
 // pool, one turn-state array, per turn one batched pass over a chunk table,
-// one merge of the chunk partials and one batched bins step; turn blocks
+// and one batched bins step; turn blocks
 // replayed from a CUDA graph.
 #include "hj_ranges.h"
 #include "hj_state.h"
@@ -9,7 +9,7 @@
 //
 // A batch holds hj_bunch objects whose particles live in one pool and whose
 // turn state lives in one device array (slot per bunch), so a poll is one
-// copy.  Per turn: k_batch_pass over the chunk table, k_batch_reduce, and
+// copy.  Per turn: k_batch_pass over the chunk table and
 // k_batch_scan (one cluster per bunch); the kernels read the bunch
 // tables and the live counts from device memory and are launched over the
 // batch's capacity, so a captured graph stays valid as bunches come and go.
@@ -33,7 +33,7 @@ struct hj_batch {
   int max_bunches = 0, max_B = 0, max_chunks = 0;
   // launch widths: the live counts rounded up to a power of two (a captured
   // graph is re-captured only when the live counts outgrow them)
-  int grid_chunks = 0, grid_bunches = 0, grid_items = 0;
+  int grid_chunks = 0, grid_bunches = 0;
   int wake = -1, qe = -1;                      // fixed by the first bunch
   int64_t pool_n = 0;
   double* pool_z = nullptr;
@@ -47,15 +47,13 @@ struct hj_batch {
   PassArgs* d_pass = nullptr;
   ScanArgs* d_bins = nullptr;
   BatchChunk* d_chunks = nullptr;
-  BatchChunk* d_items = nullptr;               // merge table: groups of a bunch's partial slots
-  int32_t* d_counts = nullptr;                 // [0] chunks, [1] bunches, [2] merge items,
-                                               // [3] the resident pass's chunk queue
+  int32_t* d_counts = nullptr;                 // [0] chunks, [1] bunches, [2] the resident
+                                               // pass's chunk queue
   bool resident = false;                       // the pass: resident blocks on a chunk queue
   int resident_blocks = 0;                     // their number (SMs x blocks per SM)
   PassArgs* h_pass = nullptr;                  // pinned staging
   ScanArgs* h_bins = nullptr;
   BatchChunk* h_chunks = nullptr;
-  BatchChunk* h_items = nullptr;
   int32_t* h_counts = nullptr;
   // the buffers above are carved from one device and one pinned cached block
   void* arena = nullptr;
@@ -104,28 +102,11 @@ hj_status batch_upload(hj_batch* bt) {
   // blocks is made of the shortest chunks
   std::stable_sort(bt->h_chunks, bt->h_chunks + nch,
                    [](const BatchChunk& x, const BatchChunk& y) { return x.count > y.count; });
-  // merge table: each bunch's partial slots in groups of kMergeGroup
-  constexpr int kMergeGroup = 4;
-  int nit = 0;
-  for (int k = 0; k < nb; ++k) {
-    const int np = bt->members[k].b->nblk;
-    for (int p0 = 0; p0 < np; p0 += kMergeGroup) {
-      if (nit >= bt->max_chunks) return set_err(ctx, HJ_ERR_STATE, "batch merge table overflow");
-      BatchChunk it;
-      it.first = p0;
-      it.count = std::min(kMergeGroup, np - p0);
-      it.bunch = k;
-      it.part = 0;
-      bt->h_items[nit++] = it;
-    }
-  }
   bt->h_counts[0] = nch;
   bt->h_counts[1] = nb;
-  bt->h_counts[2] = nit;
-  if (nch > bt->grid_chunks || nb > bt->grid_bunches || nit > bt->grid_items) {
+  if (nch > bt->grid_chunks || nb > bt->grid_bunches) {
     bt->grid_chunks = std::max(bt->grid_chunks, (int)std::min<int64_t>(next_pow2(nch), bt->max_chunks));
     bt->grid_bunches = std::max(bt->grid_bunches, (int)std::min<int64_t>(next_pow2(nb), bt->max_bunches));
-    bt->grid_items = std::max(bt->grid_items, (int)std::min<int64_t>(next_pow2(nit), bt->max_chunks));
     if (bt->graph) {
       cudaGraphExecDestroy(bt->graph);
       bt->graph = nullptr;
@@ -140,10 +121,7 @@ hj_status batch_upload(hj_batch* bt) {
   if (nch > 0)
     HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_chunks, bt->h_chunks, sizeof(BatchChunk) * nch,
                                  cudaMemcpyHostToDevice, bt->stream));
-  if (nit > 0)
-    HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_items, bt->h_items, sizeof(BatchChunk) * nit,
-                                 cudaMemcpyHostToDevice, bt->stream));
-  HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_counts, bt->h_counts, sizeof(int32_t) * 3,
+  HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_counts, bt->h_counts, sizeof(int32_t) * 2,
                                cudaMemcpyHostToDevice, bt->stream));
   bt->dirty = false;
   return HJ_OK;
@@ -153,11 +131,8 @@ hj_status batch_launch_turn(hj_batch* bt) {
   hj_ctx* ctx = bt->ctx;
   HJ_CUDA(ctx, launch_batch_pass(bt->d_pass, bt->d_chunks, bt->d_counts, bt->grid_chunks,
                                  bt->max_B, bt->wake, bt->qe, bt->cfg,
-                                 bt->resident ? bt->d_counts + 3 : nullptr, bt->resident_blocks,
+                                 bt->resident ? bt->d_counts + 2 : nullptr, bt->resident_blocks,
                                  bt->stream));
-  if (bt->wake)
-    HJ_CUDA(ctx, launch_batch_reduce(bt->d_pass, bt->d_items, bt->d_counts + 2, bt->grid_items,
-                                     bt->max_B, bt->stream));
   HJ_CUDA(ctx, launch_batch_scan(bt->d_bins, bt->d_counts + 1, bt->grid_bunches, bt->max_B,
                                  bt->stream));
   return HJ_OK;
@@ -232,7 +207,7 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   const size_t o_z = c.add<double>((size_t)bt->pool_n), o_e = c.add<double>((size_t)bt->pool_n);
   const size_t o_ts = c.add<TurnState>(nb), o_pass = c.add<PassArgs>(nb);
   const size_t o_bins = c.add<ScanArgs>(nb), o_ch = c.add<BatchChunk>(nc);
-  const size_t o_it = c.add<BatchChunk>(nc), o_cnt = c.add<int32_t>(4);
+  const size_t o_cnt = c.add<int32_t>(3);
   HJ_TRY(cache_take(ctx, false, c.off, &bt->arena, &bt->arena_cap));
   char* a = (char*)bt->arena;
   bt->pool_z = (double*)(a + o_z);
@@ -241,21 +216,19 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->d_pass = (PassArgs*)(a + o_pass);
   bt->d_bins = (ScanArgs*)(a + o_bins);
   bt->d_chunks = (BatchChunk*)(a + o_ch);
-  bt->d_items = (BatchChunk*)(a + o_it);
   bt->d_counts = (int32_t*)(a + o_cnt);
   Carve h;
   const size_t p_ts = h.add<TurnState>(nb), p_pass = h.add<PassArgs>(nb);
   const size_t p_bins = h.add<ScanArgs>(nb), p_ch = h.add<BatchChunk>(nc);
-  const size_t p_it = h.add<BatchChunk>(nc), p_cnt = h.add<int32_t>(3);
+  const size_t p_cnt = h.add<int32_t>(2);
   HJ_TRY(cache_take(ctx, true, h.off, &bt->harena, &bt->harena_cap));
   char* q = (char*)bt->harena;
   bt->h_ts = (TurnState*)(q + p_ts);
   bt->h_pass = (PassArgs*)(q + p_pass);
   bt->h_bins = (ScanArgs*)(q + p_bins);
   bt->h_chunks = (BatchChunk*)(q + p_ch);
-  bt->h_items = (BatchChunk*)(q + p_it);
   bt->h_counts = (int32_t*)(q + p_cnt);
-  HJ_CUDA(ctx, cudaMemsetAsync(bt->d_counts, 0, sizeof(int32_t) * 4, bt->stream));
+  HJ_CUDA(ctx, cudaMemsetAsync(bt->d_counts, 0, sizeof(int32_t) * 3, bt->stream));
   HJ_CUDA(ctx, cudaMemsetAsync(bt->d_ts, 0, sizeof(TurnState) * max_bunches, bt->stream));
   bt->free_ranges.push_back({0, bt->pool_n});
   for (int s = max_bunches - 1; s >= 0; --s) bt->free_slots.push_back(s);

@@ -7,7 +7,7 @@
 //
 // A bunch split over processes (one GPU each), the reference's MPI mode
 // (src/evolution.jl:206-212 with use_mpi): every rank tracks its particles;
-// once per turn the ranks sum the merged histograms and the pass's sums
+// once per turn the ranks sum the histograms and the pass's sums
 // (exchange buffers, B*3+2 u64 and kNumSums doubles) -- one all-reduce -- and
 // every rank runs the bins step on the totals, so all ranks keep the same
 // potential and E0.  The Philox draws of particle i of a shard are those of
@@ -77,9 +77,7 @@ extern "C" hj_status hj_bunch_pass(hj_bunch* b) {
   if (!b->shard) return set_err(ctx, HJ_ERR_STATE, "hj_bunch_pass is for shards (use hj_bunch_advance)");
   PassArgs a;
   fill_pass_args(b, a);
-  HJ_CUDA(ctx, launch_track_pass(a, b->nblk, b->stream));
-  HJ_CUDA(ctx, launch_hist_reduce(b->part_cnt, b->part_cic, b->nblk, b->B, b->hist, false,
-                                  b->stream, b->hist_spill));
+  HJ_CUDA(ctx, launch_bunch_pass(b, a));
   HJ_CUDA(ctx, launch_sum_parts(b->part_sum, b->nblk, b->d_sums, b->stream));
   return HJ_OK;
 }
@@ -89,7 +87,7 @@ extern "C" hj_status hj_bunch_exchange_buffers(hj_bunch* b, uint64_t** d_counts,
                                                int64_t* n_sums) {
   if (!b || !d_counts || !n_counts || !d_sums || !n_sums) return HJ_ERR_ARG;
   if (!b->shard) return set_err(b->ctx, HJ_ERR_STATE, "not a shard");
-  *d_counts = (uint64_t*)b->hist;
+  *d_counts = (uint64_t*)b->acc;
   *n_counts = 3 * (int64_t)b->B + 2;
   *d_sums = b->d_sums;
   *n_sums = kNumSums;

@@ -73,13 +73,9 @@ struct PassArgs {
   int64_t draws_first_turn;
   int64_t draws_turns;
   // per-block outputs
-  uint32_t* part_cnt;              // [grid][B]
-  unsigned long long* part_cic;    // [grid][B+1] packed cell deposit (count << 44 | Σw·2^24)
   double* part_sum;                // [grid][kNumSums]
-  unsigned long long* hist_out;    // [3B+2] merged histograms, zeroed by the pass
-  unsigned long long* hist_spill;  // [3B+2] deposits outside the hot window and beyond the
-                                   // 16-bit counters (the merged layout), cleared by the merge
-  int32_t n_parts;                 // partial slots written per turn (batches)
+  unsigned long long* acc;         // [3B+2] the turn's counts | cell counts | cell Σw·2^24, which
+                                   // every block adds its own to (zero when the pass starts)
   int64_t pair_offset;             // Philox pair index of particle 0 (shards of a bunch)
   int64_t* defer_q;                // [partial slots][warps][kDeferStage]: indices of the
                                    // particles whose Float64 normal takes the slow path
@@ -110,7 +106,9 @@ struct BinsArgs {
   int32_t use_wake;
   int32_t B, P, M, H, logH;
   const unsigned long long* cnt;   // [B] bin counts
-  const unsigned long long* cic;   // [2(B+1)] cell counts | cell Σw·2^24 (NULL: not needed)
+  unsigned long long* acc;         // [3B+2] counts | cell counts | cell Σw·2^24 (NULL: cnt alone)
+  unsigned long long* counts;      // [B] copy of the turn's counts (with acc)
+  int32_t clear;                   // with acc: leave it zero for the next turn
   const double* lam;               // [B]
   const double2* Wf;               // [M+1]
   const double2* twP;              // [P]
@@ -139,7 +137,9 @@ struct ScanArgs {
   double sigma_E0_initial;
   double particle_factor;            // src/evolution.jl:373-384
   int32_t B, J;                      // bins; last bin whose centre is <= 0
-  const unsigned long long* hist;    // [3B+2] counts | cell counts | cell Σw·2^24
+  unsigned long long* acc;           // [3B+2] counts | cell counts | cell Σw·2^24
+  unsigned long long* counts;        // [B] copy of the turn's counts
+  int32_t clear;                     // leave acc zero for the next turn
   double* pot;                       // [B]
   double2* potd;                     // [B+1] kick table for the next pass
   int32_t hi_idx;                    // as in BinsArgs
@@ -183,8 +183,7 @@ struct PassWindows {
 };
 PassWindows track_windows(int B, int cfg, bool zig);
 cudaError_t launch_track_pass(const PassArgs& a, int grid, cudaStream_t st);
-// Batched pass over a chunk table (*d_n_chunks entries live, grid max_chunks)
-// and the per-bunch merge of its partials.
+// Batched pass over a chunk table (*d_n_chunks entries live, grid max_chunks).
 cudaError_t launch_batch_pass(const PassArgs* d_bunches, const BatchChunk* d_chunks,
                               const int32_t* d_n_chunks, int max_chunks, int max_B, int wake,
                               int qe, int cfg, int32_t* d_queue, int resident_blocks,
@@ -192,14 +191,6 @@ cudaError_t launch_batch_pass(const PassArgs* d_bunches, const BatchChunk* d_chu
 // Blocks of the batched pass that fit on one SM for the batch's largest grid.
 int batch_blocks_per_sm(int max_B, int qe_mode, int use_wake, int cfg);
 cudaError_t launch_sum_parts(const double* part, int nblk, double* out, cudaStream_t st);
-cudaError_t launch_batch_reduce(const PassArgs* d_bunches, const BatchChunk* d_items,
-                                const int32_t* d_n_items, int max_items, int max_B,
-                                cudaStream_t st);
-// out: counts[B] (| cell counts[B+1] | cell Σw·2^24 [B+1] when part_cic != NULL);
-// zero_first clears out before the merge (the fused pass clears it itself).
-cudaError_t launch_hist_reduce(const uint32_t* part_cnt, const unsigned long long* part_cic,
-                               int nblk, int B, unsigned long long* out, bool zero_first,
-                               cudaStream_t st, unsigned long long* spill = nullptr);
 cudaError_t launch_flush(const FlushArgs& a, int grid, cudaStream_t st);
 // generate_particles on the device (covariance sample, correlated bunch, two-pass std)
 cudaError_t launch_gen_sample_cov(uint64_t seed, int64_t S, double mu_z, double sz, double mu_E,
@@ -213,8 +204,9 @@ cudaError_t launch_cor_parts(const double* x, const double* y, int64_t n, double
 cudaError_t launch_log_record(const double* part, int nblk, int64_t n, const TurnState* ts,
                               const unsigned long long* counts, int B, double* rec,
                               cudaStream_t st);
+// Bin counts of z into counts[B] (zeroed first).
 cudaError_t launch_histogram_only(const double* z, int64_t n, int B, double e0, double eN,
-                                  double inv_estep, uint32_t* part_cnt, int grid,
+                                  double inv_estep, unsigned long long* counts, int grid,
                                   cudaStream_t st);
 cudaError_t launch_interp_kick(const double* z, double* dE, int64_t n, const double* pot,
                                int B, double c1, double cB, double inv_cstep,

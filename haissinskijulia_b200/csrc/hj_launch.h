@@ -58,9 +58,8 @@ inline int resolve_pass_request(int r, int automatic) {
 }
 
 // Blocks of the particle pass: enough to fill the GPU, but each block should
-// move at least B/2 particles, since it writes a B-bin partial histogram
-// that the merge reads back (B/2 measured best for 1e5-1e7 particles at 4096
-// and 16384 bins).
+// move at least B/2 particles, since it clears and adds up a window of up to
+// B + 1 counters.
 inline int track_grid_size(int64_t n, int B, int num_sms, int blocks_per_sm, int cfg) {
   int64_t per_block = (int64_t)pass_cfg_ppt(cfg) * pass_cfg_threads(cfg);
   if (per_block < (int64_t)B / 2) per_block = (int64_t)B / 2;

@@ -172,7 +172,6 @@ extern "C" hj_status hj_wake_potential_noalloc(hj_ctx* ctx, const int64_t* d_cou
   g.H = H;
   g.logH = logH;
   g.cnt = reinterpret_cast<const unsigned long long*>(d_counts);
-  g.cic = nullptr;
   g.lam = lam;
   g.Wf = Wf;
   g.twP = twP;

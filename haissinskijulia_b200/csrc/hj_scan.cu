@@ -100,25 +100,29 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
   }
   grid_dependency_wait();
 
-  // 1. this turn's merged counts and cell sums, and the pass's per-block sums in
-  //    block order
+  // 1. this turn's counts and cell sums (the accumulators the pass added to, left
+  //    zero for the next one), and the pass's per-block sums in block order
   unsigned long long cn[E], cw[E];
 #pragma unroll
   for (int k = 0; k < E; ++k) {
     const int i = base + t + k * NT;
     cn[k] = cw[k] = 0ull;
     if (B > 0 && i < nc) {
-      cn[k] = __ldcg(a.hist + B + i);
-      cw[k] = __ldcg(a.hist + B + nc + i);
+      cn[k] = __ldcg(a.acc + B + i);
+      cw[k] = __ldcg(a.acc + B + nc + i);
     }
-    if (B > 0) s_g[t + k * NT] = i < B ? lam[k] * (double)__ldcg(a.hist + i) : 0.0;
+    if (B > 0) {
+      const unsigned long long n = i < B ? __ldcg(a.acc + i) : 0ull;
+      s_g[t + k * NT] = lam[k] * (double)n;
+      if (i < B) a.counts[i] = n;
+    }
   }
   // cell B of a grid that fills the cluster's C L bins: the last CTA's thread 0
   const bool extra = B == C * L && rank == C - 1 && t == 0;
   unsigned long long xn = 0ull, xw = 0ull;
   if (extra) {
-    xn = __ldcg(a.hist + B + B);
-    xw = __ldcg(a.hist + B + nc + B);
+    xn = __ldcg(a.acc + B + B);
+    xw = __ldcg(a.acc + B + nc + B);
   }
   {
     double v[kNumSums] = {0.0, 0.0, 0.0, 0.0};
@@ -159,6 +163,15 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
   }
   double sum_kick = 0.0;
   if (B > 0) {
+    if (a.clear) {
+#pragma unroll
+      for (int k = 0; k < E; ++k) {
+        const int i = base + t + k * NT;
+        if (i < B) a.acc[i] = 0ull;
+        if (i < nc) a.acc[B + i] = a.acc[B + nc + i] = 0ull;
+      }
+      if (extra) a.acc[B + B] = a.acc[B + nc + B] = 0ull;
+    }
     // 2. suffix sums: thread (E bins), warp, CTA
     double g[E];
     double2 v = make_double2(0.0, 0.0);

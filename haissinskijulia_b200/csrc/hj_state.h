@@ -91,16 +91,14 @@ struct hj_bunch {
   double* pot = nullptr;
   double2* potd = nullptr;              // [B+1] kick table (cell j: pot[j-1], step)
   int cfg = 0;                          // thread layout of the fused pass
-  unsigned long long* hist = nullptr;   // counts[B] | cell counts[B+1] | cell Σw·2^24 [B+1]
+  unsigned long long* acc = nullptr;    // counts[B] | cell counts[B+1] | cell Σw·2^24 [B+1]: the
+                                        // turn's deposits, zero between the turns of a whole bunch
+  unsigned long long* hist = nullptr;   // [B] counts of the last completed turn
   double* lam = nullptr;
   double* W = nullptr;
   double2* Wf = nullptr;
   double2* twP = nullptr;
-  uint32_t* part_cnt = nullptr;
   int64_t* defer_q = nullptr;             // [nblk][warps][kDeferStage] (Float64 normals)
-  unsigned long long* part_cic = nullptr;
-  unsigned long long* hist_spill = nullptr;   // [3B+2] the pass's deposits outside its hot
-                                              // window and beyond its 16-bit counters
   double2* rf_table = nullptr;             // [kRfTableSize] RF kick table of the pass
   double rf_Vs = 0;                        // its entry 0: V sin ϕs
   double* part_sum = nullptr;
@@ -110,7 +108,7 @@ struct hj_bunch {
   double* h_rf = nullptr;     // pinned staging of the RF table
   // the buffers above are carved from one device block and one pinned block
   // of the context's cache; without uniform centres twP is the context's
-  // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, hist and hist_spill are the first zero_bytes of the
+  // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, acc and hist are the first zero_bytes of the
   // arena's histogram part
   bool batch_member = false;
   void* tables = nullptr;
@@ -224,6 +222,10 @@ hj_status bunch_create_impl(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
 // Arguments of the fused pass and of the bins step of bunch b.
 void fill_pass_args(const hj_bunch* b, PassArgs& a);
 void fill_scan_args(const hj_bunch* b, ScanArgs& g);
+// Enqueues the particle pass of bunch b with its arguments a.  A shard's
+// accumulators, which its caller may read until the next pass, are cleared here;
+// a whole bunch's by its bins step.
+cudaError_t launch_bunch_pass(const hj_bunch* b, const PassArgs& a);
 // Enqueues the bins step of bunch b: the suffix scan, or the FFT where the
 // centres are not uniform.
 cudaError_t launch_bunch_bins(const hj_bunch* b);

@@ -20,7 +20,8 @@
 // 32-byte load/store per array (ld.global.v4.f64), so a warp touches 1 KB of
 // contiguous HBM per array per iteration; the next quad is loaded while the
 // current one is computed.  Histograms are privatised in shared memory per
-// block and written out as per-block partials, merged by k_hist_reduce.
+// block; at its end every block adds its non-zero counters to the bunch's
+// accumulators in global memory (integers: exact in any order).
 //
 // Per-particle arithmetic of the fused pass (the single-step kernels further
 // down keep the reference's exact operation order instead):
@@ -183,10 +184,9 @@ __device__ __forceinline__ double2 ld_table(const double2* p) {
 //   is bit-identical to its global entry.  Cells B-1 and B (whose step or
 //   value the bins step sets differently) are never hot.
 // * Histograms: bins and cells w0 .. w0 + h - 1 have their per-block
-//   counters in shared memory.  A deposit outside goes to the bunch's spill
-//   histograms in global memory (u64, laid out as the merged ones: counts [B]
-//   | cell counts [B+1] | cell Σw·2^24 [B+1]), which the merge folds in and
-//   clears; h = B + 1 (w0 = 0) where all cells fit.
+//   counters in shared memory.  A deposit outside goes straight to the
+//   bunch's accumulators in global memory (u64: counts [B] | cell counts [B+1]
+//   | cell Σw·2^24 [B+1]); h = B + 1 (w0 = 0) where all cells fit.
 struct PassWindow {
   const double* s_win;
   int w0;
@@ -387,14 +387,14 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
 // is s_ngp[b] (s_ngp[b >> 1]), cell c's words s_lo[c], s_hi[c], for b and c
 // in the window.  An in-range particle's bin is its cell or the one below, so
 // a cell in (w0, w0 + h) puts both in the window: when all K are there the
-// deposits run unchecked, else each is checked and spilled when outside.
+// deposits run unchecked, else each is checked and goes to global memory outside.
 // Without WIN the window holds every cell and nothing is checked.
 template <int K, bool N32, bool WIN>
 __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridConst& g,
                                               const PassWindow& hw, double& acc_z,
                                               double& acc_z2, int32_t& n_in, uint32_t* s_ngp,
                                               uint32_t* s_lo, uint32_t* s_hi,
-                                              unsigned long long* __restrict__ spill) {
+                                              unsigned long long* __restrict__ acc) {
   int nb[K], cj[K];
   bool nin[K];
   uint32_t cq[K];
@@ -438,7 +438,7 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
           if (N32) atomicAdd(&s_ngp[nb[k]], 1u);
           else ong[k] = atomicAdd(&s_ngp[nb[k] >> 1], 1u << ((nb[k] & 1) << 4));
         } else {
-          atomicAdd(spill + nb[k], 1ull);
+          atomicAdd(acc + nb[k], 1ull);
           nin[k] = false;                 // no 16-bit counter to check below
         }
       }
@@ -449,21 +449,21 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
         olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
         atomicAdd(&s_hi[cj[k]], (1u << (kCicSumBits - 32)) + (olo[k] + cq[k] < olo[k] ? 1u : 0u));
       } else {
-        atomicAdd(spill + g.B + cj[k], 1ull);
-        atomicAdd(spill + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
+        atomicAdd(acc + g.B + cj[k], 1ull);
+        atomicAdd(acc + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
       }
     }
   }
   if (!N32) {
     // 16-bit counters, two bins per word: the increment that takes a counter
-    // to 2^15 moves 2^15 counts to the spill counts (the counter has another
+    // to 2^15 moves 2^15 counts to the accumulator (the counter has another
     // 2^15 - 1 increments of room before the move lands)
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int sh = (nb[k] & 1) << 4;
       if (nin[k] && ((ong[k] >> sh) & 0xFFFFu) == 0x7FFFu) {
         atomicSub(&s_ngp[nb[k] >> 1], 0x8000u << sh);
-        atomicAdd(spill + nb[k], 0x8000ull);
+        atomicAdd(acc + nb[k], 0x8000ull);
       }
     }
   }
@@ -554,14 +554,13 @@ __device__ __forceinline__ unsigned group_normals_zig(const PhiloxKeys& rk, int6
 
 // Takes back what deposit_group added for one particle at z: the moments (to
 // rounding) and the NGP and cell deposits (exactly: the packed cell word
-// loses the 2^44 + q it gained, borrow included; the spill histograms, and
-// the spill counts in place of a 16-bit NGP counter, take the negative,
-// modulo 2^64).
+// loses the 2^44 + q it gained, borrow included; the accumulators, also in place
+// of a 16-bit NGP counter, take the negative, modulo 2^64).
 template <bool N32>
 __device__ __forceinline__ void undeposit(double z, const GridConst& g, const PassWindow& hw,
                                           double& acc_z, double& acc_z2, int32_t& n_in,
                                           uint32_t* s_ngp, uint32_t* s_lo, uint32_t* s_hi,
-                                          unsigned long long* __restrict__ spill) {
+                                          unsigned long long* __restrict__ acc) {
   acc_z = __dsub_rn(acc_z, z);
   acc_z2 = fma(-z, z, acc_z2);
   int cj, nb;
@@ -571,15 +570,15 @@ __device__ __forceinline__ void undeposit(double z, const GridConst& g, const Pa
   if (nin) {
     n_in -= 1;
     if (N32 && (uint32_t)(nb - hw.w0) < hw.h) atomicSub(&s_ngp[nb], 1u);
-    else atomicAdd(spill + nb, ~0ull);
+    else atomicAdd(acc + nb, ~0ull);
   }
   const uint32_t cq = min((uint32_t)__double2loint(fma(w, 16777216.0, kMagic)), 16777216u);
   if ((uint32_t)(cj - hw.w0) < hw.h) {
     const uint32_t old = atomicSub(&s_lo[cj], cq);
     atomicSub(&s_hi[cj], (1u << (kCicSumBits - 32)) + (old < cq ? 1u : 0u));
   } else {
-    atomicAdd(spill + g.B + cj, ~0ull);
-    atomicAdd(spill + 2 * g.B + 1 + cj, 0ull - (unsigned long long)cq);
+    atomicAdd(acc + g.B + cj, ~0ull);
+    atomicAdd(acc + 2 * g.B + 1 + cj, 0ull - (unsigned long long)cq);
   }
 }
 
@@ -593,6 +592,31 @@ struct PassRange {
   int32_t part;
   bool tail;
 };
+
+// Adds a block's window counters to the bunch's accumulators.  Each block
+// starts at another cell, so that blocks that end together do not queue at the
+// same addresses: 148 blocks adding 9868 cells took 8.6 us so and 10.6 us in the
+// same order, against 2.4 us for writing them out as per-block partials and
+// 10 us for the kernel that merged those.
+template <int THREADS, bool N32>
+__device__ __forceinline__ void flush_window(const PassArgs& a, const PassWindow& kw, int hot,
+                                             int32_t part, const uint32_t* h_ngp,
+                                             const uint32_t* h_lo, const uint32_t* h_hi) {
+  const int nc = a.B + 1;
+  const int rot = hot > 0 ? (int)(((uint32_t)part * 0x9E3779B9u) >> 8) % hot & ~31 : 0;
+  for (int i = threadIdx.x; i < hot; i += THREADS) {
+    int r = i + rot;
+    if (r >= hot) r -= hot;
+    unsigned long long* p = a.acc + kw.w0 + r;
+    const uint32_t n = N32 ? h_ngp[r] : (h_ngp[r >> 1] >> ((r & 1) << 4)) & 0xFFFFu;
+    const unsigned long long v = ((unsigned long long)h_hi[r] << 32) | h_lo[r];
+    if (n) atomicAdd(p, (unsigned long long)n);       // never at cell B, which has no bin
+    if (v) {
+      atomicAdd(p + a.B, v >> kCicSumBits);
+      atomicAdd(p + a.B + nc, v & kCicSumMask);
+    }
+  }
+}
 
 // Shared-memory tables of the pass: RF table [kRfTableSize] | the ziggurat's
 // (X_i, D_i) rows [kZigLayers].
@@ -635,9 +659,9 @@ __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedCo
   particle_turn<WAKE, true>(z1[0], e1, r, kick, rf, c, pmean, d1);
   acc_d = __dadd_rn(__dsub_rn(acc_d, dg), d1);
   if (WAKE) {
-    undeposit<N32>(zg, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.hist_spill);
+    undeposit<N32>(zg, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
     deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi,
-                               a.hist_spill);
+                               a.acc);
   }
   a.z[i] = z1[0];
   a.dE[i] = e1;
@@ -855,7 +879,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       es[j] = keep ? e0 : ee[j];
     }
     if (WAKE)
-      deposit_group<PPT, N32, WIN>(zz, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.hist_spill);
+      deposit_group<PPT, N32, WIN>(zz, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
     stp<PPT>(a.z + PPT * q, zs);
     stp<PPT>(a.dE + PPT * q, es);
     if (kDefer) {
@@ -888,7 +912,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     particle_turn<WAKE, kDefer>(z1[0], e, r, kick, rf_term<kDefer>(z1[0], c, s_rf), c, pmean,
                                acc_d);
     if (WAKE)
-      deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.hist_spill);
+      deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
     a.z[i] = z1[0];
     a.dE[i] = e;
   }
@@ -900,18 +924,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
                       a.part_sum + (size_t)rg.part * kNumSums,
                       reinterpret_cast<double(*)[4]>(s_rf));
 
-  if (WAKE) {
-    __syncthreads();
-    uint32_t* pc = a.part_cnt + (size_t)rg.part * a.B;
-    unsigned long long* pq = a.part_cic + (size_t)rg.part * nc;
-    for (int i = threadIdx.x; i < nc; i += THREADS) {   // zeros outside the hot window
-      const unsigned r = (unsigned)(i - kw.w0);
-      const bool in = r < kw.h;
-      if (i < a.B)
-        pc[i] = !in ? 0u : N32 ? h_ngp[r] : (h_ngp[r >> 1] >> ((r & 1) << 4)) & 0xFFFFu;
-      pq[i] = in ? ((unsigned long long)h_hi[r] << 32) | h_lo[r] : 0ull;
-    }
-  }
+  if (WAKE) flush_window<THREADS, N32>(a, kw, hot, rg.part, h_ngp, h_lo, h_hi);
 }
 
 // One turn over one bunch: block b takes groups b, b + grid, ... (THREADS
@@ -922,11 +935,6 @@ template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, int MINB = 1, 
 __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dependency_wait();
-  if (WAKE) {  // zero the merged histograms k_hist_reduce accumulates into this turn
-    const int gstride = gridDim.x * THREADS;
-    for (int i = blockIdx.x * THREADS + threadIdx.x; i < 3 * a.B + 2; i += gstride)
-      a.hist_out[i] = 0ull;
-  }
   const PassRange rg{(int64_t)blockIdx.x * THREADS, (int64_t)gridDim.x * THREADS, a.n / PPT,
                      (int32_t)blockIdx.x, blockIdx.x == 0};
   pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
@@ -961,9 +969,6 @@ __global__ void __launch_bounds__(THREADS, MINB)
     const BatchChunk ch = chunks[c];
     const PassArgs a = bunches[ch.bunch];
     if (a.ts->turns_left > 0) {
-      if (WAKE && ch.part == 0) {  // zero the merged histograms k_batch_reduce adds into
-        for (int i = threadIdx.x; i < 3 * a.B + 2; i += THREADS) a.hist_out[i] = 0ull;
-      }
       const PassRange rg{ch.first / PPT, THREADS, (ch.first + ch.count) / PPT, ch.part,
                          ch.first + ch.count == a.n};
       pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
@@ -974,87 +979,6 @@ __global__ void __launch_bounds__(THREADS, MINB)
     __syncthreads();
     c = s_chunk;
   }
-}
-
-// Merge of the per-block histograms.  Grid (bins/256, G): block column g sums
-// the partials of blocks g, g+G, ... and adds them to the merged arrays with
-// integer atomics (exact, so the result does not depend on their order).
-// out layout (u64): counts[B] | cell counts[B+1] | cell Σw·2^24 [B+1].
-// spill (optional): the pass's deposits outside its hot window and beyond its
-// 16-bit counters, in out's layout (counts only without part_cic); folded in
-// and cleared for the next turn.
-__global__ void k_hist_reduce(const uint32_t* __restrict__ part_cnt,
-                              const unsigned long long* __restrict__ part_cic, int nblk, int B,
-                              unsigned long long* __restrict__ out,
-                              unsigned long long* __restrict__ spill) {
-  grid_dependency_wait();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nc = B + 1;
-  if (b >= (part_cic ? nc : B)) return;
-  unsigned long long sc = 0ull, sn = 0ull, sw = 0ull;
-  if (spill && blockIdx.y == 0) {
-    if (b < B) {
-      sc = spill[b];
-      if (sc) spill[b] = 0ull;
-    }
-    if (part_cic) {
-      sn = spill[B + b];
-      sw = spill[B + nc + b];
-      if (sn) spill[B + b] = 0ull;
-      if (sw) spill[B + nc + b] = 0ull;
-    }
-  }
-  for (int k = blockIdx.y; k < nblk; k += gridDim.y) {
-    if (b < B) sc += __ldg(part_cnt + (size_t)k * B + b);
-    if (part_cic) {
-      const unsigned long long v = __ldg(part_cic + (size_t)k * nc + b);
-      sn += v >> kCicSumBits;
-      sw += v & kCicSumMask;
-    }
-  }
-  if (sc) atomicAdd(out + b, sc);
-  if (part_cic) {
-    if (sn) atomicAdd(out + B + b, sn);
-    if (sw) atomicAdd(out + B + nc + b, sw);
-  }
-}
-
-// Merge of a batch's per-chunk histograms: block (x, i) takes item i of the
-// merge table -- partial slots [first, first + count) of one bunch -- sums
-// them for 256 cells and adds the sums to the merged arrays (zeroed by the
-// bunch's first chunk in the pass) with integer atomics: exact, so neither
-// the items' order nor their grouping matters.
-__global__ void k_batch_reduce(const PassArgs* __restrict__ bunches,
-                               const BatchChunk* __restrict__ items,
-                               const int32_t* __restrict__ n_items) {
-  if ((int)blockIdx.y >= *n_items) return;
-  const BatchChunk it = items[blockIdx.y];
-  const PassArgs& a = bunches[it.bunch];
-  if (a.ts->turns_left <= 0 || !a.use_wake) return;
-  const int B = a.B, nc = B + 1;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nc) return;
-  unsigned long long sc = 0ull, sn = 0ull, sw = 0ull;
-  if (it.first == 0) {   // the spill histograms, once per bunch
-    unsigned long long* sp = a.hist_spill;
-    if (b < B) {
-      sc = sp[b];
-      if (sc) sp[b] = 0ull;
-    }
-    sn = sp[B + b];
-    sw = sp[B + nc + b];
-    if (sn) sp[B + b] = 0ull;
-    if (sw) sp[B + nc + b] = 0ull;
-  }
-  for (int64_t k = it.first; k < it.first + it.count; ++k) {
-    if (b < B) sc += __ldg(a.part_cnt + (size_t)k * B + b);
-    const unsigned long long v = __ldg(a.part_cic + (size_t)k * nc + b);
-    sn += v >> kCicSumBits;
-    sw += v & kCicSumMask;
-  }
-  if (sc) atomicAdd(a.hist_out + b, sc);
-  if (sn) atomicAdd(a.hist_out + B + b, sn);
-  if (sw) atomicAdd(a.hist_out + B + nc + b, sw);
 }
 
 // Pending kick + re-centring (optional), copy-out (optional) and the moments
@@ -1112,7 +1036,7 @@ __global__ void k_log_record(const double* __restrict__ part, int nblk, int64_t 
 // NGP histogram only (hj_histogram, hj_apply_wakefield).
 __global__ void __launch_bounds__(kTrackThreads) k_histogram(const double* __restrict__ z,
                                                             int64_t n, GridConst g,
-                                                            uint32_t* __restrict__ part_cnt) {
+                                                            unsigned long long* counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem_raw);
   for (int i = threadIdx.x; i < g.B; i += blockDim.x) s_cnt[i] = 0u;
@@ -1125,7 +1049,7 @@ __global__ void __launch_bounds__(kTrackThreads) k_histogram(const double* __res
   }
   __syncthreads();
   for (int i = threadIdx.x; i < g.B; i += blockDim.x)
-    part_cnt[(size_t)blockIdx.x * g.B + i] = s_cnt[i];
+    if (s_cnt[i]) atomicAdd(counts + i, (unsigned long long)s_cnt[i]);
 }
 
 __global__ void k_interp_kick(const double* __restrict__ z, double* __restrict__ dE, int64_t n,
@@ -1590,31 +1514,6 @@ cudaError_t launch_sum_parts(const double* part, int nblk, double* out, cudaStre
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_reduce(const PassArgs* d_bunches, const BatchChunk* d_items,
-                                const int32_t* d_n_items, int max_items, int max_B,
-                                cudaStream_t st) {
-  dim3 grid((max_B + 1 + 255) / 256, max_items > 0 ? max_items : 1);
-  k_batch_reduce<<<grid, 256, 0, st>>>(d_bunches, d_items, d_n_items);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_hist_reduce(const uint32_t* part_cnt, const unsigned long long* part_cic,
-                               int nblk, int B, unsigned long long* out, bool zero_first,
-                               cudaStream_t st, unsigned long long* spill) {
-  if (zero_first) {
-    cudaError_t e = cudaMemsetAsync(
-        out, 0, sizeof(unsigned long long) * (part_cic ? 3 * (size_t)B + 2 : (size_t)B), st);
-    if (e != cudaSuccess) return e;
-  }
-  const int G = nblk < 16 ? nblk : 16;
-  dim3 grid((B + 1 + 255) / 256, G > 0 ? G : 1);
-  PdlConfig l(grid, dim3(256), 0, st);
-  cudaError_t e = cudaLaunchKernelEx(&l.cfg, k_hist_reduce, part_cnt, part_cic, nblk, B, out,
-                                     spill);
-  if (e != cudaSuccess) return e;
-  return cudaGetLastError();
-}
-
 cudaError_t launch_log_record(const double* part, int nblk, int64_t n, const TurnState* ts,
                               const unsigned long long* counts, int B, double* rec,
                               cudaStream_t st) {
@@ -1654,11 +1553,13 @@ cudaError_t launch_flush(const FlushArgs& a, int grid, cudaStream_t st) {
 }
 
 cudaError_t launch_histogram_only(const double* z, int64_t n, int B, double e0, double eN,
-                                  double inv_estep, uint32_t* part_cnt, int grid,
+                                  double inv_estep, unsigned long long* counts, int grid,
                                   cudaStream_t st) {
   GridConst g{B, e0, eN, inv_estep, 0.0, 0.0, 0.0};
+  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * (size_t)B, st);
+  if (e != cudaSuccess) return e;
   size_t smem = (size_t)B * sizeof(uint32_t);
-  k_histogram<<<grid, kTrackThreads, smem, st>>>(z, n, g, part_cnt);
+  k_histogram<<<grid, kTrackThreads, smem, st>>>(z, n, g, counts);
   return cudaGetLastError();
 }
 

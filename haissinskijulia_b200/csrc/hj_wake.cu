@@ -536,7 +536,7 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
     // src/wakefield.jl:80-102).  With C[j] particles
     // deposited in cell j and S[j] = Σ w·2^24 over them, the same table gives
     //   Σ_i lerp(pot, z_i) = Σ_j C[j] pot_j + 2^-24 Σ_j S[j] step_j.
-    if (a.potd || a.cic) {
+    if (a.acc) {
       const int nc = a.B + 1;
       const int part = (nc + C - 1) / C;
       const int j1 = min(nc, (rank + 1) * part);
@@ -546,8 +546,14 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
           p0 = __dadd_rn(__dmul_rn(a.pot[a.hi_idx], __dsub_rn(1.0, a.hi_w)),
                          __dmul_rn(a.pot[a.hi_idx + 1], a.hi_w));
         const double d = (j > 0 && j < a.B) ? a.pot[j] - p0 : 0.0;
-        if (a.potd) a.potd[j] = make_double2(p0, d);
-        if (a.cic) sum_kick += (double)a.cic[j] * p0 + (double)a.cic[nc + j] * 5.9604644775390625e-08 * d;
+        a.potd[j] = make_double2(p0, d);
+        sum_kick += (double)a.acc[a.B + j] * p0 +
+                    (double)a.acc[a.B + nc + j] * 5.9604644775390625e-08 * d;
+        if (j < a.B) a.counts[j] = a.acc[j];
+        if (a.clear) {
+          if (j < a.B) a.acc[j] = 0ull;
+          a.acc[a.B + j] = a.acc[a.B + nc + j] = 0ull;
+        }
       }
     }
   }
