@@ -496,7 +496,7 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     size_t o[4] = {};
     if (b->use_wake) {
       // pot, potd, acc and hist are adjacent: one memset zeroes them
-      o[0] = c.add<double>(B);                                   // pot
+      o[0] = c.add<double>(B + 2);                               // pot[-1], pot, padding
       o[1] = c.add<double2>(B + 1);                              // potd
       o[2] = c.add<unsigned long long>(3 * B + 2);               // acc
       o[3] = c.add<unsigned long long>(B);                       // hist
@@ -510,7 +510,7 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     b->rf_table = (double2*)(a + o_rf);
     b->defer_q = defer ? (int64_t*)(a + o_dq) : nullptr;
     if (b->use_wake) {
-      b->pot = (double*)(a + o[0]);
+      b->pot = (double*)(a + o[0]) + 1;
       b->potd = (double2*)(a + o[1]);
       b->acc = (unsigned long long*)(a + o[2]);
       b->hist = (unsigned long long*)(a + o[3]);
@@ -601,7 +601,7 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
       HJ_CUDA(ctx, e);
       HJ_CUDA(ctx, e2);
     }
-    HJ_CUDA(ctx, cudaMemsetAsync(b->pot, 0, b->zero_bytes, b->stream));   // pot potd acc hist
+    HJ_CUDA(ctx, cudaMemsetAsync(b->pot - 1, 0, b->zero_bytes, b->stream));   // pot potd acc hist
   }
 
   // RF table, staged in the bunch's pinned block
@@ -682,6 +682,7 @@ void hj_impl::fill_pass_args(const hj_bunch* b, PassArgs& a) {
   a.n = b->n;
   a.ts = b->ts;
   a.potd = b->potd;
+  a.potl = b->pot ? b->pot - 1 : nullptr;
   a.zig = (b->qe_mode == QE_PHILOX && !(b->cfg & kPassFastNormals)) ? 1 : 0;
   if (b->use_wake) {
     const PassWindows w = track_windows(b->B, b->cfg, a.zig != 0);
@@ -738,6 +739,7 @@ void hj_impl::fill_scan_args(const hj_bunch* b, ScanArgs& g) {
   g.sigma_E0_initial = b->sigma_E0_initial;
   if (!b->use_wake) return;
   g.particle_factor = host_particle_factor(g.n, b->w.population);
+  g.n_over_n1 = g.n > 1 ? (double)g.n / (double)(g.n - 1) : 1.0;
   g.B = b->B;
   g.J = (int)b->J;
   g.acc = b->acc;

@@ -101,12 +101,12 @@ struct TurnSums {
   bool conv;                    // the bunch took the wake potential
 };
 
-// The end of a turn (one thread): E0 update and the next turn's scalars
-// (src/evolution.jl:401-451, :300-304).
-__device__ __forceinline__ void finish_turn(TurnState* ts, const hj_params& p, int64_t n,
+// The end of a turn (one thread) whose scalars are `cur`: E0 update and the next
+// turn's scalars (src/evolution.jl:401-451, :300-304).
+__device__ __forceinline__ void finish_turn(TurnState* ts, const TurnScalars& cur,
+                                            const hj_params& p, int64_t n,
                                             double sigma_E0_initial, bool use_wake,
                                             const TurnSums& u) {
-  const double E0 = ts->cur.E0;
   double mean = 0.0;
   if (p.update_E0) mean = (u.sum_d - u.sum_kick) / (double)n;
   ts->pending = 1;
@@ -119,7 +119,7 @@ __device__ __forceinline__ void finish_turn(TurnState* ts, const hj_params& p, i
   ts->last_mean_z = u.sum_z / (double)n;
   ts->turn = ts->turn + 1;
   ts->turns_left = ts->turns_left - 1;
-  ts->cur = make_turn_scalars(E0 + mean, p, sigma_E0_initial, ts->cur.sin_phis, ts->cur.cos_phis);
+  ts->cur = make_turn_scalars(cur.E0 + mean, p, sigma_E0_initial, cur.sin_phis, cur.cos_phis);
   // Flag what the turn actually used: a NaN current with no particle in
   // range never reaches the bunch (src/wakefield.jl:305-311).
   if (!isfinite(mean) || (use_wake && !isfinite(u.sigma_z)) || (u.conv && !isfinite(u.current)))

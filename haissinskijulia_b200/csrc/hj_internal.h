@@ -18,6 +18,13 @@ __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Lets the next kernel on the stream be scheduled as soon as every block of this
+// one has started; what it does before its own grid_dependency_wait() must not
+// touch what this kernel, or one before it, writes.
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 struct PdlConfig {
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
@@ -53,6 +60,8 @@ struct PassArgs {
   int64_t n;
   TurnState* ts;
   const double2* potd;     // [B+1] kick table of the previous turn (cell j: pot[j-1], step)
+  const double* potl;      // [B+1] its left values: pot[0], pot[0], pot[1], ... (16-byte aligned;
+                           // valid while the turn state's `pending` is set)
   int32_t win;             // entries of the kick table's left values held in shared memory
   // bin grid
   int32_t B;
@@ -136,11 +145,12 @@ struct ScanArgs {
   hj_params params;
   double sigma_E0_initial;
   double particle_factor;            // src/evolution.jl:373-384
+  double n_over_n1;                  // n / (n - 1)
   int32_t B, J;                      // bins; last bin whose centre is <= 0
   unsigned long long* acc;           // [3B+2] counts | cell counts | cell Σw·2^24
   unsigned long long* counts;        // [B] copy of the turn's counts
   int32_t clear;                     // leave acc zero for the next turn
-  double* pot;                       // [B]
+  double* pot;                       // [B], and pot[-1] = pot[0]
   double2* potd;                     // [B+1] kick table for the next pass
   int32_t hi_idx;                    // as in BinsArgs
   double hi_w;

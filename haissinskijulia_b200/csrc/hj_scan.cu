@@ -55,12 +55,22 @@ constexpr size_t scan_smem() {
   return sizeof(double2) * (size_t)(NT * E + kPowLo + kPowHi) + sizeof(double) * (size_t)(NT * E + 2);
 }
 
+// All threads of the block, or of the cluster.
+template <int C>
+__device__ __forceinline__ void block_or_cluster_sync() {
+  if constexpr (C > 1) cg::this_cluster().sync();
+  else __syncthreads();
+}
+
+// NT scanning threads and one more warp, which forms the turn's scalars (σ_z, the
+// current, the E0 update) beside the scan.
 template <int C, int NT, int E>
 __device__ __forceinline__ void scan_body(const ScanArgs& a) {
   constexpr int L = NT * E, NW = NT / 32;
-  static_assert(NT >= 256 && NW <= 32 && (L & (L - 1)) == 0 && C * L <= kMaxBins, "layout");
+  static_assert(NT >= 256 && NW <= 31 && (L & (L - 1)) == 0 && C * L <= kMaxBins, "layout");
   constexpr int kLogE = ilog2c(E), kLogL = ilog2c(L);
   const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool scalar = warp == NW;
   int rank = 0;
   if constexpr (C > 1) rank = (int)cg::this_cluster().block_rank();
   extern __shared__ __align__(16) double2 s_dyn[];
@@ -71,17 +81,25 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
   __shared__ double2 s_agg[NW];             // warps' sums
   __shared__ double2 s_cagg;                // the CTA's
   __shared__ double2 s_K[NW][C];            // carries into the CTAs, a copy per warp
-  __shared__ double s_red[NW][4];
-  __shared__ double s_sum[4];               // Σz, Σz², Σ(ΔE - ΔE_start), particles in range
-  __shared__ double s_sc[3];                // potential scale, σ_z, current
-  __shared__ double s_peer[C];
+  __shared__ double s_sc[2];                // potential scale (NaN allowed), particles in range
+  __shared__ double s_kick[C * NW];         // rank 0: Σ kick of every warp of the cluster
   const int B = a.use_wake ? a.B : 0, nc = B + 1;
   const int base = rank * L;
+  TurnState* ts = a.ts;
 
   // before the pass has finished: the powers of σ and the smoothing weights
-  // delta(c_i) (src/utils.jl:58-66) of this thread's bins base + t + k NT
+  // delta(c_i) (src/utils.jl:58-66) of this thread's bins base + t + k NT; the
+  // scalar warp reads the turn's state, which the previous bins step wrote
   double lam[E];
-  if (B > 0) {
+  TurnScalars cur;
+  double coef = 0.0;
+  const double inv_n = 1.0 / (double)a.n;
+  if (scalar) {
+    cur = ts->cur;
+    // the wake current over σ_z (src/evolution.jl:373-386)
+    coef = a.particle_factor / cur.E0 / (kTwoPi * a.params.radius) /
+           (cur.eta0 * (a.sigma_E0_initial * a.sigma_E0_initial));
+  } else if (B > 0) {
     if (t < kPowLo + kPowHi - 1) {
       const int n = t < kPowLo ? t : (t - kPowLo) * kPowLo;
       double2 p = make_double2(1.0, 0.0);
@@ -99,147 +117,151 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
     }
   }
   grid_dependency_wait();
+  grid_launch_dependents();
 
   // 1. this turn's counts and cell sums (the accumulators the pass added to, left
-  //    zero for the next one), and the pass's per-block sums in block order
-  unsigned long long cn[E], cw[E];
-#pragma unroll
-  for (int k = 0; k < E; ++k) {
-    const int i = base + t + k * NT;
-    cn[k] = cw[k] = 0ull;
-    if (B > 0 && i < nc) {
-      cn[k] = __ldcg(a.acc + B + i);
-      cw[k] = __ldcg(a.acc + B + nc + i);
-    }
-    if (B > 0) {
-      const unsigned long long n = i < B ? __ldcg(a.acc + i) : 0ull;
-      s_g[t + k * NT] = lam[k] * (double)n;
-      if (i < B) a.counts[i] = n;
-    }
-  }
+  //    zero for the next one), and the pass's per-block sums in a fixed order
+  unsigned long long cn[E], cw[E], xn = 0ull, xw = 0ull;
   // cell B of a grid that fills the cluster's C L bins: the last CTA's thread 0
-  const bool extra = B == C * L && rank == C - 1 && t == 0;
-  unsigned long long xn = 0ull, xw = 0ull;
-  if (extra) {
-    xn = __ldcg(a.acc + B + B);
-    xw = __ldcg(a.acc + B + nc + B);
-  }
-  {
-    double v[kNumSums] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = t; b < a.nblk; b += NT)
+  const bool extra = B > 0 && B == C * L && rank == C - 1 && t == 0;
+  double sum[kNumSums] = {0.0, 0.0, 0.0, 0.0};   // Σz, Σz², Σ(ΔE - ΔE_start), particles in range
+  double sigma_z = 0.0, current = 0.0;
+  if (scalar) {
+    const double2* part = reinterpret_cast<const double2*>(a.part_sum);
+    constexpr int U = 5;   // a wave of 148 blocks in one round of loads
+    for (int b0 = lane; b0 < a.nblk; b0 += 32 * U) {
+      double2 u[U], w[U];
 #pragma unroll
-      for (int k = 0; k < kNumSums; ++k) v[k] += __ldcg(a.part_sum + (size_t)b * kNumSums + k);
+      for (int q = 0; q < U; ++q) {
+        const int b = b0 + 32 * q;
+        u[q] = b < a.nblk ? __ldcg(part + 2 * (size_t)b) : make_double2(0.0, 0.0);
+        w[q] = b < a.nblk ? __ldcg(part + 2 * (size_t)b + 1) : make_double2(0.0, 0.0);
+      }
 #pragma unroll
-    for (int k = 0; k < kNumSums; ++k)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    if (lane == 0)
-#pragma unroll
-      for (int k = 0; k < kNumSums; ++k) s_red[warp][k] = v[k];
-  }
-  __syncthreads();
-  if (t < kNumSums) {
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) s += s_red[w][t];
-    s_sum[t] = s;
-  }
-  __syncwarp();
-  TurnState* ts = a.ts;
-  if (t == 0) {
-    double sigma_z = 0.0, current = 0.0, scale = 0.0;
-    if (B > 0) {
-      // src/evolution.jl:357, :373-386
-      const double E0 = ts->cur.E0, g0 = E0 / a.params.mass;
-      const double eta0 = a.params.alpha_c - (1.0 / (g0 * g0));
-      sigma_z = global_std_of_sums(s_sum[0], s_sum[1], a.n);
-      current = a.particle_factor / E0 / (kTwoPi * a.params.radius) * sigma_z /
-                (eta0 * (a.sigma_E0_initial * a.sigma_E0_initial));
-      if (s_sum[3] > 0.0) scale = current / s_sum[3];             // src/wakefield.jl:207, :305
+      for (int q = 0; q < U; ++q) {
+        sum[0] += u[q].x;
+        sum[1] += u[q].y;
+        sum[2] += w[q].x;
+        sum[3] += w[q].y;
+      }
     }
-    s_sc[0] = scale;
-    s_sc[1] = sigma_z;
-    s_sc[2] = current;
-  }
-  double sum_kick = 0.0;
-  if (B > 0) {
-    if (a.clear) {
 #pragma unroll
-      for (int k = 0; k < E; ++k) {
-        const int i = base + t + k * NT;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < kNumSums; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    double scale = 0.0;
+    if (B > 0) {
+      // src/utils.jl:593-605, src/evolution.jl:357
+      if (a.n > 1) {
+        const double mean = sum[0] * inv_n;
+        double v = fma(sum[1], inv_n, -(mean * mean)) * a.n_over_n1;
+        if (!(v > 0.0)) v = v != v ? v : 0.0;
+        sigma_z = sqrt(v);
+      }
+      current = coef * sigma_z;
+      if (sum[3] > 0.0) scale = current / sum[3];                // src/wakefield.jl:207, :305
+    }
+    if (lane == 0) {
+      s_sc[0] = scale;
+      s_sc[1] = sum[3];
+    }
+  } else if (B > 0) {
+    unsigned long long n[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      const int i = base + t + k * NT;
+      n[k] = i < B ? __ldcg(a.acc + i) : 0ull;
+      cn[k] = i < nc ? __ldcg(a.acc + B + i) : 0ull;
+      cw[k] = i < nc ? __ldcg(a.acc + B + nc + i) : 0ull;
+    }
+    if (extra) {
+      xn = __ldcg(a.acc + B + B);
+      xw = __ldcg(a.acc + B + nc + B);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) s_g[t + k * NT] = lam[k] * (double)n[k];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      const int i = base + t + k * NT;
+      if (i < B) a.counts[i] = n[k];
+      if (a.clear) {
         if (i < B) a.acc[i] = 0ull;
         if (i < nc) a.acc[B + i] = a.acc[B + nc + i] = 0ull;
       }
-      if (extra) a.acc[B + B] = a.acc[B + nc + B] = 0ull;
     }
-    // 2. suffix sums: thread (E bins), warp, CTA
-    double g[E];
-    double2 v = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int k = E - 1; k >= 0; --k) {
-      g[k] = s_g[t * E + k];
-      v = cfma(v, a.pw[0], make_double2(g[k], 0.0));
-    }
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      const double2 u = shfl_down2(v, 1 << s);
-      if (lane + (1 << s) < 32) v = cfma(u, a.pw[kLogE + s], v);
-    }
-    if (lane == 0) s_agg[warp] = v;
-    double2 x = shfl_down2(v, 1);                     // the warp's sum above this thread
-    if (lane == 31) x = make_double2(0.0, 0.0);
+    if (extra && a.clear) a.acc[B + B] = a.acc[B + nc + B] = 0ull;
+  }
+  if (B > 0) {
     __syncthreads();
-    double2 w = lane < NW ? s_agg[lane] : make_double2(0.0, 0.0);
+    // 2. suffix sums: thread (E bins), warp, CTA
+    double2 v = make_double2(0.0, 0.0);
+    double g[E];
+    if (!scalar) {
 #pragma unroll
-    for (int s = 0; (1 << s) < NW; ++s) {
-      const double2 u = shfl_down2(w, 1 << s);
-      if (lane + (1 << s) < NW) w = cfma(u, a.pw[kLogE + 5 + s], w);
-    }
-    if (t == 0) s_cagg = w;
-    double2 wc = make_double2(__shfl_sync(0xffffffffu, w.x, (warp + 1) & 31),
-                              __shfl_sync(0xffffffffu, w.y, (warp + 1) & 31));
-    if (warp < NW - 1) {
-      const int d = E * (31 - lane);
-      x = cfma(cmul(s_lo[d & (kPowLo - 1)], s_hi[d / kPowLo]), wc, x);
-    }
-#pragma unroll
-    for (int k = E - 1; k >= 0; --k) {
-      x = cfma(x, a.pw[0], make_double2(g[k], 0.0));
-      s_T[t * E + k] = x;
-    }
-    // 3. carries into the CTAs: K_c = T[(c+1) L]
-    const double2* sT[C];
-    sT[0] = s_T;
-    if constexpr (C > 1) {
-      cg::cluster_group cluster = cg::this_cluster();
-      cluster.sync();
-#pragma unroll
-      for (int c = 0; c < C; ++c) sT[c] = cluster.map_shared_rank(s_T, c);
-      if (lane < C) {
-        double2 K = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int c = C - 1; c > 0; --c) {
-          const double2 u = *cluster.map_shared_rank(&s_cagg, c);
-          if (c > lane) K = cfma(K, a.pw[kLogL], u);
-        }
-        s_K[warp][lane] = K;
+      for (int k = E - 1; k >= 0; --k) {
+        g[k] = s_g[t * E + k];
+        v = cfma(v, a.pw[0], make_double2(g[k], 0.0));
       }
-      __syncwarp();
-    } else {
-      __syncthreads();
+#pragma unroll
+      for (int s = 0; s < 5; ++s) {
+        const double2 u = shfl_down2(v, 1 << s);
+        if (lane + (1 << s) < 32) v = cfma(u, a.pw[kLogE + s], v);
+      }
+      if (lane == 0) s_agg[warp] = v;
+    }
+    __syncthreads();
+    if (!scalar) {
+      double2 x = shfl_down2(v, 1);                   // the warp's sum above this thread
+      if (lane == 31) x = make_double2(0.0, 0.0);
+      double2 w = lane < NW ? s_agg[lane] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int s = 0; (1 << s) < NW; ++s) {
+        const double2 u = shfl_down2(w, 1 << s);
+        if (lane + (1 << s) < NW) w = cfma(u, a.pw[kLogE + 5 + s], w);
+      }
+      if (t == 0) s_cagg = w;
+      const double2 wc = make_double2(__shfl_sync(0xffffffffu, w.x, (warp + 1) & 31),
+                                      __shfl_sync(0xffffffffu, w.y, (warp + 1) & 31));
+      if (warp < NW - 1) {
+        const int d = E * (31 - lane);
+        x = cfma(cmul(s_lo[d & (kPowLo - 1)], s_hi[d / kPowLo]), wc, x);
+      }
+#pragma unroll
+      for (int k = E - 1; k >= 0; --k) {
+        x = cfma(x, a.pw[0], make_double2(g[k], 0.0));
+        s_T[t * E + k] = x;
+      }
+    }
+    block_or_cluster_sync<C>();
+    // 3. carries into the CTAs: K_c = T[(c+1) L]
+    if (!scalar) {
+      if constexpr (C > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        if (lane < C) {
+          double2 K = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int c = C - 1; c > 0; --c) {
+            const double2 u = *cluster.map_shared_rank(&s_cagg, c);
+            if (c > lane) K = cfma(K, a.pw[kLogL], u);
+          }
+          s_K[warp][lane] = K;
+        }
+        __syncwarp();
+      }
     }
     auto pw = [&](int n) { return cmul(s_lo[n & (kPowLo - 1)], s_hi[n / kPowLo]); };
     auto T_at = [&](int m) {                          // 0 <= m < B
-      const int c = m >> kLogL, r = m & (L - 1);
-      if constexpr (C == 1) return s_T[r];
-      const double2* p = sT[0];
-#pragma unroll
-      for (int q = 1; q < C; ++q) p = c == q ? sT[q] : p;
-      return cfma(pw(L - r), s_K[warp][c], p[r]);
+      const int r = m & (L - 1);
+      if constexpr (C == 1) {
+        return s_T[r];
+      } else {
+        const int c = m >> kLogL;
+        return cfma(pw(L - r), s_K[warp][c], *cg::this_cluster().map_shared_rank(s_T + r, c));
+      }
     };
-    const double2 T0 = T_at(0);
     const double scale = s_sc[0];
-    const bool conv = s_sum[3] > 0.0;                 // src/wakefield.jl:305-311
+    const bool conv = s_sc[1] > 0.0;                  // src/wakefield.jl:305-311
+    double2 T0;
     auto pot_at = [&](int i) {
       double2 f = i >= a.J ? T_at(i - a.J) : cmul(pw(a.J - i), T0);
       if (i + 1 < B) {
@@ -251,17 +273,20 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
     };
     // 4. the potential at this CTA's bins and the one below them (s_g[1 + r] =
     //    pot[base + r])
-    __syncthreads();                                  // s_g's densities are read
+    if (!scalar) {
+      T0 = T_at(0);
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-      const int i = base + t + k * NT;
-      if (i < B) {
-        const double p = pot_at(i);
-        s_g[1 + t + k * NT] = p;
-        a.pot[i] = p;
+      for (int k = 0; k < E; ++k) {
+        const int i = base + t + k * NT;
+        if (i < B) {
+          const double p = pot_at(i);
+          s_g[1 + t + k * NT] = p;
+          a.pot[i] = p;
+          if (i == 0) a.pot[-1] = p;
+        }
       }
+      if (t == NT - 1 && base > 0 && base - 1 < B) s_g[0] = pot_at(base - 1);
     }
-    if (t == NT - 1 && base > 0 && base - 1 < B) s_g[0] = pot_at(base - 1);
     __syncthreads();
     // 5. kick table of the next pass, B + 1 cells: cell j in 1..B-1 spans centres
     // c[j-1]..c[j] and holds (pot[j-1], pot[j] - pot[j-1]); cells 0 and B are
@@ -271,54 +296,57 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
     // src/wakefield.jl:80-102).  With C[j] particles deposited in cell j and
     // S[j] = Σ w·2^24 over them, the same table gives
     //   Σ_i lerp(pot, z_i) = Σ_j C[j] pot_j + 2^-24 Σ_j S[j] step_j.
-    auto cell = [&](int j, unsigned long long n, unsigned long long sw) {
-      double p0, d = 0.0;
-      if (j < B) {
-        p0 = s_g[j - base + (j > 0 ? 0 : 1)];
-        if (j > 0) d = s_g[j - base + 1] - p0;
-      } else if (B >= 2) {
-        p0 = __dadd_rn(__dmul_rn(pot_at(a.hi_idx), __dsub_rn(1.0, a.hi_w)),
-                       __dmul_rn(pot_at(a.hi_idx + 1), a.hi_w));
-      } else {
-        p0 = pot_at(0);
+    if (!scalar) {
+      double kick = 0.0;
+      auto cell = [&](int j, unsigned long long n, unsigned long long sw) {
+        double p0, d = 0.0;
+        if (j < B) {
+          p0 = s_g[j - base + (j > 0 ? 0 : 1)];
+          if (j > 0) d = s_g[j - base + 1] - p0;
+        } else if (B >= 2) {
+          p0 = __dadd_rn(__dmul_rn(pot_at(a.hi_idx), __dsub_rn(1.0, a.hi_w)),
+                         __dmul_rn(pot_at(a.hi_idx + 1), a.hi_w));
+        } else {
+          p0 = pot_at(0);
+        }
+        a.potd[j] = make_double2(p0, d);
+        kick += (double)n * p0 + (double)sw * 5.9604644775390625e-08 * d;
+      };
+#pragma unroll
+      for (int k = 0; k < E; ++k) {
+        const int j = base + t + k * NT;
+        if (j < nc) cell(j, cn[k], cw[k]);
       }
-      a.potd[j] = make_double2(p0, d);
-      sum_kick += (double)n * p0 + (double)sw * 5.9604644775390625e-08 * d;
-    };
+      if (extra) cell(B, xn, xw);
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-      const int j = base + t + k * NT;
-      if (j < nc) cell(j, cn[k], cw[k]);
+      for (int o = 16; o > 0; o >>= 1) kick += __shfl_down_sync(0xffffffffu, kick, o);
+      if (lane == 0) {
+        double* p = s_kick + rank * NW + warp;
+        if constexpr (C > 1) p = cg::this_cluster().map_shared_rank(p, 0);
+        *p = kick;
+      }
     }
-    if (extra) cell(B, xn, xw);
-    // 6. Σ kick over the block and the cluster
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum_kick += __shfl_down_sync(0xffffffffu, sum_kick, o);
-    if (lane == 0) s_red[warp][0] = sum_kick;
-    __syncthreads();
-    if (warp == 0) {
-      sum_kick = lane < NW ? s_red[lane][0] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum_kick += __shfl_down_sync(0xffffffffu, sum_kick, o);
-    }
-    if constexpr (C > 1) {
-      cg::cluster_group cluster = cg::this_cluster();
-      if (rank > 0 && t == 0) *cluster.map_shared_rank(&s_peer[rank], 0) = sum_kick;
-      cluster.sync();
-    }
+    block_or_cluster_sync<C>();
   }
-  // E0 update and next-turn scalars (src/evolution.jl:401-451, :300-304)
-  if (rank == 0 && t == 0) {
-    if (B > 0)
-      for (int r = 1; r < C; ++r) sum_kick += s_peer[r];
-    const TurnSums u{s_sum[0], s_sum[2], s_sum[3], s_sc[1],
-                     s_sc[2],  sum_kick, B > 0 && s_sum[3] > 0.0};
-    finish_turn(ts, a.params, a.n, a.sigma_E0_initial, B > 0, u);
+  // 6. E0 update and next-turn scalars (src/evolution.jl:401-451, :300-304)
+  if (scalar && rank == 0) {
+    double kick = 0.0;
+    if (B > 0) {
+#pragma unroll
+      for (int q = 0; q < (C * NW + 31) / 32; ++q)
+        if (q * 32 + lane < C * NW) kick += s_kick[q * 32 + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) kick += __shfl_down_sync(0xffffffffu, kick, o);
+    }
+    if (lane == 0) {
+      const TurnSums u{sum[0], sum[2], sum[3], sigma_z, current, kick, B > 0 && sum[3] > 0.0};
+      finish_turn(ts, cur, a.params, a.n, a.sigma_E0_initial, B > 0, u);
+    }
   }
 }
 
 template <int C, int NT, int E>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT, 1) k_scan(ScanArgs a) {
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT + 32, 1) k_scan(ScanArgs a) {
   scan_body<C, NT, E>(a);
 }
 
@@ -326,13 +354,13 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT, 1) k_scan(ScanAr
 // past the live count and bunches with no turns left return at once (the CTAs
 // of a cluster read the same state before any writes it, so they agree).
 template <int C, int NT, int E>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT, 2)
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT + 32, 2)
     k_batch_scan(const ScanArgs* __restrict__ bunches, const int32_t* __restrict__ n_bunches) {
   const int i = (int)(blockIdx.x / C);
   if (i >= *n_bunches) return;
   __shared__ ScanArgs s_a;
   const int* src = reinterpret_cast<const int*>(bunches + i);
-  for (int k = threadIdx.x; k < (int)(sizeof(ScanArgs) / sizeof(int)); k += NT)
+  for (int k = threadIdx.x; k < (int)(sizeof(ScanArgs) / sizeof(int)); k += NT + 32)
     reinterpret_cast<int*>(&s_a)[k] = __ldg(src + k);
   __syncthreads();
   if (__ldcg(&s_a.ts->turns_left) <= 0) return;
@@ -353,11 +381,17 @@ ScanForm batch_form() {
   return {C, NT, E, (const void*)k_batch_scan<C, NT, E>, scan_smem<NT, E>()};
 }
 
+// Up to 1024 bins a CTA alone is faster than a cluster's barriers; above, one
+// bin per thread while 8 CTAs hold them (1e5 particles, us a turn: 2048 bins 15.0 as
+// 8 x 256 x 1 against 15.5 as 2 x 512 x 2 and 15.7 as 1 x 512 x 4; 4096 bins 16.2 as
+// 8 x 512 x 1 against 16.9 as 4 x 512 x 2 and 18.9 as 2 x 512 x 4; 1000 bins 13.6
+// as 1 x 512 x 2 against 14.5 as 4 x 512 x 1; 16384 bins 30.2 as 8 x 512 x 4 against
+// 33.7 as 8 x 256 x 8).
 ScanForm plain_scan_form(int B) {
   if (B <= 512) return plain_form<1, 256, 2>();
   if (B <= 1024) return plain_form<1, 512, 2>();
-  if (B <= 2048) return plain_form<2, 512, 2>();
-  if (B <= 4096) return plain_form<4, 512, 2>();
+  if (B <= 2048) return plain_form<8, 256, 1>();
+  if (B <= 4096) return plain_form<8, 512, 1>();
   if (B <= 8192) return plain_form<8, 512, 2>();
   return plain_form<8, 512, 4>();
 }
@@ -385,7 +419,7 @@ cudaError_t prepare_scan_kernels(int max_smem) {
 cudaError_t launch_scan(const ScanArgs& a, cudaStream_t st) {
   const ScanForm f = plain_scan_form(a.use_wake ? a.B : 0);
   void* args[] = {const_cast<ScanArgs*>(&a)};
-  PdlConfig l(dim3(f.C), dim3(f.NT), f.smem, st);
+  PdlConfig l(dim3(f.C), dim3(f.NT + 32), f.smem, st);
   return cudaLaunchKernelExC(&l.cfg, f.fn, args);
 }
 
@@ -393,8 +427,8 @@ cudaError_t launch_batch_scan(const ScanArgs* d_bunches, const int32_t* d_n_bunc
                               int max_bunches, int max_B, cudaStream_t st) {
   const ScanForm f = batch_scan_form(max_B);
   void* args[] = {const_cast<ScanArgs**>(&d_bunches), const_cast<int32_t**>(&d_n_bunches)};
-  return cudaLaunchKernel(f.fn, dim3(f.C * (max_bunches > 0 ? max_bunches : 1)), dim3(f.NT), args,
-                          f.smem, st);
+  return cudaLaunchKernel(f.fn, dim3(f.C * (max_bunches > 0 ? max_bunches : 1)),
+                          dim3(f.NT + 32), args, f.smem, st);
 }
 
 }  // namespace hj

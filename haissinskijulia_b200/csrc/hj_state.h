@@ -88,7 +88,7 @@ struct hj_bunch {
   int64_t turns_done = 0;
   // device buffers
   TurnState* ts = nullptr;
-  double* pot = nullptr;
+  double* pot = nullptr;                // [B], pot[-1] = pot[0] (16-byte aligned) before it
   double2* potd = nullptr;              // [B+1] kick table (cell j: pot[j-1], step)
   int cfg = 0;                          // thread layout of the fused pass
   unsigned long long* acc = nullptr;    // counts[B] | cell counts[B+1] | cell Σw·2^24 [B+1]: the

@@ -60,7 +60,7 @@ namespace {
 // The normal generator's tables (NormalTables) in global memory, filled once
 // per device when the kernels are prepared; the fused pass stages them into
 // shared memory, the other kernels read them through the cache.
-__device__ NormalTables g_normal;
+__device__ __align__(16) NormalTables g_normal;
 
 __device__ __forceinline__ void philox_normals2(uint64_t seed, int64_t turn, int64_t p,
                                                 double out[2]) {
@@ -167,6 +167,18 @@ __device__ __forceinline__ void kick_cell(double z, const GridConst& g, int& j, 
   j = (t == 0) ? (int)min(lo, (unsigned)g.B) : (t > 0 ? g.B : 0);
 }
 
+// 16 bytes from global to shared memory without a register stage (through L2);
+// both addresses 16-byte aligned.  Complete after copies_wait() and a barrier.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copies_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 __device__ __forceinline__ double2 ld_table(const double2* p) {
   double2 v;
   asm("ld.global.nc.L1::evict_last.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
@@ -175,11 +187,11 @@ __device__ __forceinline__ double2 ld_table(const double2* p) {
 
 // The pass's shared-memory windows, both starting at cell w0 (centred on the
 // cell of the last turn's mean z).
-// * Kick table: s_win[i] = pot_left[w0 + i] (the left value, .x, of table
+// * Kick table: s_win[i] = potl[w0 + i] (the left value, .x, of table
 //   cell w0 + i) for i < lim + 1, where the cells j with w0 <= j < w0 + lim
 //   are "hot": their left value and their right neighbour's left value are
 //   both in the window.  For cells 1..B-2 the step of the global table is
-//   pot[j] - pot[j-1] = pot_left[j+1] - pot_left[j], and for cell 0 it is
+//   pot[j] - pot[j-1] = potl[j+1] - potl[j], and for cell 0 it is
 //   pot[0] - pot[0] = 0, so a hot cell's (left value, step) from the window
 //   is bit-identical to its global entry.  Cells B-1 and B (whose step or
 //   value the bins step sets differently) are never hot.
@@ -720,7 +732,7 @@ template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32 = fal
 __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg,
                                           unsigned char* smem_raw) {
   // dynamic shared memory: RF table [128] | the ziggurat's rows [2048] (a.zig) |
-  // kick-table window [win] | NGP counters | cell words lo, hi [hot] for the
+  // kick-table window [win, rounded up to even] | NGP counters | cell words lo, hi [hot] for the
   // hot window's `hot` bins and cells; NGP counters: (hot+1)/2 words of two
   // 16-bit counters, or hot 32-bit ones (N32)
   const int nc = a.B + 1;                 // kick-table cells
@@ -731,13 +743,24 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   double2* s_zt = s_rf + kRfTableSize;
   double* s_win = reinterpret_cast<double*>(
       smem_raw + (a.zig ? kPassTableBytes : kRfTableSize * sizeof(double2)));
-  uint32_t* const h_ngp = reinterpret_cast<uint32_t*>(s_win + win);
+  uint32_t* const h_ngp = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
   uint32_t* const h_lo = h_ngp + nw;
   uint32_t* const h_hi = h_lo + hot;
-  for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) s_rf[i] = __ldg(a.rf_table + i);
+  // Before the previous turn's bins step has finished: the constant tables and
+  // the zeroed counters (all of the set-up that needs nothing of that step; the
+  // pass of 1e5 particles takes 2 us less for it).
+  for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) copy16_async(s_rf + i, a.rf_table + i);
   if (QE == QE_PHILOX)
     for (int i = threadIdx.x; i < kZigLayers; i += THREADS)
-      s_zt[i] = reinterpret_cast<const double2*>(g_normal.xd)[i];
+      copy16_async(s_zt + i, reinterpret_cast<const double2*>(g_normal.xd) + i);
+  if (WAKE) {
+    const int words = nw + 2 * hot;
+    uint4* const h4 = reinterpret_cast<uint4*>(h_ngp);
+    for (int i = threadIdx.x; i < words / 4; i += THREADS) h4[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < (words & 3)) h_ngp[(words & ~3) + threadIdx.x] = 0u;
+  }
+  grid_dependency_wait();
+  grid_launch_dependents();   // the bins step may be scheduled: it reads the turn state too
 
   TurnState* ts = a.ts;
   const TurnScalars sc = ts->cur;
@@ -777,11 +800,6 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   // wv - 1 (wv <= win, never beyond cell B - 1)
   PassWindow kw{s_win, 0, 0u, 0u, 0u};
   if (WAKE) {
-    for (int i = threadIdx.x; i < hot; i += THREADS) {
-      if (i < nw) h_ngp[i] = 0u;
-      h_lo[i] = 0u;
-      h_hi[i] = 0u;
-    }
     int w0 = 0;
     if (WIN && hot < nc) {   // even, so that the 16-bit pairs keep bin b at word b >> 1
       int jm;
@@ -794,10 +812,16 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     kw.inner = hot > 0 ? (unsigned)hot - 1u : 0u;
     if (win > 0) {
       const int wv = min(win, a.B - w0);
-      for (int i = threadIdx.x; i < wv; i += THREADS) s_win[i] = a.potd[w0 + i].x;
+      if (ts->pending) {   // two entries a copy; the last may take one beyond the window
+        for (int i = 2 * threadIdx.x; i < wv; i += 2 * THREADS)
+          copy16_async(s_win + i, a.potl + w0 + i);
+      } else {
+        for (int i = threadIdx.x; i < wv; i += THREADS) s_win[i] = 0.0;
+      }
       kw.lim = (unsigned)max(wv - 1, 0);
     }
   }
+  copies_wait();
   __syncthreads();
   // the histograms indexed by absolute bin and cell (valid inside the window)
   uint32_t* const s_ngp = h_ngp - (N32 ? kw.w0 : kw.w0 / 2);
@@ -934,7 +958,6 @@ template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, int MINB = 1, 
           bool WIN = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  grid_dependency_wait();
   const PassRange rg{(int64_t)blockIdx.x * THREADS, (int64_t)gridDim.x * THREADS, a.n / PPT,
                      (int32_t)blockIdx.x, blockIdx.x == 0};
   pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
@@ -1400,7 +1423,8 @@ PassWindows track_windows(int B, int cfg, bool zig) {
   const size_t tables = pass_table_bytes(zig), budget = pass_smem_budget(cfg);
   const bool kick = B > kWindowMinBins;
   const size_t per = 8 + ((cfg & kPassN32) ? 4 : 2) + (kick ? 8 : 0);
-  const size_t room = budget > tables + 4 ? budget - tables - 4 : 0;   // 4: an odd 16-bit word
+  // 12: an odd 16-bit word, an even number of kick entries
+  const size_t room = budget > tables + 12 ? budget - tables - 12 : 0;
   const size_t hot = std::min(room / per, (size_t)B + 1);
   PassWindows w;
   w.hot = (int)hot;
@@ -1414,7 +1438,8 @@ size_t track_smem_bytes(int B, int use_wake, int cfg, bool zig) {
   if (!use_wake) return pass_table_bytes(zig);
   const PassWindows w = track_windows(B, cfg, zig);
   const size_t nw = (cfg & kPassN32) ? (size_t)w.hot : (size_t)(w.hot + 1) / 2;
-  return pass_table_bytes(zig) + (size_t)w.kick * sizeof(double) + nw * sizeof(uint32_t) +
+  return pass_table_bytes(zig) + (size_t)((w.kick + 1) & ~1) * sizeof(double) +
+         nw * sizeof(uint32_t) +
          (size_t)w.hot * 2 * sizeof(uint32_t);
 }
 

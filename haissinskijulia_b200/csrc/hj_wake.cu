@@ -547,6 +547,7 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
                          __dmul_rn(a.pot[a.hi_idx + 1], a.hi_w));
         const double d = (j > 0 && j < a.B) ? a.pot[j] - p0 : 0.0;
         a.potd[j] = make_double2(p0, d);
+        if (j == 0) a.pot[-1] = p0;
         sum_kick += (double)a.acc[a.B + j] * p0 +
                     (double)a.acc[a.B + nc + j] * 5.9604644775390625e-08 * d;
         if (j < a.B) a.counts[j] = a.acc[j];
@@ -564,7 +565,7 @@ __device__ __forceinline__ void bins_body(const BinsArgs& a) {
   if (rank == 0 && threadIdx.x == 0 && !a.conv_only) {
     for (int r = 1; r < C; ++r) sum_kick += s_peer_sum[r];
     const TurnSums u{sh[0], sh[2], sh[3], sh[5], current, sum_kick, do_conv};
-    finish_turn(ts, a.params, a.n, a.sigma_E0_initial, a.use_wake != 0, u);
+    finish_turn(ts, ts->cur, a.params, a.n, a.sigma_E0_initial, a.use_wake != 0, u);
   }
 }
 
