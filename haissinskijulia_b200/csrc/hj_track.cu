@@ -98,16 +98,8 @@ __device__ __forceinline__ double kick_offset(double e0, double inv_e) {
 
 __device__ __forceinline__ int cic_hi(int B) { return B >= 2 ? B - 2 : 0; }
 
-// Packed CIC accumulator V = count·2^44 + Σ w·2^24 per cell (a block
-// deposits at most kMaxBlockParticles particles per turn, so neither field
-// overflows).  In shared memory V lives as two 32-bit words: 64-bit shared
-// atomics are several times slower than 32-bit ones on this GPU, so a deposit
-// adds q = w·2^24 to the low word with an atomic that returns the old value,
-// and 2^12 (one count) plus the carry out of the low word to the high word.
-// Every carry is counted exactly once, so the final words are exact.
-constexpr int kCicWeightBits = 24;
-constexpr int kCicSumBits = 44;
-constexpr unsigned long long kCicSumMask = (1ull << kCicSumBits) - 1ull;
+// Interpolation weights enter the cell sums as integers w·2^24.
+constexpr double kCicScale = 16777216.0;
 
 __device__ __forceinline__ void ld4(const double* p, double v[4]) {
   asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
@@ -195,16 +187,15 @@ __device__ __forceinline__ double2 ld_table(const double2* p) {
 //   pot[0] - pot[0] = 0, so a hot cell's (left value, step) from the window
 //   is bit-identical to its global entry.  Cells B-1 and B (whose step or
 //   value the bins step sets differently) are never hot.
-// * Histograms: bins and cells w0 .. w0 + h - 1 have their per-block
-//   counters in shared memory.  A deposit outside goes straight to the
-//   bunch's accumulators in global memory (u64: counts [B] | cell counts [B+1]
+// * Histograms: cells w0 .. w0 + h - 1 have their per-block
+//   counters in shared memory (two counts and a sum per cell).  A deposit
+//   outside goes straight to the bunch's accumulators in global memory (u64: counts [B] | cell counts [B+1]
 //   | cell Σw·2^24 [B+1]); h = B + 1 (w0 = 0) where all cells fit.
 struct PassWindow {
   const double* s_win;
   int w0;
   unsigned lim;
   unsigned h;
-  unsigned inner;   // max(h, 1) - 1: cells w0 + 1 .. w0 + inner have their bin inside too
 };
 
 // Table entry and weight of the kick of z (issued early: the gather's latency
@@ -264,36 +255,44 @@ __device__ __forceinline__ int ngp_bin(double z, const GridConst& g, bool& in) {
   return min(max(__double2loint(__dadd_rd(u, kMagic)), 0), g.B - 1);
 }
 
-// Bits of 1/2 - 2^-30 and the span up to 1/2 + 2^-30 (positive doubles order
-// as their bit patterns).
-constexpr long long kHalfLoBits = 0x3FDFFFFFFF000000ll;
-constexpr unsigned long long kHalfSpanBits = 0x3FE0000000800000ull - 0x3FDFFFFFFF000000ull;
-
-// Kick-table cell of z (as kick_cell) and, from the same coordinate, the
-// histogram bin of src/utils.jl:387-397.  v - 1/2 = z/Δe + 1/2 - e0/Δe - 1/2
-// lies within ~4 B 2^-53 (below 1e-11 for B <= 2^20) of the reference's
-// u = RN(RN(z - e0)/Δe), so for |w - 1/2| >= 2^-30 the bin floor(u) is
-// floor(v) - 1 + [w >= 1/2] and z is in range iff that bin is in [0, B-1];
-// within 2^-30 of a bin edge (at 1e8 particles about one particle in five
-// turns) ngp_bin evaluates the reference's own rounding.  The tests on w run
-// on its bits, so the bin costs no floating-point work.
-__device__ __forceinline__ void cell_and_bin(double z, const GridConst& g, int& j, double& w,
-                                             int& nb, bool& in) {
+// Kick-table cell j of z (as kick_cell), the half h of it that z lies in (h = 2 j
+// or 2 j + 1) and the weight q = w·2^24 rounded to nearest.  The halves give the
+// histogram of src/utils.jl:387-397: bin b is the upper half of cell b and the
+// lower half of cell b + 1; half 0 (below the grid) and half 2 B + 1 (above it)
+// belong to no bin.  v - 1/2 = z/Δe + 1/2 - e0/Δe - 1/2 lies within ~4 B 2^-53
+// (below 1e-11 for B <= 2^20) of the reference's u = RN(RN(z - e0)/Δe), so away
+// from a bin edge the half is [w >= 1/2]; within about 2^-21 of one (the two high
+// words of w around 1/2: one particle in a million) ngp_bin evaluates the
+// reference's own rounding.  That and any z outside cells 0..B take the branch;
+// n_out counts the particles outside the grid.  floor(v): see kick_cell.
+__device__ __forceinline__ void cell_half(double z, const GridConst& g, int& j, int& h,
+                                          uint32_t& q, int32_t& n_out, int32_t one) {
   const double v = fma(z, g.inv_e, g.v_off);
   const double fm = __dadd_rd(v, kMagic);
-  w = __dsub_rn(v, __dsub_rn(fm, kMagic));
+  const double w = __dsub_rn(v, __dsub_rn(fm, kMagic));
   const int t = __double2hiint(fm) - 0x43380000;
   const unsigned lo = (unsigned)__double2loint(fm);
-  j = (t == 0) ? (int)min(lo, (unsigned)g.B) : (t > 0 ? g.B : 0);
-  const unsigned long long near_edge =
-      (unsigned long long)(__double_as_longlong(w) - kHalfLoBits);
-  if (near_edge <= kHalfSpanBits) {
-    nb = ngp_bin(z, g, in);
-  } else {
-    const int jb = (int)lo - 1 + (__double2hiint(w) >= 0x3FE00000 ? 1 : 0);
-    in = (t == 0) & (jb >= 0) & (jb < g.B);
-    nb = jb;
+  const int wh = __double2hiint(w);
+  q = (uint32_t)__double2loint(fma(w, kCicScale, kMagic));
+  j = (int)lo;
+  h = 2 * (int)lo + (wh >= 0x3FE00000 ? 1 : 0);
+  if (t != 0 || lo - 1u >= (unsigned)g.B - 1u || (unsigned)(wh - 0x3FDFFFFF) <= 1u) {
+    j = (t == 0) ? (int)min(lo, (unsigned)g.B) : (t > 0 ? g.B : 0);
+    q = min(q, 16777216u);     // a NaN z lands in cell B with any q; the moments flag it
+    bool in;
+    const int nb = ngp_bin(z, g, in);
+    h = in ? 2 * j + (nb == j ? 1 : 0) : (j == 0 ? 0 : 2 * g.B + 1);
+    if (!in) n_out += one;
   }
+}
+
+// Adds n counts of half cell h to a bunch's accumulators (counts [B] | cell counts
+// [B+1] | cell Σw·2^24 [B+1]): to its cell and, unless it lies outside, its bin.
+__device__ __forceinline__ void add_halves(unsigned long long* __restrict__ acc, int B, int h,
+                                           unsigned long long n) {
+  atomicAdd(acc + B + (h >> 1), n);
+  const int b = ((h + 1) >> 1) - 1;
+  if ((unsigned)b < (unsigned)B) atomicAdd(acc + b, n);
 }
 
 // Reference-form bin for the single-step histogram kernel (any z).
@@ -390,92 +389,72 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
   acc_d += e - e_start;
 }
 
-// Moments and deposits of K particles' new z: Σz, Σz², the NGP count and, in
-// the kick-table cell the next pass reads for this z, the cell count and
-// Σ w·2^24.  The shared atomics of all K particles are issued before any of
-// their returned values is used, so their latencies overlap.  s_ngp, s_lo and
-// s_hi are the shared arrays offset by the window's start (w0 even, so that
-// bin b is at word b >> 1, half b & 1, of the 16-bit pairs): bin b's counter
-// is s_ngp[b] (s_ngp[b >> 1]), cell c's words s_lo[c], s_hi[c], for b and c
-// in the window.  An in-range particle's bin is its cell or the one below, so
-// a cell in (w0, w0 + h) puts both in the window: when all K are there the
-// deposits run unchecked, else each is checked and goes to global memory outside.
-// Without WIN the window holds every cell and nothing is checked.
+// Moments and deposits of K particles' new z: Σz, Σz², the count of z's half cell
+// and, in the kick-table cell the next pass reads for this z, Σ w·2^24.  One
+// count atomic per particle whose result nobody needs and one whose result only
+// tells whether the 32-bit sum wrapped (then the accumulator takes the 2^32, about
+// one deposit in 500): the cell's count and the histogram's bins both follow
+// from the halves, so neither has an atomic of its own (1e8 particles, 16384
+// bins: 0.743 ms a pass with three atomics).  The atomics of all K particles are
+// issued before any returned value is used, so their latencies overlap.  s_cnt
+// and s_lo are the shared arrays offset by the window's start: half h's counter is
+// s_cnt[h], or 16 bits of the word s_cnt[h >> 1] without N32; cell j's sum s_lo[j].
+// Without WIN the window holds every cell and nothing is checked; with it, when
+// all K cells are inside the deposits run unchecked, else each is checked and
+// goes to global memory outside.
 template <int K, bool N32, bool WIN>
 __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridConst& g,
                                               const PassWindow& hw, double& acc_z,
-                                              double& acc_z2, int32_t& n_in, uint32_t* s_ngp,
-                                              uint32_t* s_lo, uint32_t* s_hi,
+                                              double& acc_z2, int32_t& n_out, uint32_t* s_cnt,
+                                              uint32_t* s_lo,
                                               unsigned long long* __restrict__ acc) {
-  int nb[K], cj[K];
-  bool nin[K];
+  int cj[K], ch[K];
   uint32_t cq[K];
   bool inner = true;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     acc_z += z[k];
     acc_z2 = fma(z[k], z[k], acc_z2);
-    double w;
-    cell_and_bin(z[k], g, cj[k], w, nb[k], nin[k]);
-    n_in += nin[k] ? 1 : 0;
-    // w·2^24 rounded to nearest (at most 2^24; a NaN z lands in cell B with
-    // any q and is flagged by the moments)
-    cq[k] = min((uint32_t)__double2loint(fma(w, 16777216.0, kMagic)), 16777216u);
-    if (WIN) inner &= (uint32_t)(cj[k] - hw.w0 - 1) < hw.inner;
+    cell_half(z[k], g, cj[k], ch[k], cq[k], n_out, 1);
+    if (WIN) inner &= (uint32_t)(cj[k] - hw.w0) < hw.h;
   }
-  uint32_t ong[K], olo[K];
+  uint32_t onc[K], olo[K];
   if (inner) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      ong[k] = 0u;
-      if (nin[k]) {
-        if (N32) {
-          atomicAdd(&s_ngp[nb[k]], 1u);   // one 32-bit counter per bin, no return value used
-        } else {
-          ong[k] = atomicAdd(&s_ngp[nb[k] >> 1], 1u << ((nb[k] & 1) << 4));
-        }
-      }
+      if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
+      else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      atomicAdd(&s_hi[cj[k]], (1u << (kCicSumBits - 32)) + (olo[k] + cq[k] < olo[k] ? 1u : 0u));
+      if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
   } else {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      ong[k] = 0u;
-      if (nin[k]) {
-        if ((uint32_t)(nb[k] - hw.w0) < hw.h) {
-          if (N32) atomicAdd(&s_ngp[nb[k]], 1u);
-          else ong[k] = atomicAdd(&s_ngp[nb[k] >> 1], 1u << ((nb[k] & 1) << 4));
-        } else {
-          atomicAdd(acc + nb[k], 1ull);
-          nin[k] = false;                 // no 16-bit counter to check below
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
+      onc[k] = 0u;
       if ((uint32_t)(cj[k] - hw.w0) < hw.h) {
-        olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
-        atomicAdd(&s_hi[cj[k]], (1u << (kCicSumBits - 32)) + (olo[k] + cq[k] < olo[k] ? 1u : 0u));
+        if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
+        else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
+        const uint32_t o = atomicAdd(&s_lo[cj[k]], cq[k]);
+        if (o + cq[k] < o) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
       } else {
-        atomicAdd(acc + g.B + cj[k], 1ull);
+        add_halves(acc, g.B, ch[k], 1ull);
         atomicAdd(acc + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
       }
     }
   }
   if (!N32) {
-    // 16-bit counters, two bins per word: the increment that takes a counter
-    // to 2^15 moves 2^15 counts to the accumulator (the counter has another
-    // 2^15 - 1 increments of room before the move lands)
+    // 16-bit counters, the two halves of a cell in a word: the increment that
+    // takes a counter to 2^15 moves 2^15 counts to the accumulators (the counter
+    // has another 2^15 - 1 increments of room before the move lands)
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int sh = (nb[k] & 1) << 4;
-      if (nin[k] && ((ong[k] >> sh) & 0xFFFFu) == 0x7FFFu) {
-        atomicSub(&s_ngp[nb[k] >> 1], 0x8000u << sh);
-        atomicAdd(acc + nb[k], 0x8000ull);
+      const int sh = (ch[k] & 1) << 4;
+      if (((onc[k] >> sh) & 0xFFFFu) == 0x7FFFu) {
+        atomicSub(&s_cnt[cj[k]], 0x8000u << sh);
+        add_halves(acc, g.B, ch[k], 0x8000ull);
       }
     }
   }
@@ -565,31 +544,26 @@ __device__ __forceinline__ unsigned group_normals_zig(const PhiloxKeys& rk, int6
 }
 
 // Takes back what deposit_group added for one particle at z: the moments (to
-// rounding) and the NGP and cell deposits (exactly: the packed cell word
-// loses the 2^44 + q it gained, borrow included; the accumulators, also in place
-// of a 16-bit NGP counter, take the negative, modulo 2^64).
+// rounding) and the deposits (exactly: a borrow out of the cell's 32-bit sum is
+// taken from the accumulator, which also takes the negative of a count that may
+// have left its 16-bit counter, modulo 2^64).
 template <bool N32>
 __device__ __forceinline__ void undeposit(double z, const GridConst& g, const PassWindow& hw,
-                                          double& acc_z, double& acc_z2, int32_t& n_in,
-                                          uint32_t* s_ngp, uint32_t* s_lo, uint32_t* s_hi,
+                                          double& acc_z, double& acc_z2, int32_t& n_out,
+                                          uint32_t* s_cnt, uint32_t* s_lo,
                                           unsigned long long* __restrict__ acc) {
   acc_z = __dsub_rn(acc_z, z);
   acc_z2 = fma(-z, z, acc_z2);
-  int cj, nb;
-  double w;
-  bool nin;
-  cell_and_bin(z, g, cj, w, nb, nin);
-  if (nin) {
-    n_in -= 1;
-    if (N32 && (uint32_t)(nb - hw.w0) < hw.h) atomicSub(&s_ngp[nb], 1u);
-    else atomicAdd(acc + nb, ~0ull);
-  }
-  const uint32_t cq = min((uint32_t)__double2loint(fma(w, 16777216.0, kMagic)), 16777216u);
-  if ((uint32_t)(cj - hw.w0) < hw.h) {
+  int cj, ch;
+  uint32_t cq;
+  cell_half(z, g, cj, ch, cq, n_out, -1);
+  const bool in = (uint32_t)(cj - hw.w0) < hw.h;
+  if (N32 && in) atomicSub(&s_cnt[ch], 1u);
+  else add_halves(acc, g.B, ch, ~0ull);
+  if (in) {
     const uint32_t old = atomicSub(&s_lo[cj], cq);
-    atomicSub(&s_hi[cj], (1u << (kCicSumBits - 32)) + (old < cq ? 1u : 0u));
+    if (old < cq) atomicAdd(acc + 2 * g.B + 1 + cj, 0ull - (1ull << 32));
   } else {
-    atomicAdd(acc + g.B + cj, ~0ull);
     atomicAdd(acc + 2 * g.B + 1 + cj, 0ull - (unsigned long long)cq);
   }
 }
@@ -612,21 +586,24 @@ struct PassRange {
 // 10 us for the kernel that merged those.
 template <int THREADS, bool N32>
 __device__ __forceinline__ void flush_window(const PassArgs& a, const PassWindow& kw, int hot,
-                                             int32_t part, const uint32_t* h_ngp,
-                                             const uint32_t* h_lo, const uint32_t* h_hi) {
-  const int nc = a.B + 1;
+                                             int32_t part, const uint32_t* h_cnt,
+                                             const uint32_t* h_lo) {
   const int rot = hot > 0 ? (int)(((uint32_t)part * 0x9E3779B9u) >> 8) % hot & ~31 : 0;
+  auto halves = [&](int r) {                          // lower, upper
+    if (N32) return reinterpret_cast<const uint2*>(h_cnt)[r];
+    return make_uint2(h_cnt[r] & 0xFFFFu, h_cnt[r] >> 16);
+  };
   for (int i = threadIdx.x; i < hot; i += THREADS) {
     int r = i + rot;
     if (r >= hot) r -= hot;
-    unsigned long long* p = a.acc + kw.w0 + r;
-    const uint32_t n = N32 ? h_ngp[r] : (h_ngp[r >> 1] >> ((r & 1) << 4)) & 0xFFFFu;
-    const unsigned long long v = ((unsigned long long)h_hi[r] << 32) | h_lo[r];
-    if (n) atomicAdd(p, (unsigned long long)n);       // never at cell B, which has no bin
-    if (v) {
-      atomicAdd(p + a.B, v >> kCicSumBits);
-      atomicAdd(p + a.B + nc, v & kCicSumMask);
-    }
+    const int c = kw.w0 + r;
+    const uint2 n = halves(r);
+    // bin c: this cell's upper half and the next one's lower half
+    const uint32_t nb = n.y + (r + 1 < hot ? halves(r + 1).x : 0u);
+    if (nb && c < a.B) atomicAdd(a.acc + c, (unsigned long long)nb);
+    if (r == 0 && c > 0 && n.x) atomicAdd(a.acc + c - 1, (unsigned long long)n.x);
+    if (n.x + n.y) atomicAdd(a.acc + a.B + c, (unsigned long long)(n.x + n.y));
+    if (h_lo[r]) atomicAdd(a.acc + 2 * a.B + 1 + c, (unsigned long long)h_lo[r]);
   }
 }
 
@@ -645,9 +622,9 @@ __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedCo
                                                 const GridConst& g, const PassWindow& kw,
                                                 double pmean, int64_t turn, int64_t i,
                                                 const double2* s_zt, const double2* s_rf,
-                                                uint32_t* s_ngp, uint32_t* s_lo,
-                                                uint32_t* s_hi, double& acc_z, double& acc_z2,
-                                                double& acc_d, int32_t& n_in) {
+                                                uint32_t* s_cnt, uint32_t* s_lo, double& acc_z,
+                                                double& acc_z2, double& acc_d,
+                                                int32_t& n_out) {
   const double z0 = __ldcg(a.z + i), e0 = __ldcg(a.dE + i);
   double kick = 0.0;
   if (WAKE) {
@@ -671,9 +648,8 @@ __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedCo
   particle_turn<WAKE, true>(z1[0], e1, r, kick, rf, c, pmean, d1);
   acc_d = __dadd_rn(__dsub_rn(acc_d, dg), d1);
   if (WAKE) {
-    undeposit<N32>(zg, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
-    deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi,
-                               a.acc);
+    undeposit<N32>(zg, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
+    deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
   }
   a.z[i] = z1[0];
   a.dE[i] = e1;
@@ -693,9 +669,9 @@ __device__ __forceinline__ void drain_deferred(const PassArgs& a, const FusedCon
                                                int64_t stride, unsigned long long& pend,
                                                int64_t* wq, int& staged, bool last,
                                                const double2* s_zt, const double2* s_rf,
-                                               uint32_t* s_ngp, uint32_t* s_lo, uint32_t* s_hi,
+                                               uint32_t* s_cnt, uint32_t* s_lo,
                                                double& acc_z, double& acc_z2, double& acc_d,
-                                               int32_t& n_in) {
+                                               int32_t& n_out) {
   const int lane = threadIdx.x & 31;
   for (;;) {
     const int cnt = __popcll(pend);
@@ -720,7 +696,7 @@ __device__ __forceinline__ void drain_deferred(const PassArgs& a, const FusedCon
       staged -= n;
       if (lane < n)
         finish_deferred<WAKE, N32, WIN>(a, c, g, kw, pmean, turn, __ldcg(wq + staged + lane), s_zt,
-                                   s_rf, s_ngp, s_lo, s_hi, acc_z, acc_z2, acc_d, n_in);
+                                   s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d, n_out);
       __syncwarp();
     }
     if (total <= space) break;
@@ -732,20 +708,19 @@ template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32 = fal
 __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg,
                                           unsigned char* smem_raw) {
   // dynamic shared memory: RF table [128] | the ziggurat's rows [2048] (a.zig) |
-  // kick-table window [win, rounded up to even] | NGP counters | cell words lo, hi [hot] for the
-  // hot window's `hot` bins and cells; NGP counters: (hot+1)/2 words of two
-  // 16-bit counters, or hot 32-bit ones (N32)
+  // kick-table window [win, rounded up to even] | counts of the hot window's `hot`
+  // cells by halves: two 32-bit words a cell (N32), or one of two 16-bit counters |
+  // cell sums [hot]
   const int nc = a.B + 1;                 // kick-table cells
   const int hot = WAKE ? a.hwin : 0;
-  const int nw = N32 ? hot : (hot + 1) / 2;
+  const int nw = N32 ? 2 * hot : hot;
   const int win = WAKE ? a.win : 0;
   double2* s_rf = reinterpret_cast<double2*>(smem_raw);
   double2* s_zt = s_rf + kRfTableSize;
   double* s_win = reinterpret_cast<double*>(
       smem_raw + (a.zig ? kPassTableBytes : kRfTableSize * sizeof(double2)));
-  uint32_t* const h_ngp = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
-  uint32_t* const h_lo = h_ngp + nw;
-  uint32_t* const h_hi = h_lo + hot;
+  uint32_t* const h_cnt = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
+  uint32_t* const h_lo = h_cnt + nw;
   // Before the previous turn's bins step has finished: the constant tables and
   // the zeroed counters (all of the set-up that needs nothing of that step; the
   // pass of 1e5 particles takes 2 us less for it).
@@ -754,10 +729,10 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     for (int i = threadIdx.x; i < kZigLayers; i += THREADS)
       copy16_async(s_zt + i, reinterpret_cast<const double2*>(g_normal.xd) + i);
   if (WAKE) {
-    const int words = nw + 2 * hot;
-    uint4* const h4 = reinterpret_cast<uint4*>(h_ngp);
+    const int words = nw + hot;
+    uint4* const h4 = reinterpret_cast<uint4*>(h_cnt);
     for (int i = threadIdx.x; i < words / 4; i += THREADS) h4[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < (words & 3)) h_ngp[(words & ~3) + threadIdx.x] = 0u;
+    if (threadIdx.x < (words & 3)) h_cnt[(words & ~3) + threadIdx.x] = 0u;
   }
   grid_dependency_wait();
   grid_launch_dependents();   // the bins step may be scheduled: it reads the turn state too
@@ -798,7 +773,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   // windows centred on the cell of the last turn's mean z: histogram cells
   // w0 .. w0 + hot - 1 (never beyond cell B) and kick-table entries w0 .. w0 +
   // wv - 1 (wv <= win, never beyond cell B - 1)
-  PassWindow kw{s_win, 0, 0u, 0u, 0u};
+  PassWindow kw{s_win, 0, 0u, 0u};
   if (WAKE) {
     int w0 = 0;
     if (WIN && hot < nc) {   // even, so that the 16-bit pairs keep bin b at word b >> 1
@@ -809,7 +784,6 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     }
     kw.w0 = w0;
     kw.h = (unsigned)hot;
-    kw.inner = hot > 0 ? (unsigned)hot - 1u : 0u;
     if (win > 0) {
       const int wv = min(win, a.B - w0);
       if (ts->pending) {   // two entries a copy; the last may take one beyond the window
@@ -823,13 +797,12 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   }
   copies_wait();
   __syncthreads();
-  // the histograms indexed by absolute bin and cell (valid inside the window)
-  uint32_t* const s_ngp = h_ngp - (N32 ? kw.w0 : kw.w0 / 2);
+  // the counters indexed by absolute half cell and cell (valid inside the window)
+  uint32_t* const s_cnt = h_cnt - (N32 ? 2 * kw.w0 : kw.w0);
   uint32_t* const s_lo = h_lo - kw.w0;
-  uint32_t* const s_hi = h_hi - kw.w0;
 
   double acc_z = 0.0, acc_z2 = 0.0, acc_d = 0.0;
-  int32_t n_in = 0;
+  int32_t n_out = 0;
   const double2* __restrict__ potd = a.potd;
   const int64_t ng = rg.q_end;
   const int64_t stride = rg.q_step;
@@ -903,23 +876,22 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       es[j] = keep ? e0 : ee[j];
     }
     if (WAKE)
-      deposit_group<PPT, N32, WIN>(zz, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
+      deposit_group<PPT, N32, WIN>(zz, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
     stp<PPT>(a.z + PPT * q, zs);
     stp<PPT>(a.dE + PPT * q, es);
     if (kDefer) {
       pend = (pend << PPT) | (unsigned long long)(~ok & ((1u << PPT) - 1u));
       if ((it & 15) == 15 && __activemask() == 0xffffffffu)
         drain_deferred<WAKE, PPT, N32, WIN>(a, c, g, kw, pmean, turn, q, stride, pend, wq, staged,
-                                       false, s_zt, s_rf, s_ngp, s_lo, s_hi, acc_z, acc_z2,
-                                       acc_d, n_in);
+                                       false, s_zt, s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d,
+                                       n_out);
     }
   }
   if (kDefer) {
     __syncwarp();
     staged = __reduce_max_sync(0xffffffffu, (unsigned)staged);
     drain_deferred<WAKE, PPT, N32, WIN>(a, c, g, kw, pmean, turn, q - stride, stride, pend, wq, staged,
-                                   true, s_zt, s_rf, s_ngp, s_lo, s_hi, acc_z, acc_z2, acc_d,
-                                   n_in);
+                                   true, s_zt, s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d, n_out);
   }
   // Tail of n % PPT particles: the first threads of the tail block, scalar.
   if (rg.tail && threadIdx.x < (int)(a.n % PPT)) {
@@ -936,7 +908,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     particle_turn<WAKE, kDefer>(z1[0], e, r, kick, rf_term<kDefer>(z1[0], c, s_rf), c, pmean,
                                acc_d);
     if (WAKE)
-      deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_in, s_ngp, s_lo, s_hi, a.acc);
+      deposit_group<1, N32, WIN>(z1, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
     a.z[i] = z1[0];
     a.dE[i] = e;
   }
@@ -944,11 +916,12 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   __syncthreads();                        // the RF table's space becomes the reduction scratch
   static_assert(THREADS / 32 * 4 * sizeof(double) <= kRfTableSize * sizeof(double2),
                 "reduction scratch exceeds the RF table");
-  block_sum4<THREADS>(acc_z, acc_z2, acc_d, (double)n_in,
+  const int32_t n_mine = it * PPT + (rg.tail && threadIdx.x < (int)(a.n % PPT) ? 1 : 0);
+  block_sum4<THREADS>(acc_z, acc_z2, acc_d, WAKE ? (double)(n_mine - n_out) : 0.0,
                       a.part_sum + (size_t)rg.part * kNumSums,
                       reinterpret_cast<double(*)[4]>(s_rf));
 
-  if (WAKE) flush_window<THREADS, N32>(a, kw, hot, rg.part, h_ngp, h_lo, h_hi);
+  if (WAKE) flush_window<THREADS, N32>(a, kw, hot, rg.part, h_cnt, h_lo);
 }
 
 // One turn over one bunch: block b takes groups b, b + grid, ... (THREADS
@@ -1413,18 +1386,17 @@ size_t pass_table_bytes(bool zig) {
 
 }  // namespace
 
-// The pass's hot window for B bins: per cell a pair of cell words (8 bytes),
-// an NGP counter (4 bytes, or 2 with 16-bit pairs) and, above kWindowMinBins
-// bins, a kick-table entry (8 bytes), as many cells as the shared-memory
-// budget leaves beside the tables, at most B + 1 (up to 4096 bins the 64 KB
-// kick table stays in L1 beside the histograms: a kick window would only add
-// its load to every block, measured no gain).
+// The pass's hot window for B bins: per cell two counts (8 bytes, or 4 with
+// 16-bit ones), a sum (4 bytes) and, above kWindowMinBins bins, a kick-table
+// entry (8 bytes), as many cells as the shared-memory budget leaves beside the
+// tables, at most B + 1 (up to 4096 bins the 64 KB kick table stays in L1 beside
+// the histograms: a kick window would only add its load to every block, measured
+// no gain).
 PassWindows track_windows(int B, int cfg, bool zig) {
   const size_t tables = pass_table_bytes(zig), budget = pass_smem_budget(cfg);
   const bool kick = B > kWindowMinBins;
-  const size_t per = 8 + ((cfg & kPassN32) ? 4 : 2) + (kick ? 8 : 0);
-  // 12: an odd 16-bit word, an even number of kick entries
-  const size_t room = budget > tables + 12 ? budget - tables - 12 : 0;
+  const size_t per = ((cfg & kPassN32) ? 12 : 8) + (kick ? 8 : 0);
+  const size_t room = budget > tables + 8 ? budget - tables - 8 : 0;   // 8: kick entries are even
   const size_t hot = std::min(room / per, (size_t)B + 1);
   PassWindows w;
   w.hot = (int)hot;
@@ -1432,15 +1404,13 @@ PassWindows track_windows(int B, int cfg, bool zig) {
   return w;
 }
 
-// Tables, and with the wake the windows: kick-table entries, NGP counters and
-// cell words of the hot window.
+// Tables, and with the wake the windows: kick-table entries, counts and cell
+// sums of the hot window.
 size_t track_smem_bytes(int B, int use_wake, int cfg, bool zig) {
   if (!use_wake) return pass_table_bytes(zig);
   const PassWindows w = track_windows(B, cfg, zig);
-  const size_t nw = (cfg & kPassN32) ? (size_t)w.hot : (size_t)(w.hot + 1) / 2;
   return pass_table_bytes(zig) + (size_t)((w.kick + 1) & ~1) * sizeof(double) +
-         nw * sizeof(uint32_t) +
-         (size_t)w.hot * 2 * sizeof(uint32_t);
+         (size_t)w.hot * ((cfg & kPassN32) ? 3 : 2) * sizeof(uint32_t);
 }
 
 namespace {
