@@ -263,27 +263,31 @@ __device__ __forceinline__ int ngp_bin(double z, const GridConst& g, bool& in) {
 // (below 1e-11 for B <= 2^20) of the reference's u = RN(RN(z - e0)/Δe), so away
 // from a bin edge the half is [w >= 1/2]; within about 2^-21 of one (the two high
 // words of w around 1/2: one particle in a million) ngp_bin evaluates the
-// reference's own rounding.  That and any z outside cells 0..B take the branch;
-// n_out counts the particles outside the grid.  floor(v): see kick_cell.
-__device__ __forceinline__ void cell_half(double z, const GridConst& g, int& j, int& h,
-                                          uint32_t& q, int32_t& n_out, int32_t one) {
+// reference's own rounding.  cell_half_fast says whether none of that applies
+// (and z lies in cells 1..B-1); cell_half serves any z and counts the particles
+// outside the grid in n_out.  floor(v): see kick_cell.
+__device__ __forceinline__ bool cell_half_fast(double z, const GridConst& g, int& j, int& h,
+                                               uint32_t& q) {
   const double v = fma(z, g.inv_e, g.v_off);
   const double fm = __dadd_rd(v, kMagic);
   const double w = __dsub_rn(v, __dsub_rn(fm, kMagic));
-  const int t = __double2hiint(fm) - 0x43380000;
-  const unsigned lo = (unsigned)__double2loint(fm);
   const int wh = __double2hiint(w);
   q = (uint32_t)__double2loint(fma(w, kCicScale, kMagic));
-  j = (int)lo;
-  h = 2 * (int)lo + (wh >= 0x3FE00000 ? 1 : 0);
-  if (t != 0 || lo - 1u >= (unsigned)g.B - 1u || (unsigned)(wh - 0x3FDFFFFF) <= 1u) {
-    j = (t == 0) ? (int)min(lo, (unsigned)g.B) : (t > 0 ? g.B : 0);
-    q = min(q, 16777216u);     // a NaN z lands in cell B with any q; the moments flag it
-    bool in;
-    const int nb = ngp_bin(z, g, in);
-    h = in ? 2 * j + (nb == j ? 1 : 0) : (j == 0 ? 0 : 2 * g.B + 1);
-    if (!in) n_out += one;
-  }
+  j = __double2loint(fm);
+  h = 2 * j + (wh >= 0x3FE00000 ? 1 : 0);
+  return (__double2hiint(fm) == 0x43380000) & ((unsigned)j - 1u < (unsigned)g.B - 1u) &
+         ((unsigned)(wh - 0x3FDFFFFF) > 1u);
+}
+__device__ __forceinline__ void cell_half(double z, const GridConst& g, int& j, int& h,
+                                          uint32_t& q, int32_t& n_out, int32_t one) {
+  if (cell_half_fast(z, g, j, h, q)) return;
+  double w;
+  kick_cell(z, g, j, w);
+  q = min(q, 16777216u);     // a NaN z lands in cell B with any q; the moments flag it
+  bool in;
+  const int nb = ngp_bin(z, g, in);
+  h = in ? 2 * j + (nb == j ? 1 : 0) : (j == 0 ? 0 : 2 * g.B + 1);
+  if (!in) n_out += one;
 }
 
 // Adds n counts of half cell h to a bunch's accumulators (counts [B] | cell counts
@@ -399,9 +403,11 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
 // issued before any returned value is used, so their latencies overlap.  s_cnt
 // and s_lo are the shared arrays offset by the window's start: half h's counter is
 // s_cnt[h], or 16 bits of the word s_cnt[h >> 1] without N32; cell j's sum s_lo[j].
-// Without WIN the window holds every cell and nothing is checked; with it, when
-// all K cells are inside the deposits run unchecked, else each is checked and
-// goes to global memory outside.
+// When none of the K particles needs the reference's rounding and, with WIN, all K
+// cells are in the window, the deposits run straight through, else one by one
+// with every check; deposits outside the window go to global memory.  One branch
+// for the group where every particle had its own: 722 -> 690 us a pass of 1e8
+// particles at 16384 bins, 724 -> 685 at 4096.
 template <int K, bool N32, bool WIN>
 __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridConst& g,
                                               const PassWindow& hw, double& acc_z,
@@ -410,16 +416,16 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
                                               unsigned long long* __restrict__ acc) {
   int cj[K], ch[K];
   uint32_t cq[K];
-  bool inner = true;
+  bool plain = true;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     acc_z += z[k];
     acc_z2 = fma(z[k], z[k], acc_z2);
-    cell_half(z[k], g, cj[k], ch[k], cq[k], n_out, 1);
-    if (WIN) inner &= (uint32_t)(cj[k] - hw.w0) < hw.h;
+    plain &= cell_half_fast(z[k], g, cj[k], ch[k], cq[k]);
+    if (WIN) plain &= (uint32_t)(cj[k] - hw.w0) < hw.h;
   }
   uint32_t onc[K], olo[K];
-  if (inner) {
+  if (plain) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
@@ -431,18 +437,31 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
     for (int k = 0; k < K; ++k)
       if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
   } else {
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < K; ++k) {
-      onc[k] = 0u;
-      if ((uint32_t)(cj[k] - hw.w0) < hw.h) {
-        if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
-        else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
-        const uint32_t o = atomicAdd(&s_lo[cj[k]], cq[k]);
-        if (o + cq[k] < o) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
+      double zk = z[0];
+#pragma unroll
+      for (int m = 1; m < K; ++m) zk = k == m ? z[m] : zk;
+      int j, h;
+      uint32_t q;
+      cell_half(zk, g, j, h, q, n_out, 1);
+      uint32_t o = 0u;
+      if (!WIN || (uint32_t)(j - hw.w0) < hw.h) {
+        if (N32) atomicAdd(&s_cnt[h], 1u);
+        else o = atomicAdd(&s_cnt[j], 1u << ((h & 1) << 4));
+        const uint32_t lo = atomicAdd(&s_lo[j], q);
+        if (lo + q < lo) atomicAdd(acc + 2 * g.B + 1 + j, 1ull << 32);
       } else {
-        add_halves(acc, g.B, ch[k], 1ull);
-        atomicAdd(acc + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
+        add_halves(acc, g.B, h, 1ull);
+        atomicAdd(acc + 2 * g.B + 1 + j, (unsigned long long)q);
       }
+#pragma unroll
+      for (int m = 0; m < K; ++m)
+        if (k == m) {
+          onc[m] = o;
+          cj[m] = j;
+          ch[m] = h;
+        }
     }
   }
   if (!N32) {
@@ -571,12 +590,14 @@ __device__ __forceinline__ void undeposit(double z, const GridConst& g, const Pa
 // One turn over the bunch.  PPT particles per thread per iteration (4 with the
 // next group prefetched in registers, or 2 with twice the threads per SM).
 // Particle groups (PPT particles each) one block processes: thread t takes
-// groups q_begin + t, + q_step, ... below q_end; its partial histograms and
-// sums go to slot `part`; the `tail` block also takes the n % PPT last particles.
+// groups q_begin + t, + q_step, ... below q_end, q_end - q_begin a multiple of 32, so
+// that the warps stay whole; the fewer than 32 PPT particles left over are the
+// `tail_count` ones from tail_first, one a thread.  Its sums go to slot `part`.
 struct PassRange {
   int64_t q_begin, q_step, q_end;
+  int64_t tail_first;
+  int32_t tail_count;
   int32_t part;
-  bool tail;
 };
 
 // Adds a block's window counters to the bunch's accumulators.  Each block
@@ -826,6 +847,9 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   int64_t* wq = kDefer ? a.defer_q + ((int64_t)rg.part * (THREADS / 32) + (threadIdx.x >> 5)) *
                                          kDeferStage
                        : nullptr;
+  // with the wake two groups a trip, so that the prefetched group needs no register moves
+  // (single-precision normals 660 -> 640 us, Float64 690 -> 684)
+#pragma unroll (WAKE ? 2 : 1)
   for (; q < ng; q += stride, ++it) {
     double zz[PPT], ee[PPT], rr[PPT];
     if (kPrefetch) {
@@ -881,7 +905,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     stp<PPT>(a.dE + PPT * q, es);
     if (kDefer) {
       pend = (pend << PPT) | (unsigned long long)(~ok & ((1u << PPT) - 1u));
-      if ((it & 15) == 15 && __activemask() == 0xffffffffu)
+      if ((it & 15) == 15)   // the warp is whole: q_end - q_begin is a multiple of 32
         drain_deferred<WAKE, PPT, N32, WIN>(a, c, g, kw, pmean, turn, q, stride, pend, wq, staged,
                                        false, s_zt, s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d,
                                        n_out);
@@ -893,9 +917,10 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     drain_deferred<WAKE, PPT, N32, WIN>(a, c, g, kw, pmean, turn, q - stride, stride, pend, wq, staged,
                                    true, s_zt, s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d, n_out);
   }
-  // Tail of n % PPT particles: the first threads of the tail block, scalar.
-  if (rg.tail && threadIdx.x < (int)(a.n % PPT)) {
-    const int64_t i = (a.n / PPT) * PPT + threadIdx.x;
+  // The particles left over by whole warps: the first threads, scalar.
+  const bool tail = (int)threadIdx.x < rg.tail_count;
+  if (tail) {
+    const int64_t i = rg.tail_first + threadIdx.x;
     double r2[2] = {0.0, 0.0};
     if (QE == QE_PHILOX)
       philox_normals2_rk(a.seed, a.philox, turn, (i >> 1) + a.pair_offset, &g_normal, s_zt, r2);
@@ -916,7 +941,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   __syncthreads();                        // the RF table's space becomes the reduction scratch
   static_assert(THREADS / 32 * 4 * sizeof(double) <= kRfTableSize * sizeof(double2),
                 "reduction scratch exceeds the RF table");
-  const int32_t n_mine = it * PPT + (rg.tail && threadIdx.x < (int)(a.n % PPT) ? 1 : 0);
+  const int32_t n_mine = it * PPT + (tail ? 1 : 0);
   block_sum4<THREADS>(acc_z, acc_z2, acc_d, WAKE ? (double)(n_mine - n_out) : 0.0,
                       a.part_sum + (size_t)rg.part * kNumSums,
                       reinterpret_cast<double(*)[4]>(s_rf));
@@ -931,8 +956,10 @@ template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, int MINB = 1, 
           bool WIN = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const PassRange rg{(int64_t)blockIdx.x * THREADS, (int64_t)gridDim.x * THREADS, a.n / PPT,
-                     (int32_t)blockIdx.x, blockIdx.x == 0};
+  const int64_t groups = a.n / PPT & ~(int64_t)31;
+  const PassRange rg{(int64_t)blockIdx.x * THREADS, (int64_t)gridDim.x * THREADS, groups,
+                     groups * PPT, blockIdx.x == 0 ? (int32_t)(a.n - groups * PPT) : 0,
+                     (int32_t)blockIdx.x};
   pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
 }
 
@@ -965,8 +992,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
     const BatchChunk ch = chunks[c];
     const PassArgs a = bunches[ch.bunch];
     if (a.ts->turns_left > 0) {
-      const PassRange rg{ch.first / PPT, THREADS, (ch.first + ch.count) / PPT, ch.part,
-                         ch.first + ch.count == a.n};
+      const int64_t groups = ch.count / PPT & ~(int64_t)31;
+      const PassRange rg{ch.first / PPT, THREADS, ch.first / PPT + groups,
+                         ch.first + groups * PPT, (int32_t)(ch.count - groups * PPT), ch.part};
       pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
     }
     if (!QUEUE) break;
