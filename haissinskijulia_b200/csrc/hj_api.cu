@@ -426,8 +426,8 @@ extern "C" void hj_bunch_destroy(hj_bunch* b) {
 // buffers and enqueues the initial moments and their copy to the host;
 // bunch_create_end (after the stream has reached them) builds the grid, the
 // wake tables, the RF table and the turn state.
-// chunk > 0: a batch member, whose partial slots are its chunks of `chunk`
-// particles (the batch's chunk table) instead of one per block of the grid;
+// chunk > 0: a batch member, whose partial slots are its chunks of
+// member_chunk(n, chunk) particles (the batch's chunk table) instead of one per block of the grid;
 // cfg >= 0 pins the pass layout.
 hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
                                       const hj_params* params, const hj_wake* wake,
@@ -476,7 +476,8 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
   b->cfg = cfg >= 0 ? cfg : auto_pass_layout(ctx->pass_layout, b->B, n);
   if (chunk > 0) {
     b->batch_member = true;
-    b->nblk = (int)std::max<int64_t>((n + chunk - 1) / chunk, 1);
+    b->chunk = member_chunk(n, chunk);
+    b->nblk = (int)std::max<int64_t>((n + b->chunk - 1) / b->chunk, 1);
   } else {
     const int bps = track_blocks_per_sm(b->B, b->qe_mode, b->use_wake, b->cfg);
     b->nblk = track_grid_size(n, b->B, ctx->num_sms, bps, b->cfg);

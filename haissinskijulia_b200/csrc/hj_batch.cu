@@ -90,8 +90,8 @@ hj_status batch_upload(hj_batch* bt) {
     fill_scan_args(b, bt->h_bins[k]);
     for (int c = 0; c < b->nblk; ++c) {
       BatchChunk ch;
-      ch.first = (int64_t)c * bt->chunk;
-      ch.count = std::min<int64_t>(bt->chunk, b->n - ch.first);
+      ch.first = (int64_t)c * b->chunk;
+      ch.count = std::min<int64_t>(b->chunk, b->n - ch.first);
       ch.bunch = k;
       ch.part = c;
       if (nch >= bt->max_chunks) return set_err(ctx, HJ_ERR_STATE, "batch chunk table overflow");
@@ -118,8 +118,10 @@ hj_status batch_upload(hj_batch* bt) {
     HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_bins, bt->h_bins, sizeof(ScanArgs) * nb,
                                  cudaMemcpyHostToDevice, bt->stream));
   }
-  if (nch > 0)
-    HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_chunks, bt->h_chunks, sizeof(BatchChunk) * nch,
+  // empty chunks up to the grid
+  std::fill(bt->h_chunks + nch, bt->h_chunks + std::max(bt->grid_chunks, nch), BatchChunk{});
+  if (bt->grid_chunks > 0)
+    HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_chunks, bt->h_chunks, sizeof(BatchChunk) * bt->grid_chunks,
                                  cudaMemcpyHostToDevice, bt->stream));
   HJ_CUDA(ctx, cudaMemcpyAsync(bt->d_counts, bt->h_counts, sizeof(int32_t) * 2,
                                cudaMemcpyHostToDevice, bt->stream));
@@ -199,7 +201,10 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->max_B = max_nbins;
   bt->cfg = auto_pass_layout(layout, max_nbins, pool_particles);
   bt->pool_n = (pool_particles + 3) / 4 * 4;
-  bt->max_chunks = (int)std::min<int64_t>(bt->pool_n / chunk + max_bunches + 1, INT32_MAX);
+  // a member has at most n / chunk + 1 chunks, or kMemberBlocks smaller ones
+  // (member_chunk)
+  bt->max_chunks = (int)std::min<int64_t>(
+      bt->pool_n / chunk + (kMemberBlocks + 1) * (int64_t)max_bunches + 1, INT32_MAX);
   HJ_CUDA(ctx, cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking));
   // the pool and the tables: one device and one pinned block of the context's cache
   const size_t nb = (size_t)max_bunches, nc = (size_t)bt->max_chunks;

@@ -357,13 +357,21 @@ template <int C, int NT, int E>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(NT + 32, 2)
     k_batch_scan(const ScanArgs* __restrict__ bunches, const int32_t* __restrict__ n_bunches) {
   const int i = (int)(blockIdx.x / C);
-  if (i >= *n_bunches) return;
+  if (i >= *n_bunches) {
+    grid_dependency_wait();   // every block completes after the kernels before it
+    return;
+  }
   __shared__ ScanArgs s_a;
   const int* src = reinterpret_cast<const int*>(bunches + i);
   for (int k = threadIdx.x; k < (int)(sizeof(ScanArgs) / sizeof(int)); k += NT + 32)
     reinterpret_cast<int*>(&s_a)[k] = __ldg(src + k);
   __syncthreads();
-  if (__ldcg(&s_a.ts->turns_left) <= 0) return;
+  // written by the previous bins step, which every block of this turn's pass has
+  // waited for before it let this kernel start
+  if (__ldcg(&s_a.ts->turns_left) <= 0) {
+    grid_dependency_wait();
+    return;
+  }
   scan_body<C, NT, E>(s_a);
 }
 
@@ -427,8 +435,8 @@ cudaError_t launch_batch_scan(const ScanArgs* d_bunches, const int32_t* d_n_bunc
                               int max_bunches, int max_B, cudaStream_t st) {
   const ScanForm f = batch_scan_form(max_B);
   void* args[] = {const_cast<ScanArgs**>(&d_bunches), const_cast<int32_t**>(&d_n_bunches)};
-  return cudaLaunchKernel(f.fn, dim3(f.C * (max_bunches > 0 ? max_bunches : 1)),
-                          dim3(f.NT + 32), args, f.smem, st);
+  PdlConfig l(dim3(f.C * (max_bunches > 0 ? max_bunches : 1)), dim3(f.NT + 32), f.smem, st);
+  return cudaLaunchKernelExC(&l.cfg, f.fn, args);
 }
 
 }  // namespace hj

@@ -111,6 +111,7 @@ struct hj_bunch {
   // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, acc and hist are the first zero_bytes of the
   // arena's histogram part
   bool batch_member = false;
+  int64_t chunk = 0;                      // a member's particles per block of the pass
   void* tables = nullptr;
   size_t tables_cap = 0;
   size_t zero_bytes = 0;

@@ -680,9 +680,11 @@ __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedCo
 // particle j of the group k iterations before `qref`) into the warp's
 // staging queue wq (kDeferStage indices in global memory, `staged` of them
 // held; each lane's entries after those of the lanes below it, by a prefix
-// over the lanes' counts), and finishes them 32 at a time (finish_deferred)
-// -- all of them when `last`, else only full waves, the rest staying queued.
-// Every lane of the warp must take part.
+// over the lanes' counts), and finishes them 32 at a time (finish_deferred),
+// the rest staying queued.  At the last call nothing is queued any more: each
+// lane finishes its own particles, lanes without one take the queue's rest (a
+// block with one iteration, i.e. a small bunch, saves the queue's round trip
+// through L2).  Every lane of the warp must take part.
 template <bool WAKE, int PPT, bool N32, bool WIN>
 __device__ __forceinline__ void drain_deferred(const PassArgs& a, const FusedConst& c,
                                                const GridConst& g, const PassWindow& kw,
@@ -694,33 +696,70 @@ __device__ __forceinline__ void drain_deferred(const PassArgs& a, const FusedCon
                                                double& acc_z, double& acc_z2, double& acc_d,
                                                int32_t& n_out) {
   const int lane = threadIdx.x & 31;
+  auto pop = [&]() {                                  // the particle of pend's lowest bit
+    const int b = __ffsll(pend) - 1;
+    pend &= pend - 1ull;
+    return (int64_t)PPT * (qref - (int64_t)(b / PPT) * stride) + (b % PPT);
+  };
   for (;;) {
-    const int cnt = __popcll(pend);
-    int incl = cnt;
+    int64_t i = -1;
+    bool more = false;
+    if (last) {
+      const unsigned own = __ballot_sync(0xffffffffu, pend != 0ull);
+      if (own == 0u && staged == 0) break;
+      if (pend) {
+        i = pop();
+      } else {
+        const int rank = __popc(~own & ((1u << lane) - 1u));
+        if (rank < staged) i = __ldcg(wq + staged - 1 - rank);
+      }
+      staged -= min(staged, 32 - __popc(own));
+      more = true;
+    } else {
+      const int cnt = __popcll(pend);
+      int incl = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int space = kDeferStage - staged;
-    int slot = staged + incl - cnt;
-    while (pend && slot < kDeferStage) {
-      const int b = __ffsll(pend) - 1;
-      wq[slot++] = (int64_t)PPT * (qref - (int64_t)(b / PPT) * stride) + (b % PPT);
-      pend &= pend - 1ull;
-    }
-    staged += min(total, space);
-    __syncwarp();
-    while (staged >= 32 || (last && staged > 0)) {
-      const int n = min(staged, 32);
-      staged -= n;
-      if (lane < n)
-        finish_deferred<WAKE, N32, WIN>(a, c, g, kw, pmean, turn, __ldcg(wq + staged + lane), s_zt,
-                                   s_rf, s_cnt, s_lo, acc_z, acc_z2, acc_d, n_out);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      const int space = kDeferStage - staged;
+      int slot = staged + incl - cnt;
+      while (pend && slot < kDeferStage) wq[slot++] = pop();
+      staged += min(total, space);
+      more = total > space || staged >= 64;
       __syncwarp();
+      if (staged < 32) break;
+      staged -= 32;
+      i = __ldcg(wq + staged + lane);
     }
-    if (total <= space) break;
+    if (i >= 0)
+      finish_deferred<WAKE, N32, WIN>(a, c, g, kw, pmean, turn, i, s_zt, s_rf, s_cnt, s_lo, acc_z,
+                                      acc_z2, acc_d, n_out);
+    __syncwarp();
+    if (!more) break;
+  }
+}
+
+// The part of a pass's set-up that needs neither its bunch nor the previous turn's
+// bins step: the ziggurat's rows, and zeros in all of the shared memory behind the
+// tables (the pass of 1e5 particles takes 2 us less for doing it while the bins
+// step runs).
+template <bool WAKE, int QE, int THREADS>
+__device__ __forceinline__ void pass_setup(unsigned char* smem_raw) {
+  constexpr bool kZig = QE == QE_PHILOX;
+  double2* const s_zt = reinterpret_cast<double2*>(smem_raw) + kRfTableSize;
+  if (kZig)
+    for (int i = threadIdx.x; i < kZigLayers; i += THREADS)
+      copy16_async(s_zt + i, reinterpret_cast<const double2*>(g_normal.xd) + i);
+  if (WAKE) {
+    uint32_t bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+    constexpr uint32_t kTables = (uint32_t)(kZig ? kPassTableBytes : kRfTableSize * sizeof(double2));
+    uint4* const z = reinterpret_cast<uint4*>(smem_raw + kTables);
+    const int n = (int)((bytes - kTables) / 16);      // a multiple of 16 bytes is asked for
+    for (int i = threadIdx.x; i < n; i += THREADS) z[i] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -742,23 +781,17 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       smem_raw + (a.zig ? kPassTableBytes : kRfTableSize * sizeof(double2)));
   uint32_t* const h_cnt = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
   uint32_t* const h_lo = h_cnt + nw;
-  // Before the previous turn's bins step has finished: the constant tables and
-  // the zeroed counters (all of the set-up that needs nothing of that step; the
-  // pass of 1e5 particles takes 2 us less for it).
   for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) copy16_async(s_rf + i, a.rf_table + i);
-  if (QE == QE_PHILOX)
-    for (int i = threadIdx.x; i < kZigLayers; i += THREADS)
-      copy16_async(s_zt + i, reinterpret_cast<const double2*>(g_normal.xd) + i);
-  if (WAKE) {
-    const int words = nw + hot;
-    uint4* const h4 = reinterpret_cast<uint4*>(h_cnt);
-    for (int i = threadIdx.x; i < words / 4; i += THREADS) h4[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < (words & 3)) h_cnt[(words & ~3) + threadIdx.x] = 0u;
-  }
   grid_dependency_wait();
   grid_launch_dependents();   // the bins step may be scheduled: it reads the turn state too
-
   TurnState* ts = a.ts;
+  const bool done = ts->turns_left <= 0;      // a batch member's budget is spent
+  __syncthreads();            // the zeros are written where the kick window goes
+  if (done) {
+    copies_wait();
+    return;
+  }
+
   const TurnScalars sc = ts->cur;
   const double pmean = ts->pending ? ts->pending_mean : 0.0;
   const int64_t turn = ts->turn;
@@ -960,14 +993,26 @@ __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
   const PassRange rg{(int64_t)blockIdx.x * THREADS, (int64_t)gridDim.x * THREADS, groups,
                      groups * PPT, blockIdx.x == 0 ? (int32_t)(a.n - groups * PPT) : 0,
                      (int32_t)blockIdx.x};
+  pass_setup<WAKE, QE, THREADS>(smem_raw);
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
+}
+
+template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN>
+__device__ __forceinline__ void run_chunk(const PassArgs* __restrict__ bunches,
+                                          const BatchChunk& ch, unsigned char* smem_raw) {
+  pass_setup<WAKE, QE, THREADS>(smem_raw);
+  const PassArgs a = bunches[ch.bunch];
+  const int64_t groups = ch.count / PPT & ~(int64_t)31;
+  const PassRange rg{ch.first / PPT, THREADS, ch.first / PPT + groups,
+                     ch.first + groups * PPT, (int32_t)(ch.count - groups * PPT), ch.part};
   pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
 }
 
 // One turn over a batch of bunches.  Chunk c of the chunk table (a
 // contiguous run of one bunch's particles) is processed by one block into the
 // bunch's partial slot ch.part; chunks of bunches with no turns left are
-// skipped.  Without QUEUE, block c takes chunk c (blocks past the table's
-// length return at once).  With QUEUE (the turn's counter, zero at launch),
+// skipped.  Without QUEUE, block c takes chunk c (empty ones, past the live
+// chunks, return at once).  With QUEUE (the turn's counter, zero at launch),
 // the blocks are resident -- one per SM slot -- and each takes the next
 // chunk index from the counter until the table is exhausted.  Either way a
 // chunk's arithmetic and slot do not depend on the block that takes it.  The
@@ -981,27 +1026,22 @@ __global__ void __launch_bounds__(THREADS, MINB)
                  const int32_t* __restrict__ n_chunks, int32_t* queue) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_chunk;
-  const int nch = *n_chunks;
-  int c = (int)blockIdx.x;
   if (QUEUE) {
-    if (threadIdx.x == 0) s_chunk = atomicAdd(queue, 1);
-    __syncthreads();
-    c = s_chunk;
-  }
-  while (c < nch) {
-    const BatchChunk ch = chunks[c];
-    const PassArgs a = bunches[ch.bunch];
-    if (a.ts->turns_left > 0) {
-      const int64_t groups = ch.count / PPT & ~(int64_t)31;
-      const PassRange rg{ch.first / PPT, THREADS, ch.first / PPT + groups,
-                         ch.first + groups * PPT, (int32_t)(ch.count - groups * PPT), ch.part};
-      pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
+    const int nch = *n_chunks;
+    for (;;) {
+      if (threadIdx.x == 0) s_chunk = atomicAdd(queue, 1);
+      __syncthreads();
+      if (s_chunk >= nch) break;
+      run_chunk<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(bunches, chunks[s_chunk], smem_raw);
+      __syncthreads();                 // the chunk's shared memory is read no more
     }
-    if (!QUEUE) break;
-    __syncthreads();                   // the chunk's shared memory is read no more
-    if (threadIdx.x == 0) s_chunk = atomicAdd(queue, 1);
-    __syncthreads();
-    c = s_chunk;
+  } else {
+    const BatchChunk ch = chunks[blockIdx.x];
+    if (ch.count == 0) {               // the table is padded to the grid with empty chunks
+      grid_dependency_wait();          // every block completes after the kernels before it
+      return;
+    }
+    run_chunk<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(bunches, ch, smem_raw);
   }
 }
 
@@ -1424,7 +1464,8 @@ PassWindows track_windows(int B, int cfg, bool zig) {
   const size_t tables = pass_table_bytes(zig), budget = pass_smem_budget(cfg);
   const bool kick = B > kWindowMinBins;
   const size_t per = ((cfg & kPassN32) ? 12 : 8) + (kick ? 8 : 0);
-  const size_t room = budget > tables + 8 ? budget - tables - 8 : 0;   // 8: kick entries are even
+  // 24: an even number of kick entries, counters to a multiple of 16 bytes
+  const size_t room = budget > tables + 24 ? budget - tables - 24 : 0;
   const size_t hot = std::min(room / per, (size_t)B + 1);
   PassWindows w;
   w.hot = (int)hot;
@@ -1437,8 +1478,9 @@ PassWindows track_windows(int B, int cfg, bool zig) {
 size_t track_smem_bytes(int B, int use_wake, int cfg, bool zig) {
   if (!use_wake) return pass_table_bytes(zig);
   const PassWindows w = track_windows(B, cfg, zig);
+  const size_t hist = (size_t)w.hot * ((cfg & kPassN32) ? 3 : 2) * sizeof(uint32_t);
   return pass_table_bytes(zig) + (size_t)((w.kick + 1) & ~1) * sizeof(double) +
-         (size_t)w.hot * ((cfg & kPassN32) ? 3 : 2) * sizeof(uint32_t);
+         ((hist + 15) & ~(size_t)15);
 }
 
 namespace {
@@ -1509,8 +1551,9 @@ cudaError_t launch_batch_pass(const PassArgs* d_bunches, const BatchChunk* d_chu
     if (e != cudaSuccess) return e;
     grid = std::max(1, std::min(grid, resident_blocks));
   }
-  return cudaLaunchKernel(batch_fn(wake, qe, launch_cfg(max_B, wake, qe, cfg), d_queue != nullptr),
-                          dim3(grid), dim3(pass_cfg_threads(cfg)), args, smem, st);
+  PdlConfig l(dim3(grid), dim3(pass_cfg_threads(cfg)), smem, st);
+  return cudaLaunchKernelExC(
+      &l.cfg, batch_fn(wake, qe, launch_cfg(max_B, wake, qe, cfg), d_queue != nullptr), args);
 }
 
 int batch_blocks_per_sm(int max_B, int qe_mode, int use_wake, int cfg) {
