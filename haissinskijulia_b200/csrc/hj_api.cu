@@ -218,14 +218,12 @@ void sum_moments(const hj_bunch* b, double m[4]) {
 }
 
 hj_status read_moments(hj_bunch* b, double m[4]) {
-  HJ_CUDA(b->ctx, cudaMemcpyAsync(b->h_mom, b->part_mom, sizeof(double) * 4 * b->nblk_m,
-                                  cudaMemcpyDeviceToHost, b->stream));
   HJ_CUDA(b->ctx, cudaStreamSynchronize(b->stream));
   sum_moments(b, m);
   return HJ_OK;
 }
 
-hj_status launch_moments(hj_bunch* b, int apply, double* z_out, double* dE_out) {
+static FlushArgs flush_args(hj_bunch* b, int apply, double* z_out, double* dE_out) {
   FlushArgs f{};
   f.z = b->z;
   f.dE = b->dE;
@@ -235,15 +233,21 @@ hj_status launch_moments(hj_bunch* b, int apply, double* z_out, double* dE_out) 
   f.B = b->B;
   f.use_wake = b->use_wake;
   f.update_E0 = b->p.update_E0;
-  f.c1 = b->c1;
-  f.cB = b->cB;
-  f.inv_cstep = b->inv_c;
   f.e0 = b->e0;
   f.inv_estep = b->inv_e;
   f.apply = apply;
   f.z_out = z_out;
   f.dE_out = dE_out;
-  f.part = b->part_mom;
+  f.part = b->h_mom;
+  return f;
+}
+
+hj_status launch_moments(hj_bunch* b, int apply, double* z_out, double* dE_out, bool to_host,
+                         bool retire) {
+  FlushArgs f = flush_args(b, apply, z_out, dE_out);
+  if (to_host) f.ts_out = b->h_ts;
+  else f.part = b->part_mom;
+  f.retire = retire ? 1 : 0;
   HJ_CUDA(b->ctx, launch_flush(f, b->nblk_m, b->stream));
   return HJ_OK;
 }
@@ -432,7 +436,8 @@ extern "C" void hj_bunch_destroy(hj_bunch* b) {
 hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
                                       const hj_params* params, const hj_wake* wake,
                                       int64_t nbins, const hj_grid* grid, uint64_t seed,
-                                      void* stream, hj_bunch* b, int64_t chunk, int cfg) {
+                                      void* stream, hj_bunch* b, int64_t chunk, int cfg,
+                                      const double* z_src, const double* dE_src) {
   b->ctx = ctx;
   if (!b->holds_ctx) {
     ctx_retain(ctx);
@@ -519,18 +524,19 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     Carve hc;
     const size_t h_mom = hc.add<double>(4 * (size_t)b->nblk_m);
     const size_t h_ts = hc.add<TurnState>(1);
-    const size_t h_rf = hc.add<double>(2 * (size_t)kRfTableSize);
     HJ_TRY(cache_take(ctx, true, hc.off, &b->harena, &b->harena_cap));
     b->h_mom = (double*)((char*)b->harena + h_mom);
     b->h_ts = (TurnState*)((char*)b->harena + h_ts);
-    b->h_rf = (double*)((char*)b->harena + h_rf);
   }
 
   // Initial spreads, src/evolution.jl:247-249: enqueued here, read in
-  // bunch_create_end
-  HJ_TRY(launch_moments(b, 0, nullptr, nullptr));
-  HJ_CUDA(ctx, cudaMemcpyAsync(b->h_mom, b->part_mom, sizeof(double) * 4 * b->nblk_m,
-                               cudaMemcpyDeviceToHost, b->stream));
+  // bunch_create_end; the particles come from z_src, dE_src where those are given
+  FlushArgs f = flush_args(b, 0, z_src ? b->z : nullptr, z_src ? b->dE : nullptr);
+  if (z_src) {
+    f.z = z_src;
+    f.dE = dE_src;
+  }
+  HJ_CUDA(ctx, launch_flush(f, b->nblk_m, b->stream));
   return HJ_OK;
 }
 
@@ -602,14 +608,7 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
       HJ_CUDA(ctx, e);
       HJ_CUDA(ctx, e2);
     }
-    HJ_CUDA(ctx, cudaMemsetAsync(b->pot - 1, 0, b->zero_bytes, b->stream));   // pot potd acc hist
   }
-
-  // RF table, staged in the bunch's pinned block
-  host_rf_table(params->voltage, params->phi_s, kRfTableSize, b->h_rf);
-  b->rf_Vs = b->h_rf[0];
-  HJ_CUDA(ctx, cudaMemcpyAsync(b->rf_table, b->h_rf, sizeof(double) * 2 * kRfTableSize,
-                               cudaMemcpyHostToDevice, b->stream));
 
   TurnState t{};
   t.cur = make_turn_scalars(cp ? cp->E0 : params->E0, *params, b->sigma_E0_initial);
@@ -617,15 +616,15 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
   t.pending_mean = 0.0;
   t.turn = cp ? cp->turn : 1;
   b->turns_done = cp ? cp->turn - 1 : 0;
-  t.turns_left = INT64_MAX;   // a plain bunch runs until it is finished
+  t.turns_left = b->turns_left;
   t.status = 0;
   *b->h_ts = t;
-  // staged in pinned memory that lives as long as the bunch; later work on
-  // the stream is ordered after the copy, host reads of h_ts synchronise first
-  // (a batch member's state goes to the batch's array instead)
-  if (!b->batch_member)
-    HJ_CUDA(ctx, cudaMemcpyAsync(b->ts, b->h_ts, sizeof(TurnState), cudaMemcpyHostToDevice,
-                                 b->stream));
+  double sc[4];
+  host_sincos(params->phi_s, sc);
+  // pot, potd, acc and hist cleared, RF table, turn state
+  HJ_CUDA(ctx, launch_bunch_setup(b->use_wake ? (void*)(b->pot - 1) : nullptr,
+                                  b->use_wake ? b->zero_bytes : 0, b->rf_table, params->voltage, sc,
+                                  b->ts, t, b->stream));
   return HJ_OK;
 }
 
@@ -704,7 +703,6 @@ void hj_impl::fill_pass_args(const hj_bunch* b, PassArgs& a) {
     const long double kPiL = 3.141592653589793238462643383279502884L;
     const long double h = 2.0L * kPiL / (long double)kRfTableSize;
     a.rf_table = b->rf_table;
-    a.Vs = b->rf_Vs;
     a.rf_inv_h = (double)(1.0L / h);
     a.rf_h_hi = (double)h;
     a.rf_h_lo = (double)(h - (long double)a.rf_h_hi);
@@ -835,7 +833,7 @@ extern "C" hj_status hj_bunch_advance(hj_bunch* b, int64_t turns) {
     }
     if (b->log_every > 0 && (b->turns_done + t + 1) % b->log_every == 0) {
       const int64_t rec = kLogHeader + (b->log_density ? b->B : 0);
-      HJ_TRY(launch_moments(b, 1, nullptr, nullptr));
+      HJ_TRY(launch_moments(b, 1, nullptr, nullptr, false));
       HJ_CUDA(ctx, launch_log_record(b->part_mom, b->nblk_m, b->n, b->ts,
                                      b->log_density ? b->hist : nullptr, b->B,
                                      b->d_log + (b->log_count % b->log_capacity) * rec,
@@ -884,7 +882,7 @@ extern "C" hj_status hj_bunch_observe(hj_bunch* b, double* d_z_out, double* d_dE
   HJ_TRY(launch_moments(b, 1, d_z_out, d_dE_out));
   double m[4];
   HJ_TRY(read_moments(b, m));
-  HJ_TRY(read_state(b));
+  HJ_TRY(state_status(b));
   fill_result(b, m, res);
   return HJ_OK;
 }
@@ -894,14 +892,12 @@ extern "C" hj_status hj_bunch_finish(hj_bunch* b, hj_result* res) {
   HJ_TRY(ctx_ok(b->ctx));
   HJ_TRY(launch_moments(b, 1, b->z, b->dE));
   // nothing is pending any more: the next pass must see a zero kick table
-  const int32_t zero = 0;
-  HJ_CUDA(b->ctx, cudaMemcpyAsync(&b->ts->pending, &zero, sizeof(int32_t),
-                                  cudaMemcpyHostToDevice, b->stream));
+  HJ_CUDA(b->ctx, cudaMemsetAsync(&b->ts->pending, 0, sizeof(int32_t), b->stream));
   if (b->potd)
     HJ_CUDA(b->ctx, cudaMemsetAsync(b->potd, 0, sizeof(double2) * ((size_t)b->B + 1), b->stream));
   double m[4];
   HJ_TRY(read_moments(b, m));
-  HJ_TRY(read_state(b));
+  HJ_TRY(state_status(b));
   fill_result(b, m, res);
   return HJ_OK;
 }

@@ -68,6 +68,36 @@ struct hj_batch {
 
 namespace {
 
+// Whether p is memory of the context's device.
+bool on_device(hj_ctx* ctx, const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+}
+
+// Enqueues bunch b's retirement: pending kick and re-centring, moments, turn state
+// to the host, the slot's state left without turns, and the particles into
+// z_out, dE_out (may be NULL), written by the same kernel where both are memory of
+// this device.  keep: the pool's copy is brought up to date as well.
+hj_status enqueue_take(hj_batch* bt, hj_bunch* b, double* z_out, double* dE_out, bool keep) {
+  hj_ctx* ctx = bt->ctx;
+  const bool direct =
+      !keep && z_out && dE_out && on_device(ctx, z_out) && on_device(ctx, dE_out);
+  const bool none = !keep && !z_out && !dE_out;
+  HJ_TRY(launch_moments(b, 1, direct ? z_out : none ? nullptr : b->z,
+                        direct ? dE_out : none ? nullptr : b->dE, true, true));
+  if (direct) return HJ_OK;
+  if (z_out)
+    HJ_CUDA(ctx, cudaMemcpyAsync(z_out, b->z, sizeof(double) * b->n, cudaMemcpyDefault, bt->stream));
+  if (dE_out)
+    HJ_CUDA(ctx, cudaMemcpyAsync(dE_out, b->dE, sizeof(double) * b->n, cudaMemcpyDefault,
+                                 bt->stream));
+  return HJ_OK;
+}
+
 hj_status batch_alloc_range(hj_batch* bt, int64_t n, int64_t* start, int64_t* cap) {
   return hj_ranges::take(bt->free_ranges, n, start, cap) ? HJ_OK : HJ_ERR_FULL;
 }
@@ -340,8 +370,11 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   p.turns = turns;
   double* dz = bt->pool_z + p.start;
   double* de = bt->pool_dE + p.start;
-  cudaError_t e;
-  if (z) {
+  cudaError_t e = cudaSuccess;
+  // from this device's memory the moments' kernel copies the particles as it reads them
+  const bool direct = z && on_device(ctx, z) && on_device(ctx, dE);
+  if (direct) {
+  } else if (z) {
     e = cudaMemcpyAsync(dz, z, sizeof(double) * n, cudaMemcpyDefault, bt->stream);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(de, dE, sizeof(double) * n, cudaMemcpyDefault, bt->stream);
@@ -355,7 +388,8 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   }
   p.b = new hj_bunch();
   hj_status s = bunch_create_begin(ctx, dz, de, n, params, wake, nbins, nullptr, seed,
-                                   (void*)bt->stream, p.b, bt->chunk, bt->cfg);
+                                   (void*)bt->stream, p.b, bt->chunk, bt->cfg, direct ? z : nullptr,
+                                   direct ? dE : nullptr);
   if (s == HJ_OK && p.b->nblk > bt->max_chunks) s = set_err(ctx, HJ_ERR_FULL, "chunk table full");
   if (s != HJ_OK) {
     batch_add_abort(bt, p);
@@ -370,21 +404,14 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
 }
 
 static hj_status batch_add_end(hj_batch* bt, PendingAdd& p, int64_t* id_out) {
-  hj_ctx* ctx = bt->ctx;
-  hj_status s = bunch_create_end(ctx, p.b, nullptr);
+  // the turn state goes into the batch's array, with this bunch's turn budget
+  hj_bunch* b = p.b;
+  b->ts = bt->d_ts + p.slot;         // the arena's own TurnState stays unused
+  b->turns_left = p.turns;
+  hj_status s = bunch_create_end(bt->ctx, b, nullptr);
   if (s != HJ_OK) {
     batch_add_abort(bt, p);
     return s;
-  }
-  // move the turn state into the batch's array, with this bunch's turn budget
-  hj_bunch* b = p.b;
-  b->h_ts->turns_left = p.turns;
-  b->ts = bt->d_ts + p.slot;         // the arena's own TurnState stays unused
-  cudaError_t e = cudaMemcpyAsync(b->ts, b->h_ts, sizeof(TurnState), cudaMemcpyHostToDevice,
-                                  bt->stream);   // ordered before the next turn's kernels
-  if (e != cudaSuccess) {
-    batch_add_abort(bt, p);
-    return set_err(ctx, HJ_ERR_CUDA, "turn state upload failed: %s", cudaGetErrorString(e));
   }
   BatchMember m;
   m.id = bt->next_id++;
@@ -507,24 +534,9 @@ extern "C" hj_status hj_batch_take_many(hj_batch* bt, int32_t count, const int64
   }
   // one round trip for all: pending kick and re-centring in place, moments,
   // turn state, copies out, and every slot's state set to "no turns left"
-  TurnState dead{};
-  dead.turns_left = 0;
-  for (int k = 0; k < count; ++k) {
-    hj_bunch* b = bs[k];
-    HJ_TRY(launch_moments(b, 1, b->z, b->dE));
-    HJ_CUDA(ctx, cudaMemcpyAsync(b->h_mom, b->part_mom, sizeof(double) * 4 * b->nblk_m,
-                                 cudaMemcpyDeviceToHost, bt->stream));
-    HJ_CUDA(ctx, cudaMemcpyAsync(b->h_ts, b->ts, sizeof(TurnState), cudaMemcpyDeviceToHost,
-                                 bt->stream));
-    if (z_out && z_out[k])
-      HJ_CUDA(ctx, cudaMemcpyAsync(z_out[k], b->z, sizeof(double) * b->n, cudaMemcpyDefault,
-                                   bt->stream));
-    if (dE_out && dE_out[k])
-      HJ_CUDA(ctx, cudaMemcpyAsync(dE_out[k], b->dE, sizeof(double) * b->n, cudaMemcpyDefault,
-                                   bt->stream));
-    HJ_CUDA(ctx, cudaMemcpyAsync(b->ts, &dead, sizeof(TurnState), cudaMemcpyHostToDevice,
-                                 bt->stream));
-  }
+  for (int k = 0; k < count; ++k)
+    HJ_TRY(enqueue_take(bt, bs[k], z_out ? z_out[k] : nullptr, dE_out ? dE_out[k] : nullptr,
+                        corr_out != nullptr));
   HJ_CUDA(ctx, cudaStreamSynchronize(bt->stream));
   hj_status st = HJ_OK;
   std::vector<double> mean_z(count), mean_e(count);
@@ -631,20 +643,7 @@ extern "C" hj_status hj_batch_take(hj_batch* bt, int64_t id, double* z_out, doub
   // one round trip: pending kick and re-centring applied in place, moments
   // and turn state read, particles copied out, and the slot's state set to
   // "no turns left" for the kernels
-  HJ_TRY(launch_moments(b, 1, b->z, b->dE));
-  HJ_CUDA(ctx, cudaMemcpyAsync(b->h_mom, b->part_mom, sizeof(double) * 4 * b->nblk_m,
-                               cudaMemcpyDeviceToHost, bt->stream));
-  HJ_CUDA(ctx, cudaMemcpyAsync(b->h_ts, b->ts, sizeof(TurnState), cudaMemcpyDeviceToHost,
-                               bt->stream));
-  if (z_out)
-    HJ_CUDA(ctx, cudaMemcpyAsync(z_out, b->z, sizeof(double) * b->n, cudaMemcpyDefault, bt->stream));
-  if (dE_out)
-    HJ_CUDA(ctx, cudaMemcpyAsync(dE_out, b->dE, sizeof(double) * b->n, cudaMemcpyDefault,
-                                 bt->stream));
-  TurnState dead{};
-  dead.turns_left = 0;
-  HJ_CUDA(ctx, cudaMemcpyAsync(b->ts, &dead, sizeof(TurnState), cudaMemcpyHostToDevice,
-                               bt->stream));
+  HJ_TRY(enqueue_take(bt, b, z_out, dE_out, false));
   HJ_CUDA(ctx, cudaStreamSynchronize(bt->stream));
   double mom[4];
   sum_moments(b, mom);

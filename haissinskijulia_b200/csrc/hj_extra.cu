@@ -121,7 +121,7 @@ extern "C" hj_status hj_bunch_checkpoint(hj_bunch* b, double* d_z_out, double* d
   HJ_TRY(launch_moments(b, 1, d_z_out, d_dE_out));
   double m[4];
   HJ_TRY(read_moments(b, m));
-  HJ_TRY(read_state(b));
+  HJ_TRY(state_status(b));
   out->turn = b->h_ts->turn;
   out->E0 = b->h_ts->cur.E0;
   out->sigma_E0_initial = b->sigma_E0_initial;

@@ -148,7 +148,19 @@ void host_wake_powers(const hj_wake& w, double cJ, double step, int64_t J, doubl
     out[1] = (double)(m * sinl(x * s));
   };
   const long double d = (long double)step;
-  for (int k = 0; k < npw; ++k) put(-d * (long double)(int64_t(1) << k), pw[k]);
+  // every fourth power from its exponent, the next three by squaring (at most 8
+  // extended-precision roundings)
+  for (int k = 0; k < npw; k += 4) {
+    const long double x = -d * (long double)(int64_t(1) << k), m = expl(x * rate);
+    long double re = m * cosl(x * s), im = m * sinl(x * s);
+    for (int q = k; q < npw && q < k + 4; ++q) {
+      pw[q][0] = (double)re;
+      pw[q][1] = (double)im;
+      const long double t = re * re - im * im;
+      im = 2.0L * re * im;
+      re = t;
+    }
+  }
   put(-d * (long double)(J + 1), tau);
   // F e^{c_J (1/cτ + i s)} (1 - i a): its real part is F e^{c/cτ} (cos + a sin)
   const long double m = (long double)w.wake_factor * expl((long double)cJ * rate);
@@ -184,33 +196,25 @@ double host_particle_factor(int64_t n, double population) {
   return (1e11 / den) * (double)n;
 }
 
-// RF kick table of the fused pass: (V sin θm, V cos θm), θm = ϕs - 2π m / M,
-// m = 0..M-1, in extended precision and rounded once.
-// The extended-precision (sin θm, cos θm) of a phase are kept per (ϕs, M):
-// bunches of a voltage scan share ϕs.
-void host_rf_table(double V, double phi_s, int64_t M, double* tab_interleaved) {
-  static std::mutex mu;
-  static std::map<std::pair<uint64_t, int64_t>, std::vector<long double>> cache;
-  uint64_t bits;
-  std::memcpy(&bits, &phi_s, sizeof(bits));
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find({bits, M});
-  if (it == cache.end()) {
-    if (cache.size() >= 64) cache.clear();
-    const long double kPiL = 3.141592653589793238462643383279502884L;
-    std::vector<long double> sc(2 * (size_t)M);
-    for (int64_t m = 0; m < M; ++m) {
-      const long double a = (long double)phi_s - 2.0L * kPiL * (long double)m / (long double)M;
-      sc[2 * m] = sinl(a);
-      sc[2 * m + 1] = cosl(a);
-    }
-    it = cache.insert({{bits, M}, std::move(sc)}).first;
+namespace {
+void split(long double x, double* hi_lo) {
+  hi_lo[0] = (double)x;
+  hi_lo[1] = (double)(x - (long double)hi_lo[0]);
+}
+}  // namespace
+
+void host_rf_unit(int M, double (*unit)[4]) {
+  const long double kPiL = 3.141592653589793238462643383279502884L;
+  for (int m = 0; m < M; ++m) {
+    const long double a = 2.0L * kPiL * (long double)m / (long double)M;
+    split(cosl(a), unit[m]);
+    split(sinl(a), unit[m] + 2);
   }
-  const std::vector<long double>& sc = it->second;
-  for (int64_t m = 0; m < M; ++m) {
-    tab_interleaved[2 * m] = (double)((long double)V * sc[2 * m]);
-    tab_interleaved[2 * m + 1] = (double)((long double)V * sc[2 * m + 1]);
-  }
+}
+
+void host_sincos(double phi, double out[4]) {
+  split(sinl((long double)phi), out);
+  split(cosl((long double)phi), out + 2);
 }
 
 // exp(-2πik/P), k = 0..P-1, interleaved (re, im), in extended precision and

@@ -27,7 +27,10 @@ bool host_uniform_centers(const double* centers, int64_t B, int64_t* J, double* 
 // Particle factor of the wake current (src/evolution.jl:373-384).
 double host_particle_factor(int64_t n, double population);
 void host_twiddles(int64_t P, double* tw_interleaved);
-void host_rf_table(double V, double phi_s, int64_t M, double* tab_interleaved);
+// cos and sin of 2π m / M, m < M, each as a sum of two doubles: (cos hi, lo, sin hi, lo).
+void host_rf_unit(int M, double (*unit)[4]);
+// sin and cos of phi likewise: (sin hi, lo, cos hi, lo).
+void host_sincos(double phi, double out[4]);
 // Tables of the device's Float64 normals: a 2048-layer ziggurat for the
 // density f(x) = exp(-x²/2), x >= 0 (G. Marsaglia and W. W. Tsang, "The
 // Ziggurat Method for Generating Random Variables", J. Stat. Softw. 5(8),

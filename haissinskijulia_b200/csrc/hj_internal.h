@@ -71,9 +71,9 @@ struct PassArgs {
   // physics constants of the run
   double V, phi_s, inv_mass, alpha_c, two_pi_h;
   // RF kick: x = z k = m h + t, h = 2π / kRfTableSize (h_hi + h_lo), and
-  // rf_table[m mod kRfTableSize] = (V sin(ϕs - m h), V cos(ϕs - m h)); Vs = V sin ϕs
+  // rf_table[m mod kRfTableSize] = (V sin(ϕs - m h), V cos(ϕs - m h))
   const double2* rf_table;
-  double rf_inv_h, rf_h_hi, rf_h_lo, Vs;
+  double rf_inv_h, rf_h_hi, rf_h_lo;
   PhiloxKeys philox;       // Philox-4x32 round keys of the bunch's seed
   int32_t update_eta, update_E0, sr, qe_mode;
   int32_t cfg;             // thread layout (kNumPassCfgs)
@@ -163,19 +163,20 @@ struct ScanArgs {
 // Moments of (z, dE) per block: [Σz, Σz², ΣdE, ΣdE²], optionally after
 // applying a pending kick/re-centring (flush) and writing the result.
 struct FlushArgs {
-  double* z;          // state
-  double* dE;
+  const double* z;    // state
+  const double* dE;
   int64_t n;
-  const TurnState* ts;
+  TurnState* ts;
   const double2* potd;
   int32_t B;
   int32_t use_wake, update_E0;
-  double c1, cB, inv_cstep;
   double e0, inv_estep;   // kick-table cell coordinate
   int32_t apply;      // 1: apply pending ops
   double* z_out;      // destination (may alias z/dE); NULL -> not written
   double* dE_out;
-  double* part;       // [grid][4]
+  double* part;       // [grid][4], in device or pinned host memory
+  TurnState* ts_out;  // pinned host copy of the turn state (NULL: none)
+  int32_t retire;     // 1: leave the turn state without turns to run
 };
 
 // ---- launchers (hj_track.cu) ----
@@ -202,6 +203,12 @@ cudaError_t launch_batch_pass(const PassArgs* d_bunches, const BatchChunk* d_chu
 int batch_blocks_per_sm(int max_B, int qe_mode, int use_wake, int cfg);
 cudaError_t launch_sum_parts(const double* part, int nblk, double* out, cudaStream_t st);
 cudaError_t launch_flush(const FlushArgs& a, int grid, cudaStream_t st);
+// Set-up of a new bunch's device memory: `zero_bytes` from `zero` (a multiple of 16)
+// cleared, the RF table (V sin θm, V cos θm), θm = ϕs - 2π m / kRfTableSize, and its
+// turn state.  sincos: sin ϕs and cos ϕs, each as a sum of two doubles.
+cudaError_t launch_bunch_setup(void* zero, size_t zero_bytes, double2* rf_table, double V,
+                               const double sincos[4], TurnState* ts, const TurnState& t,
+                               cudaStream_t st);
 // generate_particles on the device (covariance sample, correlated bunch, two-pass std)
 cudaError_t launch_gen_sample_cov(uint64_t seed, int64_t S, double mu_z, double sz, double mu_E,
                                   double sE, double* out, cudaStream_t st);

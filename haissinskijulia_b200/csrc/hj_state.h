@@ -100,12 +100,11 @@ struct hj_bunch {
   double2* twP = nullptr;
   int64_t* defer_q = nullptr;             // [nblk][warps][kDeferStage] (Float64 normals)
   double2* rf_table = nullptr;             // [kRfTableSize] RF kick table of the pass
-  double rf_Vs = 0;                        // its entry 0: V sin ϕs
+  int64_t turns_left = INT64_MAX;          // turns to run (a batch member's budget)
   double* part_sum = nullptr;
   double* part_mom = nullptr;
   double* h_mom = nullptr;    // pinned
   TurnState* h_ts = nullptr;  // pinned
-  double* h_rf = nullptr;     // pinned staging of the RF table
   // the buffers above are carved from one device block and one pinned block
   // of the context's cache; without uniform centres twP is the context's
   // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, acc and hist are the first zero_bytes of the
@@ -197,8 +196,13 @@ hj_status check_grid(hj_ctx* ctx, const hj_grid* g);
 // Moments of a bunch: per-block sums on the device, summed on the host in
 // block order.
 void sum_moments(const hj_bunch* b, double m[4]);
+// launch_moments enqueues them (with apply: after the pending kick and re-centring,
+// and with outputs the particles then), into device memory or, to_host, into the
+// bunch's pinned memory together with the turn state; read_moments waits for the
+// latter.  retire: the turn state is left without turns to run.
+hj_status launch_moments(hj_bunch* b, int apply, double* z_out, double* dE_out, bool to_host = true,
+                         bool retire = false);
 hj_status read_moments(hj_bunch* b, double m[4]);
-hj_status launch_moments(hj_bunch* b, int apply, double* z_out, double* dE_out);
 hj_status state_status(hj_bunch* b);
 hj_status read_state(hj_bunch* b);
 int default_pass_layout(int B, int64_t n);
@@ -212,7 +216,8 @@ cudaError_t set_kernel_attributes(hj_ctx* ctx);
 hj_status bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
                              const hj_params* params, const hj_wake* wake, int64_t nbins,
                              const hj_grid* grid, uint64_t seed, void* stream, hj_bunch* b,
-                             int64_t chunk = 0, int cfg = -1);
+                             int64_t chunk = 0, int cfg = -1, const double* z_src = nullptr,
+                             const double* dE_src = nullptr);
 // cp: continue from a checkpoint (its turn, E0 and initial spreads)
 hj_status bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* grid,
                            const hj_checkpoint* cp = nullptr);

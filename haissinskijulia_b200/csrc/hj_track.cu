@@ -781,8 +781,9 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       smem_raw + (a.zig ? kPassTableBytes : kRfTableSize * sizeof(double2)));
   uint32_t* const h_cnt = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
   uint32_t* const h_lo = h_cnt + nw;
-  for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) copy16_async(s_rf + i, a.rf_table + i);
   grid_dependency_wait();
+  // (the RF table too: a new bunch's is written by the kernel before its first pass)
+  for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) copy16_async(s_rf + i, a.rf_table + i);
   grid_launch_dependents();   // the bins step may be scheduled: it reads the turn state too
   TurnState* ts = a.ts;
   const bool done = ts->turns_left <= 0;      // a batch member's budget is spent
@@ -797,7 +798,6 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   const int64_t turn = ts->turn;
 
   FusedConst c;
-  c.Vs = a.Vs;
   c.rf_inv_h = a.rf_inv_h;
   c.rf_h_hi = a.rf_h_hi;
   c.rf_h_lo = a.rf_h_lo;
@@ -851,6 +851,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   }
   copies_wait();
   __syncthreads();
+  c.Vs = s_rf[0].x;
   // the counters indexed by absolute half cell and cell (valid inside the window)
   uint32_t* const s_cnt = h_cnt - (N32 ? 2 * kw.w0 : kw.w0);
   uint32_t* const s_lo = h_lo - kw.w0;
@@ -1046,43 +1047,140 @@ __global__ void __launch_bounds__(THREADS, MINB)
 }
 
 // Pending kick + re-centring (optional), copy-out (optional) and the moments
-// [Σz, Σz², ΣdE, ΣdE²] per block.
+// [Σz, Σz², ΣdE, ΣdE²] per block; block 0 also hands the turn state to the host.  Bound
+// by HBM on large bunches (48 bytes per particle with the copy-out) and by latency
+// on small ones: four particles a thread with 32-byte accesses where the arrays
+// are aligned, two such groups in flight (a bunch of 1e5: 11 us with one particle
+// at a time, 5 us so).
+__device__ __forceinline__ void ld_group(const double* p, bool vec, double v[4]) {
+  if (vec) {
+    ld4(p, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = p[k];
+  }
+}
+__device__ __forceinline__ void st_group(double* p, bool vec, const double v[4]) {
+  if (vec) {
+    st4(p, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = v[k];
+  }
+}
+
 __global__ void __launch_bounds__(kTrackThreads) k_flush(FlushArgs a) {
   const bool apply = a.apply && a.ts && a.ts->pending;
   const double pmean = apply ? a.ts->pending_mean : 0.0;
-  GridConst g{a.B, a.e0, 0.0, a.inv_estep, a.c1, a.cB, a.inv_cstep,
-              kick_offset(a.e0, a.inv_estep)};
+  GridConst g{a.B, a.e0, 0.0, a.inv_estep, 0.0, 0.0, 0.0, kick_offset(a.e0, a.inv_estep)};
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-    double z = a.z[i], e = a.dE[i];
+  auto one = [&](double z, double& e) {
     if (apply) {
       if (a.use_wake) e = e - wake_kick(z, g, a.potd);
       if (a.update_E0) e = __dsub_rn(e, pmean);
     }
-    if (a.z_out) a.z_out[i] = z;
-    if (a.dE_out) a.dE_out[i] = e;
     s0 += z;
     s1 = fma(z, z, s1);
     s2 += e;
     s3 = fma(e, e, s3);
+  };
+  const bool vin = (((uintptr_t)a.z | (uintptr_t)a.dE) & 31) == 0;
+  const bool vout = (((uintptr_t)a.z_out | (uintptr_t)a.dE_out) & 31) == 0;
+  double* const z_out = a.z_out == a.z ? nullptr : a.z_out;   // z is unchanged in place
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t ng = a.n / 4;
+#pragma unroll 2
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < ng; q += stride) {
+    double z[4], e[4];
+    ld_group(a.z + 4 * q, vin, z);
+    ld_group(a.dE + 4 * q, vin, e);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) one(z[k], e[k]);
+    if (z_out) st_group(z_out + 4 * q, vout, z);
+    if (a.dE_out) st_group(a.dE_out + 4 * q, vout, e);
+  }
+  if (blockIdx.x == 0 && (int64_t)threadIdx.x < a.n - 4 * ng) {
+    const int64_t i = 4 * ng + threadIdx.x;
+    const double z = a.z[i];
+    double e = a.dE[i];
+    one(z, e);
+    if (z_out) z_out[i] = z;
+    if (a.dE_out) a.dE_out[i] = e;
   }
   __shared__ double red[kTrackThreads / 32][4];
   block_sum4<kTrackThreads>(s0, s1, s2, s3, a.part + (size_t)blockIdx.x * 4, red);
+  if (blockIdx.x == 0) {
+    if (a.ts_out) {
+      const int* src = reinterpret_cast<const int*>(a.ts);
+      for (int k = threadIdx.x; k < (int)(sizeof(TurnState) / sizeof(int)); k += blockDim.x)
+        reinterpret_cast<int*>(a.ts_out)[k] = src[k];
+    }
+    __syncthreads();
+    if (a.retire && threadIdx.x == 0) a.ts->turns_left = 0;
+  }
+}
+
+// cos and sin of m h, h = 2π / kRfTableSize, each as a sum of two doubles (cos hi, lo,
+// sin hi, lo), filled when the kernels are prepared.
+__device__ double g_rf_unit[kRfTableSize][4];
+
+// a b as a sum of two doubles, a and b being such sums.
+__device__ __forceinline__ double2 mul_dd(double ah, double al, double bh, double bl) {
+  const double p = __dmul_rn(ah, bh);
+  return make_double2(p, fma(ah, bh, -p) + fma(ah, bl, al * bh));
+}
+// x + y, |x| and |y| arbitrary (two-sum).
+__device__ __forceinline__ double2 add_dd(double2 x, double2 y) {
+  const double s = __dadd_rn(x.x, y.x), t = __dsub_rn(s, x.x);
+  const double e = __dadd_rn(__dsub_rn(x.x, __dsub_rn(s, t)), __dsub_rn(y.x, t));
+  return make_double2(s, e + (x.y + y.y));
+}
+
+// See launch_bunch_setup: one launch instead of a host table (128 extended-precision
+// sines), two copies and a memset per admitted bunch.
+struct SetupArgs {
+  uint4* zero;
+  int64_t zero_words;
+  double2* rf_table;
+  double V;
+  double sh, sl, ch, cl;
+  TurnState* ts;
+  TurnState t;
+};
+__global__ void __launch_bounds__(256) k_bunch_setup(SetupArgs a) {
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = i0; i < a.zero_words; i += (int64_t)gridDim.x * blockDim.x)
+    a.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (i0 < kRfTableSize) {
+    // sin and cos of ϕs - m h by angle addition, times V, rounded once
+    const double* u = g_rf_unit[i0];
+    const double2 sn = add_dd(mul_dd(a.sh, a.sl, u[0], u[1]), mul_dd(-a.ch, -a.cl, u[2], u[3]));
+    const double2 cs = add_dd(mul_dd(a.ch, a.cl, u[0], u[1]), mul_dd(a.sh, a.sl, u[2], u[3]));
+    const double2 vs = mul_dd(a.V, 0.0, sn.x, sn.y), vc = mul_dd(a.V, 0.0, cs.x, cs.y);
+    a.rf_table[i0] = make_double2(vs.x + vs.y, vc.x + vc.y);
+  }
+  if (i0 == 0) *a.ts = a.t;
 }
 
 // One record of a bunch's turn log: [turn, E0, σ_z, σ_E, mean z, mean ΔE, wake
 // current, particles in the bins] of the state after the last completed turn
 // (moments from k_flush with the pending kick applied), then the B bin
 // counts of that turn when `counts` is given.
-__global__ void k_log_record(const double* __restrict__ part, int nblk, int64_t n,
+__global__ void __launch_bounds__(512) k_log_record(const double* __restrict__ part, int nblk, int64_t n,
                              const TurnState* __restrict__ ts,
                              const unsigned long long* __restrict__ counts, int B,
                              double* __restrict__ rec) {
-  if (threadIdx.x == 0) {
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = 0; b < nblk; ++b)
-      for (int k = 0; k < 4; ++k) s[k] += part[(size_t)b * 4 + k];
+  __shared__ double red[16][4];
+  __shared__ double s[4];
+  if (blockIdx.x == 0) {       // the blocks' moments, in a fixed order
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < nblk; b += 512)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] += part[(size_t)b * 4 + k];
+    block_sum4<512>(v[0], v[1], v[2], v[3], s, red);
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     const double nd = n > 0 ? (double)n : 1.0;
     rec[0] = (double)(ts->turn - 1);
     rec[1] = ts->cur.E0;
@@ -1094,7 +1192,8 @@ __global__ void k_log_record(const double* __restrict__ part, int nblk, int64_t 
     rec[7] = ts->last_n_in;
   }
   if (counts)
-    for (int i = threadIdx.x; i < B; i += blockDim.x) rec[kLogHeader + i] = (double)counts[i];
+    for (int i = blockIdx.x * 512 + threadIdx.x; i < B; i += gridDim.x * 512)
+      rec[kLogHeader + i] = (double)counts[i];
 }
 
 // NGP histogram only (hj_histogram, hj_apply_wakefield).
@@ -1501,6 +1600,9 @@ cudaError_t prepare_track_kernels(int max_smem) {
     std::unique_ptr<NormalTables> tab(new NormalTables);   // 48 KB: not on the stack
     host_normal_tables(tab.get());
     cudaError_t e = cudaMemcpyToSymbol(g_normal, tab.get(), sizeof(NormalTables));
+    double unit[kRfTableSize][4];
+    host_rf_unit(kRfTableSize, unit);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_rf_unit, unit, sizeof(unit));
     if (e != cudaSuccess) return e;
   }
   for (int w = 0; w < 2; ++w)
@@ -1583,7 +1685,7 @@ cudaError_t launch_sum_parts(const double* part, int nblk, double* out, cudaStre
 cudaError_t launch_log_record(const double* part, int nblk, int64_t n, const TurnState* ts,
                               const unsigned long long* counts, int B, double* rec,
                               cudaStream_t st) {
-  k_log_record<<<1, 256, 0, st>>>(part, nblk, n, ts, counts, B, rec);
+  k_log_record<<<counts ? 8 : 1, 512, 0, st>>>(part, nblk, n, ts, counts, B, rec);
   return cudaGetLastError();
 }
 
@@ -1615,6 +1717,16 @@ cudaError_t launch_cor_parts(const double* x, const double* y, int64_t n, double
 
 cudaError_t launch_flush(const FlushArgs& a, int grid, cudaStream_t st) {
   k_flush<<<grid, kTrackThreads, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_bunch_setup(void* zero, size_t zero_bytes, double2* rf_table, double V,
+                               const double sincos[4], TurnState* ts, const TurnState& t,
+                               cudaStream_t st) {
+  SetupArgs a{(uint4*)zero, (int64_t)(zero_bytes / 16), rf_table, V,
+              sincos[0], sincos[1], sincos[2], sincos[3], ts, t};
+  const int64_t blocks = std::min<int64_t>((a.zero_words + 1023) / 1024, 148);
+  k_bunch_setup<<<(int)std::max<int64_t>(blocks, 1), 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 
