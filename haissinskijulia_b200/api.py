@@ -770,13 +770,18 @@ class Batch:
         n = self._size(bid)
         z = np.empty(n) if copy_out else None
         dE = np.empty(n) if copy_out else None
+        return z, dE, self._take_into(bid, z, dE)
+
+    def _take_into(self, bid: int, z: Optional[np.ndarray],
+                   dE: Optional[np.ndarray]) -> EvolveResult:
+        """take() into the given contiguous arrays (None: not copied out)."""
         r = HjResult()
         live = self._live()
         rc = self.ctx._lib.hj_batch_take(
-            self.handle, int(bid), z.ctypes.data_as(ctypes.c_void_p) if copy_out else None,
-            dE.ctypes.data_as(ctypes.c_void_p) if copy_out else None, ctypes.byref(r))
+            self.handle, int(bid), z.ctypes.data_as(ctypes.c_void_p) if z is not None else None,
+            dE.ctypes.data_as(ctypes.c_void_p) if dE is not None else None, ctypes.byref(r))
         self._forget([bid], rc, live)
-        return z, dE, EvolveResult.from_c(r)
+        return EvolveResult.from_c(r)
 
     def _live(self) -> int:
         """Bunches the library holds in this batch (hj_batch_stats, host only)."""

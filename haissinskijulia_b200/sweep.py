@@ -27,6 +27,7 @@ batched bins step per turn, turn blocks replayed from a CUDA graph.
 from __future__ import annotations
 
 import math
+import threading
 import time
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional
@@ -120,6 +121,29 @@ class Tuning:
     resident: bool = False      # resident blocks on a chunk queue, or one block per chunk
 
 
+class _Outputs:
+    """Host arrays for the final particles of all points, slices of one block per
+    coordinate.  Fresh pages cost more to fault in than the copies into them (40
+    points, 64 MB: 20 ms one array each, 7 ms as large blocks, which get huge
+    pages), so a thread touches them while the GPU runs the first turns."""
+
+    def __init__(self, points: List[Point]):
+        self._first = np.concatenate([[0], np.cumsum([p.n for p in points])])
+        total = int(self._first[-1])
+        self._z, self._dE = np.empty(total), np.empty(total)
+        self._thread = threading.Thread(target=self._touch, daemon=True)
+        self._thread.start()
+
+    def _touch(self) -> None:
+        for a in (self._z, self._dE):
+            a[::512] = 0.0                      # one double a page
+
+    def of(self, i: int):
+        self._thread.join()
+        s = slice(int(self._first[i]), int(self._first[i + 1]))
+        return self._z[s], self._dE[s]
+
+
 def run_batched(ctx: Context, points: List[Point], *, pool_particles: Optional[int] = None,
                 max_bunches: Optional[int] = None, tuning: Tuning = Tuning(),
                 block_turns: int = 64, copy_out: bool = False) -> List[Solve]:
@@ -134,6 +158,7 @@ def run_batched(ctx: Context, points: List[Point], *, pool_particles: Optional[i
     pending = list(range(len(points)))
     live: Dict[int, int] = {}
     out: List[Optional[Solve]] = [None] * len(points)
+    store = _Outputs(points) if copy_out and points else None
     t0 = time.perf_counter()
     try:
         while pending or live:
@@ -154,9 +179,10 @@ def run_batched(ctx: Context, points: List[Point], *, pool_particles: Optional[i
             bt.advance(block_turns)
             for bid in bt.poll():
                 i = live.pop(bid)
-                z, dE, r = bt.take(bid, copy_out=copy_out)
                 s = out[i]
-                s.result, s.z, s.dE = r, z, dE
+                if store is not None:
+                    s.z, s.dE = store.of(i)
+                s.result = bt._take_into(bid, s.z, s.dE)
                 s.finished = time.perf_counter() - t0
     finally:
         bt.close()
