@@ -431,7 +431,7 @@ extern "C" void hj_bunch_destroy(hj_bunch* b) {
 // bunch_create_end (after the stream has reached them) builds the grid, the
 // wake tables, the RF table and the turn state.
 // chunk > 0: a batch member, whose partial slots are its chunks of
-// member_chunk(n, chunk) particles (the batch's chunk table) instead of one per block of the grid;
+// `chunk` particles (the batch's chunk table) instead of one per block of the grid;
 // cfg >= 0 pins the pass layout.
 hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, int64_t n,
                                       const hj_params* params, const hj_wake* wake,
@@ -481,7 +481,7 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
   b->cfg = cfg >= 0 ? cfg : auto_pass_layout(ctx->pass_layout, b->B, n);
   if (chunk > 0) {
     b->batch_member = true;
-    b->chunk = member_chunk(n, chunk);
+    b->chunk = chunk;
     b->nblk = (int)std::max<int64_t>((n + b->chunk - 1) / b->chunk, 1);
   } else {
     const int bps = track_blocks_per_sm(b->B, b->qe_mode, b->use_wake, b->cfg);
@@ -757,13 +757,16 @@ void hj_impl::fill_scan_args(const hj_bunch* b, ScanArgs& g) {
   std::copy(b->wake_pw, b->wake_pw + kScanPowers, g.pw);
 }
 
-cudaError_t hj_impl::launch_bunch_pass(const hj_bunch* b, const PassArgs& a) {
+cudaError_t hj_impl::launch_bunch_pass(hj_bunch* b, const PassArgs& a) {
   if (b->shard) {
     cudaError_t e = cudaMemsetAsync(b->acc, 0, sizeof(unsigned long long) * (3 * (size_t)b->B + 2),
                                     b->stream);
     if (e != cudaSuccess) return e;
   }
-  return launch_track_pass(a, b->nblk, b->stream);
+  // the first pass follows the kernel that set the bunch up
+  const bool overlap = b->passed;
+  b->passed = true;
+  return launch_track_pass(a, b->nblk, b->stream, overlap);
 }
 
 cudaError_t hj_impl::launch_bunch_bins(const hj_bunch* b) {

@@ -231,10 +231,10 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->max_B = max_nbins;
   bt->cfg = auto_pass_layout(layout, max_nbins, pool_particles);
   bt->pool_n = (pool_particles + 3) / 4 * 4;
-  // a member has at most n / chunk + 1 chunks, or kMemberBlocks smaller ones
+  // a member has at most n / chunk + 1 chunks, or member_blocks smaller ones
   // (member_chunk)
   bt->max_chunks = (int)std::min<int64_t>(
-      bt->pool_n / chunk + (kMemberBlocks + 1) * (int64_t)max_bunches + 1, INT32_MAX);
+      bt->pool_n / chunk + (member_blocks(max_bunches) + 1) * (int64_t)max_bunches + 1, INT32_MAX);
   HJ_CUDA(ctx, cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking));
   // the pool and the tables: one device and one pinned block of the context's cache
   const size_t nb = (size_t)max_bunches, nc = (size_t)bt->max_chunks;
@@ -388,7 +388,7 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   }
   p.b = new hj_bunch();
   hj_status s = bunch_create_begin(ctx, dz, de, n, params, wake, nbins, nullptr, seed,
-                                   (void*)bt->stream, p.b, bt->chunk, bt->cfg, direct ? z : nullptr,
+                                   (void*)bt->stream, p.b, member_chunk(n, bt->chunk, bt->max_bunches), bt->cfg, direct ? z : nullptr,
                                    direct ? dE : nullptr);
   if (s == HJ_OK && p.b->nblk > bt->max_chunks) s = set_err(ctx, HJ_ERR_FULL, "chunk table full");
   if (s != HJ_OK) {

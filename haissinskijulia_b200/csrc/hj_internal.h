@@ -193,7 +193,9 @@ struct PassWindows {
   int32_t hot, kick;
 };
 PassWindows track_windows(int B, int cfg, bool zig);
-cudaError_t launch_track_pass(const PassArgs& a, int grid, cudaStream_t st);
+// overlap: the pass's set-up may run before the previous kernel has finished, which
+// must not have written the RF table.
+cudaError_t launch_track_pass(const PassArgs& a, int grid, cudaStream_t st, bool overlap);
 // Batched pass over a chunk table (*d_n_chunks entries live, grid max_chunks).
 cudaError_t launch_batch_pass(const PassArgs* d_bunches, const BatchChunk* d_chunks,
                               const int32_t* d_n_chunks, int max_chunks, int max_B, int wake,

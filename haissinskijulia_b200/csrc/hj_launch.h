@@ -57,18 +57,24 @@ inline int resolve_pass_request(int r, int automatic) {
   return r;
 }
 
-// Particles per block of a batch member of n particles in a batch created with
-// `chunk` particles per block: about kMemberBlocks blocks of kMinChunk to 2 chunk
-// particles.  A block costs about 8 us beside its particles (1 us a thousand), so
-// large bunches take large blocks, while a batch of few or small bunches must not
-// wait for one block each.  Measured, us a turn, against `chunk` = 65536 for all:
-// 256 bunches of 1e4 to 2e6 874 -> 861, 32 bunches of 1e6 312 -> 278, 16 served
-// ones (1.6e6 particles) 86 -> 67, 64 of 1e4 to 5e4 62 -> 37.  A function of n and
-// chunk alone: a bunch's sums do not depend on the bunches that share its batch.
-constexpr int64_t kMemberBlocks = 8;
+// Particles per block of a batch member of n particles, in a batch of `slots`
+// bunches created with `chunk` particles per block: member_blocks(slots) blocks of
+// kMinChunk to 2 chunk particles.  A block costs about 8 us beside its particles (1
+// us a thousand), so large bunches take large blocks, while a batch of few or
+// small bunches must not wait for one block each: eight, or what fills the SMs
+// twice when every slot is taken.  Measured, us a turn, against `chunk` = 65536 for
+// all: 256 bunches of 1e4 to 2e6 874 -> 861, 32 bunches of 1e6 312 -> 278, 64 of 1e4
+// to 5e4 62 -> 37, 16 served ones (1.6e6 particles) 86 -> 67 with eight blocks.
+// A function of n and of how the batch was created: a bunch's sums do not depend
+// on the bunches that share it.
 constexpr int64_t kMinChunk = 16384;
-inline int64_t member_chunk(int64_t n, int64_t chunk) {
-  int64_t c = (n + kMemberBlocks - 1) / kMemberBlocks;
+inline int64_t member_blocks(int64_t slots) {
+  const int64_t b = 2 * 148 / (slots > 0 ? slots : 1);
+  return b > 8 ? b : 8;
+}
+inline int64_t member_chunk(int64_t n, int64_t chunk, int64_t slots) {
+  const int64_t blocks = member_blocks(slots);
+  int64_t c = (n + blocks - 1) / blocks;
   c = (c + 127) / 128 * 128;                       // whole warps of four-particle groups
   if (c < kMinChunk) c = kMinChunk;
   int64_t most = 2 * chunk;

@@ -109,6 +109,7 @@ struct hj_bunch {
   // of the context's cache; without uniform centres twP is the context's
   // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, acc and hist are the first zero_bytes of the
   // arena's histogram part
+  bool passed = false;                    // a pass has been enqueued
   bool batch_member = false;
   int64_t chunk = 0;                      // a member's particles per block of the pass
   void* tables = nullptr;
@@ -231,7 +232,7 @@ void fill_scan_args(const hj_bunch* b, ScanArgs& g);
 // Enqueues the particle pass of bunch b with its arguments a.  A shard's
 // accumulators, which its caller may read until the next pass, are cleared here;
 // a whole bunch's by its bins step.
-cudaError_t launch_bunch_pass(const hj_bunch* b, const PassArgs& a);
+cudaError_t launch_bunch_pass(hj_bunch* b, const PassArgs& a);
 // Enqueues the bins step of bunch b: the suffix scan, or the FFT where the
 // centres are not uniform.
 cudaError_t launch_bunch_bins(const hj_bunch* b);

@@ -781,10 +781,19 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       smem_raw + (a.zig ? kPassTableBytes : kRfTableSize * sizeof(double2)));
   uint32_t* const h_cnt = reinterpret_cast<uint32_t*>(s_win + ((win + 1) & ~1));
   uint32_t* const h_lo = h_cnt + nw;
-  grid_dependency_wait();
-  // (the RF table too: a new bunch's is written by the kernel before its first pass)
   for (int i = threadIdx.x; i < kRfTableSize; i += THREADS) copy16_async(s_rf + i, a.rf_table + i);
+  grid_dependency_wait();
   grid_launch_dependents();   // the bins step may be scheduled: it reads the turn state too
+  // the first group streams in while the turn's scalars and the kick window do
+  constexpr bool kPrefetch = PREFETCH;
+  const int64_t ng = rg.q_end;
+  const int64_t stride = rg.q_step;
+  int64_t q = rg.q_begin + threadIdx.x;
+  double zn[PPT], en[PPT];
+  if (kPrefetch && q < ng) {
+    ldp<PPT>(a.z + PPT * q, zn);
+    ldp<PPT>(a.dE + PPT * q, en);
+  }
   TurnState* ts = a.ts;
   const bool done = ts->turns_left <= 0;      // a batch member's budget is spent
   __syncthreads();            // the zeros are written where the kick window goes
@@ -859,15 +868,6 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   double acc_z = 0.0, acc_z2 = 0.0, acc_d = 0.0;
   int32_t n_out = 0;
   const double2* __restrict__ potd = a.potd;
-  const int64_t ng = rg.q_end;
-  const int64_t stride = rg.q_step;
-  int64_t q = rg.q_begin + threadIdx.x;
-  constexpr bool kPrefetch = PREFETCH;
-  double zn[PPT], en[PPT];
-  if (kPrefetch && q < ng) {
-    ldp<PPT>(a.z + PPT * q, zn);
-    ldp<PPT>(a.dE + PPT * q, en);
-  }
   // With the Float64 normals (QE_PHILOX), a particle whose draw fails the
   // ziggurat's fast test (about 0.23 %) is turned and deposited like the
   // others with its rejected candidate but stored as loaded, and its bit set in
@@ -1632,10 +1632,11 @@ int track_blocks_per_sm(int B, int qe_mode, int use_wake, int cfg) {
   return bps < 1 ? 1 : bps;
 }
 
-cudaError_t launch_track_pass(const PassArgs& a, int grid, cudaStream_t st) {
+cudaError_t launch_track_pass(const PassArgs& a, int grid, cudaStream_t st, bool overlap) {
   const size_t smem = track_smem_bytes(a.B, a.use_wake, a.cfg, a.zig != 0);
   void* args[] = {const_cast<PassArgs*>(&a)};
   PdlConfig l(dim3(grid), dim3(pass_cfg_threads(a.cfg)), smem, st);
+  if (!overlap) l.cfg.numAttrs = 0;
   const int cfg = a.use_wake && a.hwin < a.B + 1 ? (a.cfg | kPassWindowed) : a.cfg;
   return cudaLaunchKernelExC(&l.cfg, pass_fn(a.use_wake, a.qe_mode, cfg), args);
 }

@@ -15,9 +15,11 @@ DRIVER = r"""
 #include <cstdio>
 #include "hj_launch.h"
 int main() {
-  long long n, chunk;
-  printf("%lld %lld\n", (long long)hj::kMaxBlockParticles, (long long)hj::kMemberBlocks);
-  while (scanf("%lld %lld", &n, &chunk) == 2) printf("%lld\n", (long long)hj::member_chunk(n, chunk));
+  long long n, chunk, slots;
+  printf("%lld\n", (long long)hj::kMaxBlockParticles);
+  while (scanf("%lld %lld %lld", &n, &chunk, &slots) == 3)
+    printf("%lld %lld\n", (long long)hj::member_chunk(n, chunk, slots),
+           (long long)hj::member_blocks(slots));
 }
 """
 
@@ -33,10 +35,11 @@ def test_member_chunk(tmp_path, chunk):
     rng = random.Random(chunk)
     ns = [1, 2, 127, 128, 129, 16383, 16384, 16385, 131071, 131072, 131073, 2**20, 10**8]
     ns += [rng.randrange(1, 2**24) for _ in range(200)]
-    out = subprocess.run([exe], input="".join(f"{n} {chunk}\n" for n in ns), capture_output=True,
-                         text=True, check=True).stdout.split()
-    most, blocks = int(out[0]), int(out[1])
-    for n, c in zip(ns, map(int, out[2:])):
+    cases = [(n, slots) for n in ns for slots in (1, 2, 16, 37, 148, 1000)]
+    out = subprocess.run([exe], input="".join(f"{n} {chunk} {s}\n" for n, s in cases),
+                         capture_output=True, text=True, check=True).stdout.split()
+    most = int(out[0])
+    for (n, slots), c, blocks in zip(cases, map(int, out[1::2]), map(int, out[2::2])):
         assert 0 < c <= min(2 * chunk, most)
         assert c % 4 == 0
         assert -(-n // c) <= n // chunk + blocks + 1, (n, c)
