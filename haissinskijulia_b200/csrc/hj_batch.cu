@@ -166,7 +166,7 @@ hj_status batch_launch_turn(hj_batch* bt) {
                                  bt->resident ? bt->d_counts + 2 : nullptr, bt->resident_blocks,
                                  bt->stream));
   HJ_CUDA(ctx, launch_batch_scan(bt->d_bins, bt->d_counts + 1, bt->grid_bunches, bt->max_B,
-                                 bt->stream));
+                                 bt->max_bunches, bt->stream));
   return HJ_OK;
 }
 
