@@ -672,14 +672,14 @@ class Batch:
     """Independent bunches advanced together on one GPU (hj_batch_*).
 
     Each bunch has its own particles, RF voltage, wake intensity, bins, seed
-    and turn count; every turn is one batched particle pass, one histogram
-    merge and one batched bins step for all live bunches, and blocks of
-    `graph_turns` turns replay a captured CUDA graph.  A bunch's results do
+    and turn count; every turn is one batched particle pass and one
+    batched bins step for all live bunches, and blocks of `graph_turns` turns replay a captured CUDA graph.  A bunch's results do
     not depend on which other bunches share the batch.
 
     pool_particles: particle capacity (16 B each on the device); max_bunches:
     bunch slots; max_nbins: largest bin count; chunk: particles per block of
-    the pass (multiple of 4); layout: pass thread layout (-1 = default).
+    the pass (multiple of 4; small bunches are split finer, large ones up to
+    twice as coarse); layout: pass thread layout (-1 = default).
     """
 
     def __init__(self, ctx: Context, pool_particles: int, max_bunches: int, max_nbins: int,

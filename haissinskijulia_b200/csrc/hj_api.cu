@@ -417,7 +417,7 @@ extern "C" void hj_bunch_destroy(hj_bunch* b) {
   cache_give(b->ctx, true, b->harena, b->harena_cap);
   cache_give(b->ctx, false, b->tables, b->tables_cap);
   if (b->d_sums) cudaFree(b->d_sums);
-  if (b->d_log) cudaFree(b->d_log);
+  cache_give(b->ctx, false, b->d_log, b->d_log_cap);
   for (cudaEvent_t e : b->events) cudaEventDestroy(e);
   hj_ctx* ctx = b->ctx;
   const bool held = b->holds_ctx;

@@ -68,8 +68,9 @@ struct hj_batch {
 
 namespace {
 
-// Whether p is memory of the context's device.
+// Whether p is an array of doubles in the memory of the context's device.
 bool on_device(hj_ctx* ctx, const void* p) {
+  if ((uintptr_t)p & 7) return false;
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();

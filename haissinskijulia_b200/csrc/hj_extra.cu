@@ -167,14 +167,21 @@ extern "C" hj_status hj_bunch_set_log(hj_bunch* b, int64_t every, int64_t capaci
     return set_err(ctx, HJ_ERR_ARG, "log every >= 0 turns into capacity > 0 records");
   if (density && !b->use_wake) return set_err(ctx, HJ_ERR_STATE, "no line density without the wakefield");
   HJ_CUDA(ctx, cudaStreamSynchronize(b->stream));
-  if (b->d_log) cudaFree(b->d_log);
+  cache_give(ctx, false, b->d_log, b->d_log_cap);
   b->d_log = nullptr;
   b->log_every = every;
   b->log_capacity = capacity;
   b->log_density = density ? 1 : 0;
   b->log_count = 0;
-  if (every > 0)
-    HJ_TRY(dalloc(ctx, &b->d_log, (size_t)capacity * (kLogHeader + (b->log_density ? b->B : 0))));
+  if (every > 0) {
+    void* p = nullptr;
+    b->log_every = 0;            // until the log has its memory
+    HJ_TRY(cache_take(ctx, false,
+                      sizeof(double) * (size_t)capacity * (kLogHeader + (b->log_density ? b->B : 0)),
+                      &p, &b->d_log_cap));
+    b->d_log = (double*)p;
+    b->log_every = every;
+  }
   return HJ_OK;
 }
 

@@ -90,7 +90,7 @@ struct PassArgs {
                                    // particles whose Float64 normal takes the slow path
   int32_t zig;                     // 1: shared memory holds the ziggurat's rows (the pass
                                    // draws the Float64 normals), 0: the RF table alone
-  int32_t hwin;                    // bins and cells of the pass's hot histogram window
+  int32_t hwin;                    // cells of the pass's hot histogram window
 };
 
 // One entry of a batch's chunk table: particles [first, first + count) of
@@ -187,7 +187,7 @@ int track_blocks_per_sm(int B, int qe_mode, int use_wake, int cfg);
 // so its shared memory holds the ziggurat's rows.
 size_t track_smem_bytes(int B, int use_wake, int cfg, bool zig);
 // Shared-memory windows of the fused pass for B bins (with the wake): `hot`
-// bins and cells whose per-block histograms are in shared memory (at most
+// cells whose per-block counters are in shared memory (at most
 // B + 1), and `kick` kick-table entries (0 up to 4096 bins, else min(hot, B)).
 struct PassWindows {
   int32_t hot, kick;

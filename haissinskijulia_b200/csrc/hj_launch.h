@@ -6,8 +6,8 @@
 
 namespace hj {
 
-// Particles one block of the fused pass may deposit per turn (the packed CIC
-// counter keeps a 20-bit count per cell).
+// Particles one block of the fused pass may deposit per turn (its counters and
+// trip counts are 32-bit; the bound leaves them far from wrapping).
 constexpr int64_t kMaxBlockParticles = (1 << 20) - 8;
 
 // Thread layouts of the fused pass (particles/thread x threads/block; the next
@@ -91,10 +91,9 @@ inline int track_grid_size(int64_t n, int B, int num_sms, int blocks_per_sm, int
   int64_t g = (n + per_block - 1) / per_block;
   int64_t cap = (int64_t)num_sms * blocks_per_sm;
   if (g > cap) g = cap;
-  // The packed CIC counter holds at most kMaxBlockParticles per block and
-  // turn.  Block b takes the groups of PPT particles b·T + t + k·g·T: at most
-  // ceil((n / PPT) / (g·T)) steps of T·PPT particles, and block 0 also the
-  // n mod PPT tail.  So g is raised until no block takes more steps than fit.
+  // At most kMaxBlockParticles per block and turn.  Block b takes the groups of PPT particles b·T + t + k·g·T: at most
+  // ceil((n / PPT) / (g·T)) steps of T·PPT particles, and block 0 also
+  // the tail that whole warps leave over.  So g is raised until no block takes more steps than fit.
   const int64_t threads = pass_cfg_threads(cfg);
   const int64_t steps = kMaxBlockParticles / ((int64_t)pass_cfg_ppt(cfg) * threads);
   const int64_t groups = n / pass_cfg_ppt(cfg);

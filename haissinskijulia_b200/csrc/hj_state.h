@@ -77,14 +77,15 @@ struct hj_bunch {
   int nblk = 1, nblk_m = 1;
   // a shard of a bunch split over processes: its particles are
   // [first_particle, first_particle + n) of n_global; the bins step reads the
-  // exchanged totals (d_sums, hist) instead of this shard's partials
+  // exchanged totals (d_sums, acc) instead of this shard's partials
   bool shard = false;
   int64_t n_global = 0, first_particle = 0;
   double* d_sums = nullptr;
   // turn log: a record every log_every turns into a ring of log_capacity
   int64_t log_every = 0, log_capacity = 0, log_count = 0;
   int log_density = 0;
-  double* d_log = nullptr;
+  double* d_log = nullptr;     // a block of the context's cache
+  size_t d_log_cap = 0;
   int64_t turns_done = 0;
   // device buffers
   TurnState* ts = nullptr;

@@ -4,8 +4,8 @@ The reference scans parameters one point after another
 (src/parameter_sensitivity/scan.jl:182-184, each point a full
 longitudinal_evolve!).  Here every point is a bunch of its own (particles,
 RF voltage, intensity, bins, seed, turns) and all live points advance
-together in a Batch: one batched particle pass, one histogram merge and one
-batched bins step per turn, turn blocks replayed from a CUDA graph.
+together in a Batch: one batched particle pass and one batched bins step per
+turn, turn blocks replayed from a CUDA graph.
 
 * `sweep_points` / `intensity_scan`: the ragged 256-point sweep and the
   32-bunch intensity scan, seeded.

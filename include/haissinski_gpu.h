@@ -339,8 +339,8 @@ hj_status hj_bunch_bins(hj_bunch* b);
 /* ---------------------------------------------------------------- batches
  * Many independent bunches -- each with its own particle count, RF voltage,
  * intensity, bins, seed and number of turns -- advanced together: every turn
- * is one particle-pass launch over a chunk table of all live bunches, one
- * histogram merge and one bins-step launch with a two-CTA cluster per bunch.
+ * is one particle-pass launch over a chunk table of all live bunches and one
+ * bins-step launch with a cluster per bunch.
  * Blocks of K turns replay a captured CUDA graph.  A bunch's results do not
  * depend on which other bunches share the batch.  No reference counterpart:
  * the reference runs parameter points one after another
@@ -349,8 +349,8 @@ hj_status hj_bunch_bins(hj_bunch* b);
 /* A batch on ctx's device with its own stream: a particle pool of
  * pool_particles (16 B each), up to max_bunches bunches of up to max_nbins
  * bins, chunk_particles particles per block of the pass (a multiple of 4, at
- * most 2^20 - 8, what a block's packed cell counters can count; 0 = 65536)
- * and pass layout `layout` (-1 = the default for max_nbins; values as for
+ * most 2^20 - 8; 0 = 65536; small bunches are split finer and large ones up to
+ * twice as coarse, by a rule on the bunch's size and max_bunches) and pass layout `layout` (-1 = the default for max_nbins; values as for
  * hj_set_pass_layout). */
 hj_status hj_batch_create(hj_ctx* ctx, int64_t pool_particles, int32_t max_bunches,
                           int32_t max_nbins, int64_t chunk_particles, int32_t layout,
