@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -71,13 +72,17 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
     BUILD.mkdir(exist_ok=True)
     nvcc = _nvcc()
     objs = []
+    cmds = []
     for src in CU_SOURCES:
         obj = BUILD / (Path(src).stem + ".o")
         cmd = [nvcc, *ARCH, *NVCC_FLAGS, f"-I{INCLUDE}", "-c", str(CSRC / src), "-o", str(obj)]
         if ptxas_verbose:
             cmd += ["-Xptxas", "-v"]
-        _run(cmd, verbose or ptxas_verbose)
+        cmds.append(cmd)
         objs.append(obj)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:   # one nvcc per source
+        for done in [pool.submit(_run, cmd, verbose or ptxas_verbose) for cmd in cmds]:
+            done.result()
     cxx = os.environ.get("CXX", "g++")
     for src in CPP_SOURCES:
         obj = BUILD / (Path(src).stem + ".o")
