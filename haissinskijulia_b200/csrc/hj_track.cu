@@ -101,8 +101,12 @@ __device__ __forceinline__ int cic_hi(int B) { return B >= 2 ? B - 2 : 0; }
 // Interpolation weights enter the cell sums as integers w·2^24.
 constexpr double kCicScale = 16777216.0;
 
+// The global loads below stay behind a kernel's grid_dependency_wait() (volatile
+// statements keep their order) and are coherent ones: .nc would promise memory that
+// nobody writes while the kernel lives, and a kernel started ahead of its
+// predecessors' end is alive while they write what it reads after the wait.
 __device__ __forceinline__ void ld4(const double* p, double v[4]) {
-  asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
       : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
       : "l"(p));
 }
@@ -173,7 +177,9 @@ __device__ __forceinline__ void copies_wait() {
 
 __device__ __forceinline__ double2 ld_table(const double2* p) {
   double2 v;
-  asm("ld.global.nc.L1::evict_last.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  asm volatile("ld.global.L1::evict_last.v2.f64 {%0,%1}, [%2];"
+               : "=d"(v.x), "=d"(v.y)
+               : "l"(p));
   return v;
 }
 
@@ -513,11 +519,13 @@ __device__ __forceinline__ void block_sum4(double a0, double a1, double a2, doub
 template <int PPT>
 __device__ __forceinline__ void ldp(const double* p, double v[PPT]) {
   if (PPT == 4) {
-    asm("ld.global.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];"
-        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
-        : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
   } else {
-    asm("ld.global.L1::no_allocate.v2.f64 {%0,%1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v2.f64 {%0,%1}, [%2];"
+                 : "=d"(v[0]), "=d"(v[1])
+                 : "l"(p));
   }
 }
 
@@ -925,7 +933,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
     } else if (QE == QE_DRAWS) {
       if (drow) {
 #pragma unroll
-        for (int j = 0; j < PPT; ++j) rr[j] = __ldg(drow + PPT * q + j);
+        for (int j = 0; j < PPT; ++j) rr[j] = __ldcg(drow + PPT * q + j);
       }
     }
     double rf[PPT];
@@ -969,7 +977,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       philox_normals2_rk(a.seed, a.philox, turn, (i >> 1) + a.pair_offset, &g_normal, s_zt, r2);
     if (QE == QE_PHILOX_FAST) philox_normals2_fast(a.philox, turn, (i >> 1) + a.pair_offset, r2);
     double r = r2[i & 1];
-    if (QE == QE_DRAWS) r = drow ? __ldg(drow + i) : 0.0;
+    if (QE == QE_DRAWS) r = drow ? __ldcg(drow + i) : 0.0;
     double z1[1] = {a.z[i]};
     double e = a.dE[i];
     const double kick = WAKE ? wake_kick(z1[0], g, potd) : 0.0;
