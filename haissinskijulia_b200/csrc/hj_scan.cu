@@ -55,6 +55,18 @@ constexpr size_t scan_smem() {
   return sizeof(double2) * (size_t)(NT * E + kPowLo + kPowHi) + sizeof(double) * (size_t)(NT * E + 2);
 }
 
+// The turn's scalars past L1, which may hold the line as it was before the previous
+// bins step wrote it: only a kernel's own wait makes plain loads see what other
+// kernels wrote, and this one comes before it.
+__device__ __forceinline__ TurnScalars load_scalars(const TurnScalars* p) {
+  static_assert(sizeof(TurnScalars) % sizeof(long long) == 0, "whole words");
+  TurnScalars s;
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(TurnScalars) / sizeof(long long)); ++k)
+    reinterpret_cast<long long*>(&s)[k] = __ldcg(reinterpret_cast<const long long*>(p) + k);
+  return s;
+}
+
 // All threads of the block, or of the cluster.
 template <int C>
 __device__ __forceinline__ void block_or_cluster_sync() {
@@ -89,13 +101,14 @@ __device__ __forceinline__ void scan_body(const ScanArgs& a) {
 
   // before the pass has finished: the powers of σ and the smoothing weights
   // delta(c_i) (src/utils.jl:58-66) of this thread's bins base + t + k NT; the
-  // scalar warp reads the turn's state, which the previous bins step wrote
+  // scalar warp reads the turn's scalars, which the previous bins step wrote: every
+  // block of this turn's pass had waited for it before it let this kernel start
   double lam[E];
   TurnScalars cur;
   double coef = 0.0;
   const double inv_n = 1.0 / (double)a.n;
   if (scalar) {
-    cur = ts->cur;
+    cur = load_scalars(&ts->cur);
     // the wake current over σ_z (src/evolution.jl:373-386)
     coef = a.particle_factor / cur.E0 / (kTwoPi * a.params.radius) /
            (cur.eta0 * (a.sigma_E0_initial * a.sigma_E0_initial));

@@ -28,3 +28,12 @@ def test_the_pass_reads_through_no_non_coherent_intrinsic():
     code = _code(CSRC / "hj_track.cu")
     body = code[code.index("void pass_body("):code.index("k_batch_pass(")]
     assert "grid_dependency_wait" in body and "__ldg" not in body
+
+
+def test_the_scan_reads_ahead_of_its_wait_past_l1():
+    code = _code(CSRC / "hj_scan.cu")
+    early = code[code.index("void scan_body("):]
+    early = early[:early.index("grid_dependency_wait()")]
+    assert "load_scalars(&ts->cur)" in early
+    assert "ts->" not in early.replace("&ts->cur", "")
+    assert "__ldcg" in code[code.index("load_scalars("):code.index("void scan_body(")]
