@@ -409,12 +409,19 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
 // issued before any returned value is used, so their latencies overlap.  s_cnt
 // and s_lo are the shared arrays offset by the window's start: half h's counter is
 // s_cnt[h], or 16 bits of the word s_cnt[h >> 1] without N32; cell j's sum s_lo[j].
-// When none of the K particles needs the reference's rounding and, with WIN, all K
-// cells are in the window, the deposits run straight through, else one by one
-// with every check; deposits outside the window go to global memory.  One branch
-// for the group where every particle had its own: 722 -> 690 us a pass of 1e8
-// particles at 16384 bins, 724 -> 685 at 4096.
-template <int K, bool N32, bool WIN>
+// Particles that need the reference's rounding, or lie off the grid (cell_half), and
+// with WIN those outside the window, are sorted out first: the latter's deposits go
+// to global memory, and in shared memory they take the spare cell behind the window,
+// which nobody reads.  So the deposits themselves run straight through for all, and a
+// bunch wider than its window pays for its own outliers alone.  us a pass of 2e7
+// particles at 16384 bins, bunches 1, 1.2, 1.5 and 2 times as long as their grid
+// assumes: 147 150 163 184; with one branch for the group, its other side one by one,
+// 168 230 349 351; with three atomics and a branch per particle 157 162 179 196 (4096
+// bins: 138 139 139 142, 138 138 148 223 and 147 for any length).
+// MASK: the outliers as a mask, which takes fewer registers than a flag each: the
+// batched pass spills otherwise (us a turn of 256 bunches 869 against 959, of 32 of
+// 1e6 258 against 277), the plain pass is 2 % faster with flags.
+template <int K, bool N32, bool WIN, bool MASK = true>
 __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridConst& g,
                                               const PassWindow& hw, double& acc_z,
                                               double& acc_z2, int32_t& n_out, uint32_t* s_cnt,
@@ -422,54 +429,65 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
                                               unsigned long long* __restrict__ acc) {
   int cj[K], ch[K];
   uint32_t cq[K];
-  bool plain = true;
+  bool fast[K], plain = true;
+  unsigned rare = 0u;                     // for cell_half: near a bin edge or off the grid
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     acc_z += z[k];
     acc_z2 = fma(z[k], z[k], acc_z2);
-    plain &= cell_half_fast(z[k], g, cj[k], ch[k], cq[k]);
+    const bool ok = cell_half_fast(z[k], g, cj[k], ch[k], cq[k]);
+    if (MASK) rare |= ok ? 0u : 1u << k;
+    else plain &= fast[k] = ok;
     if (WIN) plain &= (uint32_t)(cj[k] - hw.w0) < hw.h;
   }
-  uint32_t onc[K], olo[K];
-  if (plain) {
+  const int spare = hw.w0 + (int)hw.h;
+  if (MASK || !plain) {
+    if (!MASK) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
-      else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
+      for (int k = 0; k < K; ++k) rare |= fast[k] ? 0u : 1u << k;
     }
-#pragma unroll
-    for (int k = 0; k < K; ++k) olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
-  } else {
 #pragma unroll 1
-    for (int k = 0; k < K; ++k) {
+    while (rare) {                        // rolled: out of the main loop's registers
+      const int k = K == 1 ? 0 : __ffs((int)rare) - 1;
+      rare &= rare - 1u;
       double zk = z[0];
 #pragma unroll
       for (int m = 1; m < K; ++m) zk = k == m ? z[m] : zk;
       int j, h;
       uint32_t q;
       cell_half(zk, g, j, h, q, n_out, 1);
-      uint32_t o = 0u;
-      if (!WIN || (uint32_t)(j - hw.w0) < hw.h) {
-        if (N32) atomicAdd(&s_cnt[h], 1u);
-        else o = atomicAdd(&s_cnt[j], 1u << ((h & 1) << 4));
-        const uint32_t lo = atomicAdd(&s_lo[j], q);
-        if (lo + q < lo) atomicAdd(acc + 2 * g.B + 1 + j, 1ull << 32);
-      } else {
-        add_halves(acc, g.B, h, 1ull);
-        atomicAdd(acc + 2 * g.B + 1 + j, (unsigned long long)q);
-      }
+      if (WIN) plain &= (uint32_t)(j - hw.w0) < hw.h;
 #pragma unroll
       for (int m = 0; m < K; ++m)
         if (k == m) {
-          onc[m] = o;
           cj[m] = j;
           ch[m] = h;
+          cq[m] = q;
+        }
+    }
+    if (WIN && !plain) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if ((uint32_t)(cj[k] - hw.w0) >= hw.h) {
+          add_halves(acc, g.B, ch[k], 1ull);
+          atomicAdd(acc + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
+          cj[k] = spare;
+          ch[k] = 2 * spare;
+          cq[k] = 0u;
         }
     }
   }
+  uint32_t onc[K], olo[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
+    else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
   if (!N32) {
     // 16-bit counters, the two halves of a cell in a word: the increment that
     // takes a counter to 2^15 moves 2^15 counts to the accumulators (the counter
@@ -477,7 +495,7 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int sh = (ch[k] & 1) << 4;
-      if (((onc[k] >> sh) & 0xFFFFu) == 0x7FFFu) {
+      if (((onc[k] >> sh) & 0xFFFFu) == 0x7FFFu && !(WIN && cj[k] == spare)) {
         atomicSub(&s_cnt[cj[k]], 0x8000u << sh);
         add_halves(acc, g.B, ch[k], 0x8000ull);
       }
@@ -771,17 +789,16 @@ __device__ __forceinline__ void pass_setup(unsigned char* smem_raw) {
   }
 }
 
-template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32 = false,
-          bool WIN = false>
+template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN, bool MASK>
 __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg,
                                           unsigned char* smem_raw) {
   // dynamic shared memory: RF table [128] | the ziggurat's rows [2048] (a.zig) |
   // kick-table window [win, rounded up to even] | counts of the hot window's `hot`
   // cells by halves: two 32-bit words a cell (N32), or one of two 16-bit counters |
-  // cell sums [hot]
+  // cell sums [hot]; counts and sums with a spare cell behind the window's
   const int nc = a.B + 1;                 // kick-table cells
   const int hot = WAKE ? a.hwin : 0;
-  const int nw = N32 ? 2 * hot : hot;
+  const int nw = N32 ? 2 * (hot + 1) : hot + 1;
   const int win = WAKE ? a.win : 0;
   double2* s_rf = reinterpret_cast<double2*>(smem_raw);
   double2* s_zt = s_rf + kRfTableSize;
@@ -951,7 +968,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       es[j] = keep ? e0 : ee[j];
     }
     if (WAKE)
-      deposit_group<PPT, N32, WIN>(zz, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
+      deposit_group<PPT, N32, WIN, MASK>(zz, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
     stp<PPT>(a.z + PPT * q, zs);
     stp<PPT>(a.dE + PPT * q, es);
     if (kDefer) {
@@ -1012,7 +1029,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
                      groups * PPT, blockIdx.x == 0 ? (int32_t)(a.n - groups * PPT) : 0,
                      (int32_t)blockIdx.x};
   pass_setup<WAKE, QE, THREADS>(smem_raw);
-  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, false>(a, rg, smem_raw);
 }
 
 template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN>
@@ -1023,7 +1040,7 @@ __device__ __forceinline__ void run_chunk(const PassArgs* __restrict__ bunches,
   const int64_t groups = ch.count / PPT & ~(int64_t)31;
   const PassRange rg{ch.first / PPT, THREADS, ch.first / PPT + groups,
                      ch.first + groups * PPT, (int32_t)(ch.count - groups * PPT), ch.part};
-  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, true>(a, rg, smem_raw);
 }
 
 // One turn over a batch of bunches.  Chunk c of the chunk table (a
@@ -1580,8 +1597,8 @@ PassWindows track_windows(int B, int cfg, bool zig) {
   const size_t tables = pass_table_bytes(zig), budget = pass_smem_budget(cfg);
   const bool kick = B > kWindowMinBins;
   const size_t per = ((cfg & kPassN32) ? 12 : 8) + (kick ? 8 : 0);
-  // 24: an even number of kick entries, counters to a multiple of 16 bytes
-  const size_t room = budget > tables + 24 ? budget - tables - 24 : 0;
+  // 36: the spare cell, an even number of kick entries, counters to a multiple of 16 bytes
+  const size_t room = budget > tables + 36 ? budget - tables - 36 : 0;
   const size_t hot = std::min(room / per, (size_t)B + 1);
   PassWindows w;
   w.hot = (int)hot;
@@ -1594,7 +1611,7 @@ PassWindows track_windows(int B, int cfg, bool zig) {
 size_t track_smem_bytes(int B, int use_wake, int cfg, bool zig) {
   if (!use_wake) return pass_table_bytes(zig);
   const PassWindows w = track_windows(B, cfg, zig);
-  const size_t hist = (size_t)w.hot * ((cfg & kPassN32) ? 3 : 2) * sizeof(uint32_t);
+  const size_t hist = ((size_t)w.hot + 1) * ((cfg & kPassN32) ? 3 : 2) * sizeof(uint32_t);
   return pass_table_bytes(zig) + (size_t)((w.kick + 1) & ~1) * sizeof(double) +
          ((hist + 15) & ~(size_t)15);
 }
