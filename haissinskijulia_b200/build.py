@@ -29,10 +29,7 @@ CPP_SOURCES = ["hj_host.cpp"]
 HEADERS = ["hj_device.cuh", "hj_internal.h", "hj_host.h", "hj_launch.h", "hj_ranges.h", "hj_state.h"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# --split-compile: hj_track.cu's 150 kernels are optimised on all cores (4 min 10 -> 2 min 4
-# on 8 cores, the same register counts)
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-              "--split-compile=0"]
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 CXX_FLAGS = ["-O2", "-fPIC", "-std=c++17", "-ffp-contract=off", "-fno-fast-math"]
 
 
