@@ -233,8 +233,8 @@ static FlushArgs flush_args(hj_bunch* b, int apply, double* z_out, double* dE_ou
   f.B = b->B;
   f.use_wake = b->use_wake;
   f.update_E0 = b->p.update_E0;
-  f.e0 = b->e0;
-  f.inv_estep = b->inv_e;
+  f.kick_inv = b->kick_inv;
+  f.kick_off = b->kick_off;
   f.apply = apply;
   f.z_out = z_out;
   f.dE_out = dE_out;
@@ -479,6 +479,8 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
     b->logH = b->H >= 1 ? ilog2(b->H) : 0;
   }
   b->cfg = cfg >= 0 ? cfg : auto_pass_layout(ctx->pass_layout, b->B, n);
+  b->split = b->use_wake && grid && !host_cells_halve_bins(*grid);
+  if (b->split) b->cfg = split_pass_cfg(b->cfg);
   if (chunk > 0) {
     b->batch_member = true;
     b->chunk = chunk;
@@ -579,6 +581,8 @@ hj_status hj_impl::bunch_create_end(hj_ctx* ctx, hj_bunch* b, const hj_grid* gri
       b->hi_idx = (int)(idx1 - 1);
       b->hi_w = u - fl;
     }
+    host_kick_cells(!b->split, B, b->e0, b->inv_e, b->c1, b->cB, b->inv_c, &b->kick_inv,
+                    &b->kick_off);
     if (b->uniform) {
       host_wake_powers(b->w, b->cJ, b->cstep, b->J, &b->wake_A.x, &b->wake_tau.x,
                        reinterpret_cast<double(*)[2]>(b->wake_pw), kScanPowers);
@@ -694,9 +698,8 @@ void hj_impl::fill_pass_args(const hj_bunch* b, PassArgs& a) {
   a.e0 = b->e0;
   a.eN = b->eN;
   a.inv_estep = b->inv_e;
-  a.c1 = b->c1;
-  a.cB = b->cB;
-  a.inv_cstep = b->inv_c;
+  a.kick_inv = b->kick_inv;
+  a.kick_off = b->kick_off;
   a.V = b->p.voltage;
   a.phi_s = b->p.phi_s;
   {

@@ -185,6 +185,32 @@ bool host_uniform_centers(const double* c, int64_t B, int64_t* J, double* step) 
   return true;
 }
 
+bool host_cells_halve_bins(const hj_grid& g) {
+  const int64_t B = g.nbins;
+  const double h = g.edge_step;
+  const double tol = 4.0 * 0x1p-52 * std::fmax(std::fabs(g.edge_first), std::fabs(g.edge_last));
+  return h > 0.0 && std::fabs(g.centers[0] - (g.edge_first + 0.5 * h)) <= tol &&
+         std::fabs(g.centers[B - 1] - (g.edge_last - 0.5 * h)) <= tol &&
+         std::fabs(g.edge_last - (g.edge_first + h * (double)B)) <= tol;
+}
+
+void host_kick_cells(bool halves, int64_t B, double e0, double inv_e, double c1, double cB,
+                     double inv_c, double* inv, double* off) {
+  if (halves) {
+    *inv = inv_e;
+    *off = 0.5 - e0 * inv_e;
+  } else if (B < 2) {            // one centre: flat on both sides
+    *inv = 0.0;
+    *off = 0.5;
+  } else if (!(cB > c1)) {       // clamp(z, c1, cB) gives cB for every z
+    *inv = 0.0;
+    *off = (double)B;
+  } else {
+    *inv = inv_c;
+    *off = (double)(1.0L - (long double)c1 * (long double)inv_c);
+  }
+}
+
 double host_particle_factor(int64_t n, double population) {
   if (population > 0.0) return population;
   int pw = -1;                                   // floor(log10 n) by digit count

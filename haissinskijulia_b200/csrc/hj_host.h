@@ -24,6 +24,14 @@ void host_wake_powers(const hj_wake& w, double cJ, double step, int64_t J, doubl
 // Whether the B centres are uniform to rounding with a positive step and reach
 // <= 0, i.e. the wake table is that sequence; J and the step when so.
 bool host_uniform_centers(const double* centers, int64_t B, int64_t* J, double* step);
+// Whether the interpolation cells of a caller's grid (between its centres) start half a
+// bin off its histogram's bins (between its edges) throughout, to rounding: then the
+// halves of a cell are those of two neighbouring bins.
+bool host_cells_halve_bins(const hj_grid& g);
+// Cell coordinate v = z inv + off of the kick table (cell j between centres j-1 and j):
+// from the edges where the cells halve the bins, else from the centres c1 and cB.
+void host_kick_cells(bool halves, int64_t B, double e0, double inv_e, double c1, double cB,
+                     double inv_c, double* inv, double* off);
 // Particle factor of the wake current (src/evolution.jl:373-384).
 double host_particle_factor(int64_t n, double population);
 void host_twiddles(int64_t P, double* tw_interleaved);

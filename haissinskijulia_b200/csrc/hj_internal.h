@@ -67,7 +67,7 @@ struct PassArgs {
   int32_t B;
   int32_t use_wake;
   double e0, eN, inv_estep;       // histogram (edges)
-  double c1, cB, inv_cstep;       // interpolation (centers)
+  double kick_inv, kick_off;      // cell coordinate where the grid is split (host_kick_cells)
   // physics constants of the run
   double V, phi_s, inv_mass, alpha_c, two_pi_h;
   // RF kick: x = z k = m h + t, h = 2π / kRfTableSize (h_hi + h_lo), and
@@ -170,7 +170,7 @@ struct FlushArgs {
   const double2* potd;
   int32_t B;
   int32_t use_wake, update_E0;
-  double e0, inv_estep;   // kick-table cell coordinate
+  double kick_inv, kick_off;   // kick-table cell coordinate
   int32_t apply;      // 1: apply pending ops
   double* z_out;      // destination (may alias z/dE); NULL -> not written
   double* dE_out;

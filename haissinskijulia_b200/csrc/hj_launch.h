@@ -23,6 +23,10 @@ constexpr int kPassFastNormals = 16;  // + single-precision quantum-excitation n
 // Launch-only bit (never in a caller's configuration): the pass's hot window
 // holds fewer than all B + 1 cells, so its deposits are range-checked.
 constexpr int kPassWindowed = 32;
+// Bit of a bunch's configuration (never in a caller's): its grid's cells do not halve its
+// bins, which one layout serves (0 with 32-bit counters).
+constexpr int kPassSplit = 64;
+inline int split_pass_cfg(int cfg) { return kPassSplit | kPassN32 | (cfg & kPassFastNormals); }
 
 inline int pass_cfg_threads(int cfg) {
   const int l = cfg & kPassLayoutMask;

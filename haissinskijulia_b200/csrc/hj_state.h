@@ -59,6 +59,10 @@ struct hj_bunch {
   int use_wake = 0;
   int B = 0, P = 0, M = 0, H = 0, logH = 0;
   double e0 = 0, eN = 0, estep = 0, inv_e = 0, c1 = 0, cB = 0, inv_c = 0;
+  // a caller's grid whose interpolation cells do not halve its bins: the pass counts
+  // cells and bins apart; kick-table cell coordinate (host_kick_cells)
+  bool split = false;
+  double kick_inv = 0, kick_off = 0;
   // interpolation the reference applies to every z >= cB (src/wakefield.jl:80-102):
   // u = (cB - c1)/Δc, cell clamp(floor(u), 0, B-2), weight u - floor(u)
   int hi_idx = 0;

@@ -50,6 +50,7 @@
 //     QE), all exact, so the pass has no per-particle branches on them.
 #include <algorithm>
 #include <memory>
+#include <type_traits>
 
 #include "hj_host.h"
 #include "hj_internal.h"
@@ -89,6 +90,14 @@ struct GridConst {
   int B;
   double e0, eN, inv_e, c1, cB, inv_c;
   double v_off;   // 1/2 - e0/Δe: v = z/Δe + v_off is the cell coordinate of the kick table
+  static constexpr bool split = false;
+  __device__ __forceinline__ double cell_coordinate(double z) const { return fma(z, inv_e, v_off); }
+};
+// A grid whose cells do not halve its bins (host_cells_halve_bins): they follow the centres.
+struct SplitGrid : GridConst {
+  double k_inv, k_off;
+  static constexpr bool split = true;
+  __device__ __forceinline__ double cell_coordinate(double z) const { return fma(z, k_inv, k_off); }
 };
 
 // 1/2 - e0/Δe, rounded the same way by every kernel that forms cell coordinates.
@@ -144,8 +153,8 @@ __device__ __forceinline__ void cic_cell(double z, const GridConst& g, int& idx,
   idx = min(max(__double2loint(fm), 0), cic_hi(g.B));
 }
 
-// Cell of the kick table (B + 1 cells): v = z/Δe + 1/2 - e0/Δe (one FMA),
-// j = floor(v) clamped to [0, B], w = v - floor(v).  Cell j >= 1 is the
+// Cell of the kick table (B + 1 cells): v = z/Δe + 1/2 - e0/Δe (one FMA; where a
+// caller's edges and centres do not fit together, z/Δc + 1 - c1/Δc), j = floor(v) clamped to [0, B], w = v - floor(v).  Cell j >= 1 is the
 // reference's interpolation cell j-1 between centres c[j-1] and c[j]
 // (src/wakefield.jl:64-78); cells 0 and B hold the flat ends pot[0] and pot[B-1]
 // that the reference's clamp of z to [c1, cB] gives, so out-of-range particles need
@@ -154,8 +163,9 @@ __device__ __forceinline__ void cic_cell(double z, const GridConst& g, int& idx,
 // floor(v): the low word of (v + 1.5·2^52 rounded down) when the high word is
 // 0x43380000 (0 <= v < 2^32); other high words mean v < 0 (cell 0) or v >= 2^32,
 // +inf and NaN (cell B) -- every z lands in a valid cell.
-__device__ __forceinline__ void kick_cell(double z, const GridConst& g, int& j, double& w) {
-  const double v = fma(z, g.inv_e, g.v_off);
+template <class G>
+__device__ __forceinline__ void kick_cell(double z, const G& g, int& j, double& w) {
+  const double v = g.cell_coordinate(z);
   const double fm = __dadd_rd(v, kMagic);
   w = __dsub_rn(v, __dsub_rn(fm, kMagic));
   const int t = __double2hiint(fm) - 0x43380000;
@@ -210,8 +220,8 @@ struct PassWindow {
 struct KickFetch {
   double p0, d, w;
 };
-__device__ __forceinline__ KickFetch kick_fetch(double z, const GridConst& g,
-                                                const PassWindow& kw,
+template <class G>
+__device__ __forceinline__ KickFetch kick_fetch(double z, const G& g, const PassWindow& kw,
                                                 const double2* __restrict__ potd) {
   int j;
   KickFetch f;
@@ -231,7 +241,8 @@ __device__ __forceinline__ KickFetch kick_fetch(double z, const GridConst& g,
 
 // Kick of the fused pass: lerp from the kick table, cell j holding
 // (pot at its left centre, pot step to its right centre), zero step in cells 0 and B.
-__device__ __forceinline__ double wake_kick(double z, const GridConst& g,
+template <class G>
+__device__ __forceinline__ double wake_kick(double z, const G& g,
                                             const double2* __restrict__ potd) {
   int j;
   double w;
@@ -271,25 +282,35 @@ __device__ __forceinline__ int ngp_bin(double z, const GridConst& g, bool& in) {
 // words of w around 1/2: one particle in a million) ngp_bin evaluates the
 // reference's own rounding.  cell_half_fast says whether none of that applies
 // (and z lies in cells 1..B-1); cell_half serves any z and counts the particles
-// outside the grid in n_out.  floor(v): see kick_cell.
-__device__ __forceinline__ bool cell_half_fast(double z, const GridConst& g, int& j, int& h,
+// outside the grid in n_out.  floor(v): see kick_cell.  A caller's grid may have
+// edges and centres that do not fit together so (SplitGrid): every z goes through
+// cell_half then, a cell's first counter holds its particles and its second one
+// those of the bin of the same number.
+template <class G>
+__device__ __forceinline__ bool cell_half_fast(double z, const G& g, int& j, int& h,
                                                uint32_t& q) {
-  const double v = fma(z, g.inv_e, g.v_off);
+  const double v = g.cell_coordinate(z);
   const double fm = __dadd_rd(v, kMagic);
   const double w = __dsub_rn(v, __dsub_rn(fm, kMagic));
   const int wh = __double2hiint(w);
   q = (uint32_t)__double2loint(fma(w, kCicScale, kMagic));
   j = __double2loint(fm);
   h = 2 * j + (wh >= 0x3FE00000 ? 1 : 0);
-  return (__double2hiint(fm) == 0x43380000) & ((unsigned)j - 1u < (unsigned)g.B - 1u) &
+  return !G::split & (__double2hiint(fm) == 0x43380000) &
+         ((unsigned)j - 1u < (unsigned)g.B - 1u) &
          ((unsigned)(wh - 0x3FDFFFFF) > 1u);
 }
-__device__ __forceinline__ void cell_half(double z, const GridConst& g, int& j, int& h,
-                                          uint32_t& q, int32_t& n_out, int32_t one) {
+template <class G>
+__device__ __forceinline__ void cell_half(double z, const G& g, int& j, int& h, uint32_t& q,
+                                          int32_t& n_out, int32_t one) {
   if (cell_half_fast(z, g, j, h, q)) return;
   double w;
   kick_cell(z, g, j, w);
   q = min(q, 16777216u);     // a NaN z lands in cell B with any q; the moments flag it
+  if (G::split) {            // the cell's first counter; count_bin adds the bin
+    h = 2 * j;
+    return;
+  }
   bool in;
   const int nb = ngp_bin(z, g, in);
   h = in ? 2 * j + (nb == j ? 1 : 0) : (j == 0 ? 0 : 2 * g.B + 1);
@@ -304,12 +325,31 @@ __device__ __forceinline__ void add_halves(unsigned long long* __restrict__ acc,
   const int b = ((h + 1) >> 1) - 1;
   if ((unsigned)b < (unsigned)B) atomicAdd(acc + b, n);
 }
+// The same of particles outside the window; with split their cell alone.
+template <class G>
+__device__ __forceinline__ void add_outside(unsigned long long* __restrict__ acc, const G& g,
+                                            int h, unsigned long long n) {
+  if (G::split) atomicAdd(acc + g.B + (h >> 1), n);
+  else add_halves(acc, g.B, h, n);
+}
 
 // Reference-form bin for the single-step histogram kernel (any z).
 __device__ __forceinline__ int ngp_bin_any(double z, const GridConst& g, bool& in) {
   in = (z >= g.e0) & (z <= g.eN);
   const int j = __double2int_rd(__dmul_rn(__dsub_rn(z, g.e0), g.inv_e));
   return min(max(j, 0), g.B - 1);
+}
+
+// With split: one particle more (or less) in the bin of z, in the second counter of the
+// cell of its number or outside the window in the accumulators.
+__device__ __forceinline__ void count_bin(double z, const GridConst& g, const PassWindow& hw,
+                                          uint32_t* s_cnt, unsigned long long* __restrict__ acc,
+                                          int32_t& n_out, int32_t one) {
+  bool in;
+  const int nb = ngp_bin_any(z, g, in);
+  if (!in) n_out += one;
+  else if ((uint32_t)(nb - hw.w0) < hw.h) atomicAdd(&s_cnt[2 * nb + 1], (uint32_t)one);
+  else atomicAdd(acc + nb, (unsigned long long)(int64_t)one);
 }
 
 // V(sin(ϕs - x) - sin ϕs), x = z k (see the header comment): x = m h + t with
@@ -421,8 +461,8 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
 // MASK: the outliers as a mask, which takes fewer registers than a flag each: the
 // batched pass spills otherwise (us a turn of 256 bunches 869 against 959, of 32 of
 // 1e6 258 against 277), the plain pass is 2 % faster with flags.
-template <int K, bool N32, bool WIN, bool MASK = true>
-__device__ __forceinline__ void deposit_group(const double (&z)[K], const GridConst& g,
+template <int K, bool N32, bool WIN, bool MASK = true, class G>
+__device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
                                               const PassWindow& hw, double& acc_z,
                                               double& acc_z2, int32_t& n_out, uint32_t* s_cnt,
                                               uint32_t* s_lo,
@@ -456,6 +496,7 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
       int j, h;
       uint32_t q;
       cell_half(zk, g, j, h, q, n_out, 1);
+      if (G::split) count_bin(zk, g, hw, s_cnt, acc, n_out, 1);
       if (WIN) plain &= (uint32_t)(j - hw.w0) < hw.h;
 #pragma unroll
       for (int m = 0; m < K; ++m)
@@ -469,7 +510,7 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const GridCo
 #pragma unroll
       for (int k = 0; k < K; ++k)
         if ((uint32_t)(cj[k] - hw.w0) >= hw.h) {
-          add_halves(acc, g.B, ch[k], 1ull);
+          add_outside(acc, g, ch[k], 1ull);
           atomicAdd(acc + 2 * g.B + 1 + cj[k], (unsigned long long)cq[k]);
           cj[k] = spare;
           ch[k] = 2 * spare;
@@ -592,8 +633,8 @@ __device__ __forceinline__ unsigned group_normals_zig(const PhiloxKeys& rk, int6
 // rounding) and the deposits (exactly: a borrow out of the cell's 32-bit sum is
 // taken from the accumulator, which also takes the negative of a count that may
 // have left its 16-bit counter, modulo 2^64).
-template <bool N32>
-__device__ __forceinline__ void undeposit(double z, const GridConst& g, const PassWindow& hw,
+template <bool N32, class G>
+__device__ __forceinline__ void undeposit(double z, const G& g, const PassWindow& hw,
                                           double& acc_z, double& acc_z2, int32_t& n_out,
                                           uint32_t* s_cnt, uint32_t* s_lo,
                                           unsigned long long* __restrict__ acc) {
@@ -602,9 +643,10 @@ __device__ __forceinline__ void undeposit(double z, const GridConst& g, const Pa
   int cj, ch;
   uint32_t cq;
   cell_half(z, g, cj, ch, cq, n_out, -1);
+  if (G::split) count_bin(z, g, hw, s_cnt, acc, n_out, -1);
   const bool in = (uint32_t)(cj - hw.w0) < hw.h;
   if (N32 && in) atomicSub(&s_cnt[ch], 1u);
-  else add_halves(acc, g.B, ch, ~0ull);
+  else add_outside(acc, g, ch, ~0ull);
   if (in) {
     const uint32_t old = atomicSub(&s_lo[cj], cq);
     if (old < cq) atomicAdd(acc + 2 * g.B + 1 + cj, 0ull - (1ull << 32));
@@ -631,7 +673,7 @@ struct PassRange {
 // same addresses: 148 blocks adding 9868 cells took 8.6 us so and 10.6 us in the
 // same order, against 2.4 us for writing them out as per-block partials and
 // 10 us for the kernel that merged those.
-template <int THREADS, bool N32>
+template <int THREADS, bool N32, bool SPLIT>
 __device__ __forceinline__ void flush_window(const PassArgs& a, const PassWindow& kw, int hot,
                                              int32_t part, const uint32_t* h_cnt,
                                              const uint32_t* h_lo) {
@@ -645,12 +687,17 @@ __device__ __forceinline__ void flush_window(const PassArgs& a, const PassWindow
     if (r >= hot) r -= hot;
     const int c = kw.w0 + r;
     const uint2 n = halves(r);
+    if (h_lo[r]) atomicAdd(a.acc + 2 * a.B + 1 + c, (unsigned long long)h_lo[r]);
+    if (SPLIT) {
+      if (n.x) atomicAdd(a.acc + a.B + c, (unsigned long long)n.x);
+      if (n.y && c < a.B) atomicAdd(a.acc + c, (unsigned long long)n.y);
+      continue;
+    }
     // bin c: this cell's upper half and the next one's lower half
     const uint32_t nb = n.y + (r + 1 < hot ? halves(r + 1).x : 0u);
     if (nb && c < a.B) atomicAdd(a.acc + c, (unsigned long long)nb);
     if (r == 0 && c > 0 && n.x) atomicAdd(a.acc + c - 1, (unsigned long long)n.x);
     if (n.x + n.y) atomicAdd(a.acc + a.B + c, (unsigned long long)(n.x + n.y));
-    if (h_lo[r]) atomicAdd(a.acc + 2 * a.B + 1 + c, (unsigned long long)h_lo[r]);
   }
 }
 
@@ -664,9 +711,9 @@ constexpr size_t kPassTableBytes = (size_t)(kRfTableSize + kZigLayers) * 16u;
 // turn is evaluated again, bit for bit (particle_turn rounds where written),
 // and taken back (undeposit, and its share of the sums); the turn with the
 // normal from the ziggurat's slow path is then applied, deposited and stored.
-template <bool WAKE, bool N32, bool WIN>
+template <bool WAKE, bool N32, bool WIN, class G>
 __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedConst& c,
-                                                const GridConst& g, const PassWindow& kw,
+                                                const G& g, const PassWindow& kw,
                                                 double pmean, int64_t turn, int64_t i,
                                                 const double2* s_zt, const double2* s_rf,
                                                 uint32_t* s_cnt, uint32_t* s_lo, double& acc_z,
@@ -711,9 +758,9 @@ __device__ __forceinline__ void finish_deferred(const PassArgs& a, const FusedCo
 // lane finishes its own particles, lanes without one take the queue's rest (a
 // block with one iteration, i.e. a small bunch, saves the queue's round trip
 // through L2).  Every lane of the warp must take part.
-template <bool WAKE, int PPT, bool N32, bool WIN>
+template <bool WAKE, int PPT, bool N32, bool WIN, class G>
 __device__ __forceinline__ void drain_deferred(const PassArgs& a, const FusedConst& c,
-                                               const GridConst& g, const PassWindow& kw,
+                                               const G& g, const PassWindow& kw,
                                                double pmean, int64_t turn, int64_t qref,
                                                int64_t stride, unsigned long long& pend,
                                                int64_t* wq, int& staged, bool last,
@@ -789,7 +836,8 @@ __device__ __forceinline__ void pass_setup(unsigned char* smem_raw) {
   }
 }
 
-template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN, bool MASK>
+template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN, bool MASK,
+          class G = GridConst>
 __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg,
                                           unsigned char* smem_raw) {
   // dynamic shared memory: RF table [128] | the ziggurat's rows [2048] (a.zig) |
@@ -854,8 +902,17 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   c.coeff0z = sc.drift_ok ? sc.coeff0z : 0.0;
   c.drift_ok = sc.drift_ok;
   c.update_eta = a.update_eta;
-  GridConst g{a.B, a.e0, a.eN, a.inv_estep, a.c1, a.cB, a.inv_cstep,
-              kick_offset(a.e0, a.inv_estep)};
+  G g;
+  g.B = a.B;
+  g.e0 = a.e0;
+  g.eN = a.eN;
+  g.inv_e = a.inv_estep;
+  if constexpr (G::split) {
+    g.k_inv = a.kick_inv;
+    g.k_off = a.kick_off;
+  } else {
+    g.v_off = kick_offset(a.e0, a.inv_estep);
+  }
 
   const double* drow = nullptr;
   if (QE == QE_DRAWS) {
@@ -1014,14 +1071,14 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
                       a.part_sum + (size_t)rg.part * kNumSums,
                       reinterpret_cast<double(*)[4]>(s_rf));
 
-  if (WAKE) flush_window<THREADS, N32>(a, kw, hot, rg.part, h_cnt, h_lo);
+  if (WAKE) flush_window<THREADS, N32, G::split>(a, kw, hot, rg.part, h_cnt, h_lo);
 }
 
 // One turn over one bunch: block b takes groups b, b + grid, ... (THREADS
 // apart) and writes partial slot b; block 0 takes the tail.  WIN: the hot
-// window holds fewer than all cells (kPassWindowed).
+// window holds fewer than all cells (kPassWindowed).  SPLIT: SplitGrid.
 template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, int MINB = 1, bool N32 = false,
-          bool WIN = false>
+          bool WIN = false, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t groups = a.n / PPT & ~(int64_t)31;
@@ -1029,7 +1086,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
                      groups * PPT, blockIdx.x == 0 ? (int32_t)(a.n - groups * PPT) : 0,
                      (int32_t)blockIdx.x};
   pass_setup<WAKE, QE, THREADS>(smem_raw);
-  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, false>(a, rg, smem_raw);
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, SPLIT,
+            std::conditional_t<SPLIT, SplitGrid, GridConst>>(a, rg, smem_raw);
 }
 
 template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN>
@@ -1106,7 +1164,7 @@ __device__ __forceinline__ void st_group(double* p, bool vec, const double v[4])
 __global__ void __launch_bounds__(kTrackThreads) k_flush(FlushArgs a) {
   const bool apply = a.apply && a.ts && a.ts->pending;
   const double pmean = apply ? a.ts->pending_mean : 0.0;
-  GridConst g{a.B, a.e0, 0.0, a.inv_estep, 0.0, 0.0, 0.0, kick_offset(a.e0, a.inv_estep)};
+  const GridConst g{a.B, 0.0, 0.0, a.kick_inv, 0.0, 0.0, 0.0, a.kick_off};
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   auto one = [&](double z, double& e) {
     if (apply) {
@@ -1511,7 +1569,24 @@ const void* pass_fn_w(int qe, int cfg) {
   }
 }
 
+// The pass on grids whose cells do not halve their bins: one layout, 32-bit counters.
+template <int Q>
+const void* pass_fn_split(int cfg) {
+  return (cfg & kPassWindowed)
+             ? (const void*)k_track_pass<true, Q, 4, 512, true, 1, true, true, true>
+             : (const void*)k_track_pass<true, Q, 4, 512, true, 1, true, false, true>;
+}
+
 const void* pass_fn(int wake, int qe, int cfg) {
+  if (cfg & kPassSplit) {
+    switch (qe) {
+      case QE_PHILOX:
+        return (cfg & kPassFastNormals) ? pass_fn_split<QE_PHILOX_FAST>(cfg)
+                                        : pass_fn_split<QE_PHILOX>(cfg);
+      case QE_DRAWS: return pass_fn_split<QE_DRAWS>(cfg);
+      default: return pass_fn_split<QE_OFF>(cfg);
+    }
+  }
   return wake ? pass_fn_w<true>(qe, cfg) : pass_fn_w<false>(qe, cfg);
 }
 
@@ -1652,6 +1727,12 @@ cudaError_t prepare_track_kernels(int max_smem) {
                 e = allow_dynamic_smem(batch_fn(w, q, c, u != 0), max_smem);
               if (e != cudaSuccess) return e;
             }
+  for (int q = 0; q < 3; ++q)
+    for (int k = 0; k < 4; ++k) {
+      const int c = split_pass_cfg((k & 1) ? kPassFastNormals : 0) | ((k & 2) ? kPassWindowed : 0);
+      cudaError_t e = allow_dynamic_smem(pass_fn(1, q, c), max_smem);
+      if (e != cudaSuccess) return e;
+    }
   return allow_dynamic_smem((const void*)k_histogram, max_smem);
 }
 

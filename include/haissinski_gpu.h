@@ -99,7 +99,9 @@ typedef struct hj_wake {
  * The histogram uses edge_first, edge_last and step(edges)
  * (src/utils.jl:367-380); the wake table and the interpolation use the
  * centers (src/wakefield.jl:39-42, :194-196).  A Julia caller passes the
- * values of its own ranges so that bins agree bit for bit.
+ * values of its own ranges so that bins agree bit for bit.  Where the centers
+ * are not the midpoints of such edges the histogram still follows the edges
+ * and the wake and its kick the centers (the pass takes a third longer then).
  */
 typedef struct hj_grid {
   int64_t nbins;
