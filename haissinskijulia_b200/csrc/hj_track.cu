@@ -439,29 +439,62 @@ __device__ __forceinline__ void particle_turn(double& z, double& e, double r, do
   acc_d += e - e_start;
 }
 
+// The shared-memory deposits of K particles.  One count atomic per particle whose
+// result nobody needs and one whose result only tells whether the 32-bit sum wrapped
+// (then the accumulator takes the 2^32, about one deposit in 500): the cell's count and
+// the histogram's bins both follow from the halves, so neither has an atomic of its own
+// (1e8 particles, 16384 bins: 0.743 ms a pass with three atomics).  The atomics of all K
+// particles are issued before any returned value is used, so their latencies overlap.
+// s_cnt and s_lo are the shared arrays offset by the window's start: half h's counter is
+// s_cnt[h], or 16 bits of the word s_cnt[h >> 1] without N32; cell j's sum s_lo[j];
+// `spare` is the cell behind the window.
+template <int K, bool N32>
+__device__ __forceinline__ void add_deposits(const int (&cj)[K], const int (&ch)[K],
+                                             const uint32_t (&cq)[K], int spare, int B,
+                                             uint32_t* s_cnt, uint32_t* s_lo,
+                                             unsigned long long* __restrict__ acc) {
+  uint32_t onc[K], olo[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
+    else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * B + 1 + cj[k], 1ull << 32);
+  if (!N32) {
+    // 16-bit counters, the two halves of a cell in a word: the increment that
+    // takes a counter to 2^15 moves 2^15 counts to the accumulators (the counter
+    // has another 2^15 - 1 increments of room before the move lands)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int sh = (ch[k] & 1) << 4;
+      if (((onc[k] >> sh) & 0xFFFFu) == 0x7FFFu && cj[k] != spare) {
+        atomicSub(&s_cnt[cj[k]], 0x8000u << sh);
+        add_halves(acc, B, ch[k], 0x8000ull);
+      }
+    }
+  }
+}
+
 // Moments and deposits of K particles' new z: Σz, Σz², the count of z's half cell
-// and, in the kick-table cell the next pass reads for this z, Σ w·2^24.  One
-// count atomic per particle whose result nobody needs and one whose result only
-// tells whether the 32-bit sum wrapped (then the accumulator takes the 2^32, about
-// one deposit in 500): the cell's count and the histogram's bins both follow
-// from the halves, so neither has an atomic of its own (1e8 particles, 16384
-// bins: 0.743 ms a pass with three atomics).  The atomics of all K particles are
-// issued before any returned value is used, so their latencies overlap.  s_cnt
-// and s_lo are the shared arrays offset by the window's start: half h's counter is
-// s_cnt[h], or 16 bits of the word s_cnt[h >> 1] without N32; cell j's sum s_lo[j].
+// and, in the kick-table cell the next pass reads for this z, Σ w·2^24.
 // Particles that need the reference's rounding, or lie off the grid (cell_half), and
 // with WIN those outside the window, are sorted out first: the latter's deposits go
 // to global memory, and in shared memory they take the spare cell behind the window,
 // which nobody reads.  So the deposits themselves run straight through for all, and a
 // bunch wider than its window pays for its own outliers alone.  us a pass of 2e7
 // particles at 16384 bins, bunches 1, 1.2, 1.5 and 2 times as long as their grid
-// assumes: 147 150 163 184; with one branch for the group, its other side one by one,
-// 168 230 349 351; with three atomics and a branch per particle 157 162 179 196 (4096
-// bins: 138 139 139 142, 138 138 148 223 and 147 for any length).
-// MASK: the outliers as a mask, which takes fewer registers than a flag each: the
-// batched pass spills otherwise (us a turn of 256 bunches 869 against 959, of 32 of
-// 1e6 258 against 277), the plain pass is 2 % faster with flags.
-template <int K, bool N32, bool WIN, bool MASK = true, class G>
+// assumes: 144 148 158 176; with one branch for the group, its other side one by one,
+// 165 229 346 338; with three atomics and a branch per particle 157 162 179 196 (4096
+// bins: 135 135 135 142, 136 137 145 216 and 147 for any length).
+// TWICE: the deposits once more behind the sorting, so that a group without outliers
+// goes straight from its test to them: the plain pass at 4096 bins, where it helps
+// (139 -> 135); the batched pass loses by it (256 bunches 866 -> 884 us a turn) and
+// the windowed one gains nothing.
+template <int K, bool N32, bool WIN, bool TWICE = false, class G>
 __device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
                                               const PassWindow& hw, double& acc_z,
                                               double& acc_z2, int32_t& n_out, uint32_t* s_cnt,
@@ -470,22 +503,19 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
   int cj[K], ch[K];
   uint32_t cq[K];
   bool fast[K], plain = true;
-  unsigned rare = 0u;                     // for cell_half: near a bin edge or off the grid
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     acc_z += z[k];
     acc_z2 = fma(z[k], z[k], acc_z2);
-    const bool ok = cell_half_fast(z[k], g, cj[k], ch[k], cq[k]);
-    if (MASK) rare |= ok ? 0u : 1u << k;
-    else plain &= fast[k] = ok;
+    fast[k] = cell_half_fast(z[k], g, cj[k], ch[k], cq[k]);
+    plain &= fast[k];
     if (WIN) plain &= (uint32_t)(cj[k] - hw.w0) < hw.h;
   }
   const int spare = hw.w0 + (int)hw.h;
-  if (MASK || !plain) {
-    if (!MASK) {
+  if (!plain) {
+    unsigned rare = 0u;
 #pragma unroll
-      for (int k = 0; k < K; ++k) rare |= fast[k] ? 0u : 1u << k;
-    }
+    for (int k = 0; k < K; ++k) rare |= fast[k] ? 0u : 1u << k;
 #pragma unroll 1
     while (rare) {                        // rolled: out of the main loop's registers
       const int k = K == 1 ? 0 : __ffs((int)rare) - 1;
@@ -497,7 +527,6 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
       uint32_t q;
       cell_half(zk, g, j, h, q, n_out, 1);
       if (G::split) count_bin(zk, g, hw, s_cnt, acc, n_out, 1);
-      if (WIN) plain &= (uint32_t)(j - hw.w0) < hw.h;
 #pragma unroll
       for (int m = 0; m < K; ++m)
         if (k == m) {
@@ -506,7 +535,7 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
           cq[m] = q;
         }
     }
-    if (WIN && !plain) {
+    if (WIN) {
 #pragma unroll
       for (int k = 0; k < K; ++k)
         if ((uint32_t)(cj[k] - hw.w0) >= hw.h) {
@@ -517,31 +546,12 @@ __device__ __forceinline__ void deposit_group(const double (&z)[K], const G& g,
           cq[k] = 0u;
         }
     }
-  }
-  uint32_t onc[K], olo[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (N32) atomicAdd(&s_cnt[ch[k]], 1u);
-    else onc[k] = atomicAdd(&s_cnt[cj[k]], 1u << ((ch[k] & 1) << 4));
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) olo[k] = atomicAdd(&s_lo[cj[k]], cq[k]);
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-    if (olo[k] + cq[k] < olo[k]) atomicAdd(acc + 2 * g.B + 1 + cj[k], 1ull << 32);
-  if (!N32) {
-    // 16-bit counters, the two halves of a cell in a word: the increment that
-    // takes a counter to 2^15 moves 2^15 counts to the accumulators (the counter
-    // has another 2^15 - 1 increments of room before the move lands)
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int sh = (ch[k] & 1) << 4;
-      if (((onc[k] >> sh) & 0xFFFFu) == 0x7FFFu && !(WIN && cj[k] == spare)) {
-        atomicSub(&s_cnt[cj[k]], 0x8000u << sh);
-        add_halves(acc, g.B, ch[k], 0x8000ull);
-      }
+    if (TWICE) {
+      add_deposits<K, N32>(cj, ch, cq, spare, g.B, s_cnt, s_lo, acc);
+      return;
     }
   }
+  add_deposits<K, N32>(cj, ch, cq, spare, g.B, s_cnt, s_lo, acc);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -836,8 +846,8 @@ __device__ __forceinline__ void pass_setup(unsigned char* smem_raw) {
   }
 }
 
-template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN, bool MASK,
-          class G = GridConst>
+template <bool WAKE, int QE, int PPT, int THREADS, bool PREFETCH, bool N32, bool WIN,
+          bool TWICE = false, class G = GridConst>
 __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg,
                                           unsigned char* smem_raw) {
   // dynamic shared memory: RF table [128] | the ziggurat's rows [2048] (a.zig) |
@@ -1025,7 +1035,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
       es[j] = keep ? e0 : ee[j];
     }
     if (WAKE)
-      deposit_group<PPT, N32, WIN, MASK>(zz, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
+      deposit_group<PPT, N32, WIN, TWICE>(zz, g, kw, acc_z, acc_z2, n_out, s_cnt, s_lo, a.acc);
     stp<PPT>(a.z + PPT * q, zs);
     stp<PPT>(a.dE + PPT * q, es);
     if (kDefer) {
@@ -1086,7 +1096,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_track_pass(PassArgs a) {
                      groups * PPT, blockIdx.x == 0 ? (int32_t)(a.n - groups * PPT) : 0,
                      (int32_t)blockIdx.x};
   pass_setup<WAKE, QE, THREADS>(smem_raw);
-  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, SPLIT,
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, !WIN,
             std::conditional_t<SPLIT, SplitGrid, GridConst>>(a, rg, smem_raw);
 }
 
@@ -1098,7 +1108,7 @@ __device__ __forceinline__ void run_chunk(const PassArgs* __restrict__ bunches,
   const int64_t groups = ch.count / PPT & ~(int64_t)31;
   const PassRange rg{ch.first / PPT, THREADS, ch.first / PPT + groups,
                      ch.first + groups * PPT, (int32_t)(ch.count - groups * PPT), ch.part};
-  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN, true>(a, rg, smem_raw);
+  pass_body<WAKE, QE, PPT, THREADS, PREFETCH, N32, WIN>(a, rg, smem_raw);
 }
 
 // One turn over a batch of bunches.  Chunk c of the chunk table (a
