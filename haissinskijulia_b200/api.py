@@ -678,8 +678,9 @@ class Batch:
 
     pool_particles: particle capacity (16 B each on the device); max_bunches:
     bunch slots; max_nbins: largest bin count; chunk: particles per block of
-    the pass (multiple of 4; small bunches are split finer, large ones up to
-    twice as coarse); layout: pass thread layout (-1 = default).
+    the pass (multiple of 4; the default 65536 leaves the size to the library,
+    by each bunch's particles and max_bunches); layout: pass thread layout (-1 =
+    default).
     """
 
     def __init__(self, ctx: Context, pool_particles: int, max_bunches: int, max_nbins: int,

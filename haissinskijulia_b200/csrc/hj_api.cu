@@ -484,7 +484,7 @@ hj_status hj_impl::bunch_create_begin(hj_ctx* ctx, double* d_z, double* d_dE, in
   if (chunk > 0) {
     b->batch_member = true;
     b->chunk = chunk;
-    b->nblk = (int)std::max<int64_t>((n + b->chunk - 1) / b->chunk, 1);
+    b->nblk = (int)std::max<int64_t>(member_chunks(n, b->chunk), 1);
   } else {
     const int bps = track_blocks_per_sm(b->B, b->qe_mode, b->use_wake, b->cfg);
     b->nblk = track_grid_size(n, b->B, ctx->num_sms, bps, b->cfg);

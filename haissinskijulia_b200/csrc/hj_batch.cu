@@ -13,8 +13,8 @@
 // k_batch_scan (one cluster per bunch); the kernels read the bunch
 // tables and the live counts from device memory and are launched over the
 // batch's capacity, so a captured graph stays valid as bunches come and go.
-// A bunch's chunking depends only on its own size and the batch's chunk size,
-// so its sums -- and its results -- do not depend on the other bunches.
+// A bunch's chunking depends only on its own size and on how the batch was created
+// (its chunk size and its slots), so its sums -- and its results -- do not depend on the other bunches.
 
 struct BatchMember {
   int64_t id = 0;
@@ -29,7 +29,7 @@ struct hj_batch {
   bool holds_ctx = false;                      // counted in ctx->live_objects
   cudaStream_t stream = nullptr;
   int cfg = 0;
-  int64_t chunk = 65536;
+  int64_t chunk = kDefaultChunk;
   int max_bunches = 0, max_B = 0, max_chunks = 0;
   // launch widths: the live counts rounded up to a power of two (a captured
   // graph is re-captured only when the live counts outgrow them)
@@ -121,8 +121,8 @@ hj_status batch_upload(hj_batch* bt) {
     fill_scan_args(b, bt->h_bins[k]);
     for (int c = 0; c < b->nblk; ++c) {
       BatchChunk ch;
-      ch.first = (int64_t)c * b->chunk;
-      ch.count = std::min<int64_t>(b->chunk, b->n - ch.first);
+      ch.first = member_first(c, b->chunk);
+      ch.count = member_end(c, b->n, b->chunk) - ch.first;
       ch.bunch = k;
       ch.part = c;
       if (nch >= bt->max_chunks) return set_err(ctx, HJ_ERR_STATE, "batch chunk table overflow");
@@ -232,8 +232,8 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   bt->max_B = max_nbins;
   bt->cfg = auto_pass_layout(layout, max_nbins, pool_particles);
   bt->pool_n = (pool_particles + 3) / 4 * 4;
-  // a member has at most n / chunk + 1 chunks, or member_blocks smaller ones
-  // (member_chunk)
+  // a member has at most n / chunk + 1 chunks, or member_blocks ones of the default
+  // chunk's rule (member_chunk)
   bt->max_chunks = (int)std::min<int64_t>(
       bt->pool_n / chunk + (member_blocks(max_bunches) + 1) * (int64_t)max_bunches + 1, INT32_MAX);
   HJ_CUDA(ctx, cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking));
@@ -284,7 +284,7 @@ extern "C" hj_status hj_batch_create(hj_ctx* ctx, int64_t pool_particles, int32_
   if (max_nbins > kMaxBins)
     return set_err(ctx, HJ_ERR_TOO_LARGE, "max_nbins = %d exceeds the supported %lld",
                    max_nbins, (long long)kMaxBins);
-  if (chunk_particles == 0) chunk_particles = 65536;
+  if (chunk_particles == 0) chunk_particles = kDefaultChunk;
   if (chunk_particles < 4 || chunk_particles % 4 || chunk_particles > kMaxBlockParticles)
     return set_err(ctx, HJ_ERR_ARG, "chunk_particles must be a positive multiple of 4, at most %lld",
                    (long long)kMaxBlockParticles);
@@ -389,8 +389,9 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   }
   p.b = new hj_bunch();
   hj_status s = bunch_create_begin(ctx, dz, de, n, params, wake, nbins, nullptr, seed,
-                                   (void*)bt->stream, p.b, member_chunk(n, bt->chunk, bt->max_bunches), bt->cfg, direct ? z : nullptr,
-                                   direct ? dE : nullptr);
+                                   (void*)bt->stream, p.b,
+                                   member_chunk(n, bt->chunk, bt->max_bunches), bt->cfg,
+                                   direct ? z : nullptr, direct ? dE : nullptr);
   if (s == HJ_OK && p.b->nblk > bt->max_chunks) s = set_err(ctx, HJ_ERR_FULL, "chunk table full");
   if (s != HJ_OK) {
     batch_add_abort(bt, p);

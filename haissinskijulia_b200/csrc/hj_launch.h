@@ -62,28 +62,41 @@ inline int resolve_pass_request(int r, int automatic) {
 }
 
 // Particles per block of a batch member of n particles, in a batch of `slots`
-// bunches created with `chunk` particles per block: member_blocks(slots) blocks of
-// kMinChunk to 2 chunk particles.  A block costs about 8 us beside its particles (1
+// bunches created with `chunk` particles per block.  A chunk of the caller's own is
+// taken as it is.  The default one leaves the size to this rule: member_blocks(slots)
+// blocks of kMinChunk to 2 kDefaultChunk particles.  A block costs about 8 us beside its particles (1
 // us a thousand), so large bunches take large blocks, while a batch of few or
 // small bunches must not wait for one block each: eight, or what fills the SMs
-// twice when every slot is taken.  Measured, us a turn, against `chunk` = 65536 for
+// twice when every slot is taken.  Measured, us a turn, against 65536 for
 // all: 256 bunches of 1e4 to 2e6 874 -> 861, 32 bunches of 1e6 312 -> 278, 64 of 1e4
 // to 5e4 62 -> 37, 16 served ones (1.6e6 particles) 86 -> 67 with eight blocks.
 // A function of n and of how the batch was created: a bunch's sums do not depend
 // on the bunches that share it.
+constexpr int64_t kDefaultChunk = 65536;
 constexpr int64_t kMinChunk = 16384;
 inline int64_t member_blocks(int64_t slots) {
   const int64_t b = 2 * 148 / (slots > 0 ? slots : 1);
   return b > 8 ? b : 8;
 }
 inline int64_t member_chunk(int64_t n, int64_t chunk, int64_t slots) {
+  constexpr int64_t kMost = kMaxBlockParticles & ~int64_t(127);
+  if (chunk != kDefaultChunk) return chunk < kMost - 128 ? chunk : kMost;
   const int64_t blocks = member_blocks(slots);
   int64_t c = (n + blocks - 1) / blocks;
   c = (c + 127) / 128 * 128;                       // whole warps of four-particle groups
   if (c < kMinChunk) c = kMinChunk;
-  int64_t most = 2 * chunk;
-  if (most > (kMaxBlockParticles & ~int64_t(127))) most = kMaxBlockParticles & ~int64_t(127);
-  return c < most ? c : most;
+  return c < 2 * kDefaultChunk ? c : 2 * kDefaultChunk;
+}
+// First particle of block i of a member split into blocks of `chunk`: on a whole warp of
+// four-particle groups, so that only the bunch's last block has particles left over by
+// its warps, while the blocks keep `chunk` particles on average (a chunk that fills the
+// GPU's waves still does).
+inline int64_t member_first(int64_t i, int64_t chunk) {
+  return chunk >= 128 ? i * chunk & ~int64_t(127) : i * chunk;
+}
+inline int64_t member_chunks(int64_t n, int64_t chunk) { return (n + chunk - 1) / chunk; }
+inline int64_t member_end(int64_t i, int64_t n, int64_t chunk) {
+  return i + 1 < member_chunks(n, chunk) ? member_first(i + 1, chunk) : n;
 }
 
 // Blocks of the particle pass: enough to fill the GPU, but each block should

@@ -229,8 +229,9 @@ def autotune(ctx: Context, points: List[Point], *, trial_turns: int = 64,
              chunks=None, layouts=(8, 9, 13), graph_turns=(8, 32),
              sample: int = 64) -> Tuning:
     """Times each candidate (particles per block, pass layout, graph turns) on
-    up to `sample` of the points for `trial_turns` turns after a warm-up and
-    returns the fastest.  Default block sizes: 16K, 64K, 256K particles and,
+    up to `sample` of the points for `trial_turns` turns after a warm-up, in a
+    batch with a slot for every point (as run_batched's), and returns the
+    fastest.  Default block sizes: 16K, the library's choice (65536), 256K and,
     when the trial runs the whole workload, those that fill one, two or four
     waves of the GPU with it (on a sample they would be sized for the sample)."""
     if chunks is None:
@@ -247,7 +248,7 @@ def autotune(ctx: Context, points: List[Point], *, trial_turns: int = 64,
     for c in chunks:
         for L in layouts:
             for K in graph_turns:
-                bt = Batch(ctx, pool, len(pts), max(p.nbins for p in pts), chunk=c, layout=L,
+                bt = Batch(ctx, pool, len(points), max(p.nbins for p in pts), chunk=c, layout=L,
                            graph_turns=K)
                 try:
                     for p, cfg in data:
