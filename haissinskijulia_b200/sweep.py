@@ -26,7 +26,9 @@ turn, turn blocks replayed from a CUDA graph.
 """
 from __future__ import annotations
 
+import ctypes
 import math
+import mmap
 import threading
 import time
 from dataclasses import dataclass, field
@@ -121,27 +123,36 @@ class Tuning:
     resident: bool = False      # resident blocks on a chunk queue, or one block per chunk
 
 
+_MADV_POPULATE_WRITE = 23      # Linux 5.14: faults pages in, leaves their contents
+_libc = ctypes.CDLL(None)
+_libc.madvise.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
+
+
 class _Outputs:
-    """Host arrays for the final particles of all points, slices of one block per
-    coordinate.  Fresh pages cost more to fault in than the copies into them (40
-    points, 64 MB: 20 ms one array each, 7 ms as large blocks, which get huge
-    pages), so a thread touches them while the GPU runs the first turns."""
+    """Host arrays for the final particles of all points, each an array of its own
+    (keeping one solve's particles keeps no other's alive).  Fresh pages cost more to
+    fault in one by one than the copies into them, so a thread has them mapped, an array
+    at a time, while the GPU runs the first turns (40 points, 64 MB, the whole call: 67
+    ms without it, 56 with the pages touched one by one, 45 so, 48 with slices of one
+    block).  Where the kernel cannot, the copies fault them in."""
 
     def __init__(self, points: List[Point]):
-        self._first = np.concatenate([[0], np.cumsum([p.n for p in points])])
-        total = int(self._first[-1])
-        self._z, self._dE = np.empty(total), np.empty(total)
-        self._thread = threading.Thread(target=self._touch, daemon=True)
+        self._arrays = [(np.empty(p.n), np.empty(p.n)) for p in points]
+        self._thread = threading.Thread(target=self._populate, daemon=True)
         self._thread.start()
 
-    def _touch(self) -> None:
-        for a in (self._z, self._dE):
-            a[::512] = 0.0                      # one double a page
+    def _populate(self) -> None:
+        page = mmap.PAGESIZE
+        for i in range(len(self._arrays)):
+            for a in self._arrays[i] or ():
+                first = -(-a.ctypes.data // page) * page          # whole pages of the array
+                size = (a.ctypes.data + a.nbytes) // page * page - first
+                if size > 0:
+                    _libc.madvise(first, size, _MADV_POPULATE_WRITE)
 
     def of(self, i: int):
-        self._thread.join()
-        s = slice(int(self._first[i]), int(self._first[i + 1]))
-        return self._z[s], self._dE[s]
+        pair, self._arrays[i] = self._arrays[i], None
+        return pair
 
 
 def run_batched(ctx: Context, points: List[Point], *, pool_particles: Optional[int] = None,
