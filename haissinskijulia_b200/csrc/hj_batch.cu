@@ -167,7 +167,7 @@ hj_status batch_launch_turn(hj_batch* bt) {
                                  bt->resident ? bt->d_counts + 2 : nullptr, bt->resident_blocks,
                                  bt->stream));
   HJ_CUDA(ctx, launch_batch_scan(bt->d_bins, bt->d_counts + 1, bt->grid_bunches, bt->max_B,
-                                 bt->max_bunches, bt->stream));
+                                 ctx->num_sms / bt->max_bunches, bt->stream));
   return HJ_OK;
 }
 
@@ -235,7 +235,8 @@ static hj_status batch_create_impl(hj_ctx* ctx, int64_t pool_particles, int32_t 
   // a member has at most n / chunk + 1 chunks, or member_blocks ones of the default
   // chunk's rule (member_chunk)
   bt->max_chunks = (int)std::min<int64_t>(
-      bt->pool_n / chunk + (member_blocks(max_bunches) + 1) * (int64_t)max_bunches + 1, INT32_MAX);
+      bt->pool_n / chunk + (member_blocks(max_bunches, ctx->num_sms) + 1) * (int64_t)max_bunches + 1,
+      INT32_MAX);
   HJ_CUDA(ctx, cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking));
   // the pool and the tables: one device and one pinned block of the context's cache
   const size_t nb = (size_t)max_bunches, nc = (size_t)bt->max_chunks;
@@ -390,7 +391,7 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   p.b = new hj_bunch();
   hj_status s = bunch_create_begin(ctx, dz, de, n, params, wake, nbins, nullptr, seed,
                                    (void*)bt->stream, p.b,
-                                   member_chunk(n, bt->chunk, bt->max_bunches), bt->cfg,
+                                   member_chunk(n, bt->chunk, bt->max_bunches, ctx->num_sms), bt->cfg,
                                    direct ? z : nullptr, direct ? dE : nullptr);
   if (s == HJ_OK && p.b->nblk > bt->max_chunks) s = set_err(ctx, HJ_ERR_FULL, "chunk table full");
   if (s != HJ_OK) {

@@ -255,8 +255,9 @@ size_t bins_smem_bytes(int H);
 // ---- launchers (hj_scan.cu) ----
 cudaError_t prepare_scan_kernels(int max_smem);    // once per device: dynamic smem limits
 cudaError_t launch_scan(const ScanArgs& a, cudaStream_t st);
+// room: SMs per slot of the batch.
 cudaError_t launch_batch_scan(const ScanArgs* d_bunches, const int32_t* d_n_bunches,
-                              int max_bunches, int max_B, int slots, cudaStream_t st);
+                              int max_bunches, int max_B, int room, cudaStream_t st);
 
 // ---- context access for entry points outside hj_api.cu ----
 int ctx_device(const hj_ctx* ctx);

@@ -74,14 +74,14 @@ inline int resolve_pass_request(int r, int automatic) {
 // on the bunches that share it.
 constexpr int64_t kDefaultChunk = 65536;
 constexpr int64_t kMinChunk = 16384;
-inline int64_t member_blocks(int64_t slots) {
-  const int64_t b = 2 * 148 / (slots > 0 ? slots : 1);
+inline int64_t member_blocks(int64_t slots, int64_t sms = 148) {
+  const int64_t b = 2 * sms / (slots > 0 ? slots : 1);
   return b > 8 ? b : 8;
 }
-inline int64_t member_chunk(int64_t n, int64_t chunk, int64_t slots) {
+inline int64_t member_chunk(int64_t n, int64_t chunk, int64_t slots, int64_t sms = 148) {
   constexpr int64_t kMost = kMaxBlockParticles & ~int64_t(127);
   if (chunk != kDefaultChunk) return chunk < kMost - 128 ? chunk : kMost;
-  const int64_t blocks = member_blocks(slots);
+  const int64_t blocks = member_blocks(slots, sms);
   int64_t c = (n + blocks - 1) / blocks;
   c = (c + 127) / 128 * 128;                       // whole warps of four-particle groups
   if (c < kMinChunk) c = kMinChunk;

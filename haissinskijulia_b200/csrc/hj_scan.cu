@@ -426,13 +426,12 @@ ScanForm plain_scan_form(int B) {
   return plain_form<8, 512, 4>();
 }
 
-// A batch of `slots` bunches of up to max_B bins: the most CTAs per bunch that fit the
-// SMs at once for all slots, beyond that the fewest that hold the bins (us a turn:
+// A batch of bunches of up to max_B bins with `room` SMs for each of its slots: the most
+// CTAs per bunch that fit the SMs at once for all slots, beyond that the fewest that hold the bins (us a turn:
 // 32 bunches of 8192 bins 268 -> 259 with 4 x 512 x 4 instead of 4 x 256 x 8, 64 of
 // 2048 37 -> 31, 16 of up to 8192 48 -> 44; 256 of 4096 877 -> 869 with 1 x 512 x 8
 // instead of 2 x 256 x 8, 886 with 4 x 256 x 4).
-ScanForm batch_scan_form(int max_B, int slots) {
-  const int room = 148 / (slots > 0 ? slots : 1);     // CTAs a slot may take
+ScanForm batch_scan_form(int max_B, int room) {
   if (max_B <= 512) return batch_form<1, 256, 2>();
   if (max_B <= 1024) return batch_form<1, 512, 2>();
   if (max_B <= 2048) {
@@ -460,8 +459,8 @@ ScanForm batch_scan_form(int max_B, int slots) {
 cudaError_t prepare_scan_kernels(int max_smem) {
   for (int B = 256; B <= (int)kMaxBins; B *= 2) {
     cudaError_t e = allow_dynamic_smem(plain_scan_form(B).fn, max_smem);
-    for (int slots = 16; slots <= 256 && e == cudaSuccess; slots *= 2)
-      e = allow_dynamic_smem(batch_scan_form(B, slots).fn, max_smem);
+    for (int room = 1; room <= 8 && e == cudaSuccess; room *= 2)
+      e = allow_dynamic_smem(batch_scan_form(B, room).fn, max_smem);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -475,8 +474,8 @@ cudaError_t launch_scan(const ScanArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_batch_scan(const ScanArgs* d_bunches, const int32_t* d_n_bunches,
-                              int max_bunches, int max_B, int slots, cudaStream_t st) {
-  const ScanForm f = batch_scan_form(max_B, slots);
+                              int max_bunches, int max_B, int room, cudaStream_t st) {
+  const ScanForm f = batch_scan_form(max_B, room);
   void* args[] = {const_cast<ScanArgs**>(&d_bunches), const_cast<int32_t**>(&d_n_bunches)};
   PdlConfig l(dim3(f.C * (max_bunches > 0 ? max_bunches : 1)), dim3(f.NT + 32), f.smem, st);
   return cudaLaunchKernelExC(&l.cfg, f.fn, args);

@@ -1851,7 +1851,7 @@ cudaError_t launch_bunch_setup(void* zero, size_t zero_bytes, double2* rf_table,
                                cudaStream_t st) {
   SetupArgs a{(uint4*)zero, (int64_t)(zero_bytes / 16), rf_table, V,
               sincos[0], sincos[1], sincos[2], sincos[3], ts, t};
-  const int64_t blocks = std::min<int64_t>((a.zero_words + 1023) / 1024, 148);
+  const int64_t blocks = (a.zero_words + 1023) / 1024;   // 57 at 16384 bins
   k_bunch_setup<<<(int)std::max<int64_t>(blocks, 1), 256, 0, st>>>(a);
   return cudaGetLastError();
 }

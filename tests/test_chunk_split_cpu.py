@@ -17,8 +17,9 @@ DRIVER = r"""
 #include "hj_launch.h"
 int main() {
   long long n, chunk, slots;
-  while (scanf("%lld %lld %lld", &n, &chunk, &slots) == 3) {
-    const int64_t c = hj::member_chunk(n, chunk, slots), k = hj::member_chunks(n, c);
+  long long sms;
+  while (scanf("%lld %lld %lld %lld", &n, &chunk, &slots, &sms) == 4) {
+    const int64_t c = hj::member_chunk(n, chunk, slots, sms), k = hj::member_chunks(n, c);
     printf("%lld %lld", (long long)c, (long long)k);
     for (int64_t i = 0; i < k; ++i)
       printf(" %lld %lld", (long long)hj::member_first(i, c), (long long)hj::member_end(i, n, c));
@@ -38,8 +39,9 @@ def split(tmp_path_factory):
     exe = str(d / "s")
     subprocess.run([gxx, "-std=c++17", "-I", CSRC, str(d / "s.cpp"), "-o", exe], check=True)
 
-    def run(cases):
-        out = subprocess.run([exe], input="".join("%d %d %d\n" % c for c in cases),
+    def run(cases, sms=148):
+        text = "".join("%d %d %d %d\n" % (*c, sms) for c in cases)
+        out = subprocess.run([exe], input=text,
                              capture_output=True, text=True, check=True).stdout.splitlines()
         rows = []
         for line in out:
@@ -81,3 +83,9 @@ def test_the_autotuner_tries_different_splits(split, points):
     seen = {tuple(len(b) for _, b in split([(p.n, c, len(points)) for p in points]))
             for c in chunks}
     assert len(seen) == len(chunks)
+
+
+def test_the_default_follows_the_number_of_sms(split):
+    for sms in (37, 74, 148):
+        assert len(split([(10_000_000, 65536, 2)], sms)[0][1]) == max(sms, -(-10_000_000 // 131072))
+        assert len(split([(1_000_000, 65536, 32)], sms)[0][1]) == max(8, 2 * sms // 32)
