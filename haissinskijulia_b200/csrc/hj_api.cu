@@ -6,6 +6,7 @@
 // (E0, pending kick, turn counter) lives in device memory, so turns never
 // wait for the host.
 #include <memory>
+#include "hj_ranges.h"
 #include "hj_state.h"
 
 namespace {
@@ -81,22 +82,15 @@ hj_status scratch(hj_ctx* ctx, size_t bytes, void** out) {
 // ---- block cache.  A bunch's buffers come from one device block and one
 // pinned block; released blocks are kept (up to a cap) for the next request
 // of the same size class, so admitting and retiring bunches of recurring
-// sizes allocates nothing.  Size classes: 2^k x {1, 1.25, 1.5, 1.75}.
+// sizes allocates nothing (hj_ranges::size_class).
 constexpr size_t kDevCacheCap = size_t(8) << 30;
 constexpr size_t kHostCacheCap = size_t(256) << 20;
-
-size_t size_class(size_t b) {
-  if (b <= 4096) return 4096;
-  const int lg = 63 - __builtin_clzll((unsigned long long)b);
-  const size_t step = size_t(1) << (lg - 2);
-  return (b + step - 1) / step * step;
-}
 
 constexpr size_t kSlabBlockMax = size_t(16) << 20;
 constexpr size_t kSlabSize = size_t(256) << 20;
 
 hj_status cache_take(hj_ctx* ctx, bool host, size_t bytes, void** out, size_t* cap) {
-  const size_t c = size_class(bytes);
+  const size_t c = hj_ranges::size_class(bytes, host ? kHostCacheCap : kDevCacheCap);
   auto& fl = host ? ctx->host_free : ctx->dev_free;
   auto it = fl.find(c);
   if (it != fl.end()) {

@@ -1,9 +1,11 @@
-// hj_ranges.h -- the free ranges of a batch's particle pool (host only, no
-// CUDA), first fit: admission takes room for a bunch, retirement gives it
-// back and merges it with its free neighbours.
+// hj_ranges.h -- memory bookkeeping (host only, no CUDA): the free ranges of a
+// batch's particle pool, first fit (admission takes room for a bunch, retirement
+// gives it back and merges it with its free neighbours), and the sizes of cached
+// blocks.
 #pragma once
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <utility>
 #include <vector>
@@ -52,6 +54,17 @@ inline int64_t largest(const Ranges& fr) {
   int64_t m = 0;
   for (const auto& r : fr) m = std::max(m, r.second);
   return m;
+}
+
+// Size of the block that serves b bytes: 2^k x {1, 1.25, 1.5, 1.75}, so that requests of
+// similar sizes reuse each other's blocks, at least 4096.  A request beyond what the cache
+// keeps (`kept` bytes) is not reused anyway and takes only its own pages: a turn log or a
+// pool may need most of the device's memory.
+inline size_t size_class(size_t b, size_t kept) {
+  if (b <= 4096) return 4096;
+  const int lg = b > kept ? 14 : 63 - __builtin_clzll((unsigned long long)b);
+  const size_t step = size_t(1) << (lg - 2);
+  return (b + step - 1) / step * step;
 }
 
 }  // namespace hj_ranges

@@ -190,7 +190,6 @@ hj_status scratch(hj_ctx* ctx, size_t bytes, void** out);
 
 // Block cache (see hj_api.cu): blocks by size class, small device blocks
 // carved from slabs.
-size_t size_class(size_t b);
 hj_status cache_take(hj_ctx* ctx, bool host, size_t bytes, void** out, size_t* cap);
 void cache_give(hj_ctx* ctx, bool host, void* p, size_t cap);
 void cache_clear(hj_ctx* ctx, bool slabs = false);
