@@ -2,6 +2,8 @@
 // pool, one turn-state array, per turn one batched pass over a chunk table,
 // and one batched bins step; turn blocks
 // replayed from a CUDA graph.
+#include <cuda.h>
+
 #include "hj_ranges.h"
 #include "hj_state.h"
 
@@ -68,15 +70,34 @@ struct hj_batch {
 
 namespace {
 
-// Whether p is an array of doubles in the memory of the context's device.
-bool on_device(hj_ctx* ctx, const void* p) {
+// Whether p is an array of n doubles in one allocation of the context's device, so that
+// a kernel may use it.  What is not (host, managed or peer memory, odd addresses, arrays
+// that end before n) is left to a copy, which takes it or refuses it.
+bool on_device(hj_ctx* ctx, const void* p, int64_t n) {
   if ((uintptr_t)p & 7) return false;
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+  using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Fn get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess) {
+      cudaGetLastError();
+      return (Fn) nullptr;
+    }
+    return q == cudaDriverEntryPointSuccess ? (Fn)f : (Fn) nullptr;
+  }();
+  unsigned type = 0, managed = 0;
+  int device = -1;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  CUpointer_attribute ask[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                               CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                               CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                               CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[] = {&type, &managed, &device, &base, &size};
+  if (!get || get(5, ask, to, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_DEVICE && !managed && device == ctx->device &&
+         hj_ranges::covers(base, size, (uint64_t)(uintptr_t)p, sizeof(double) * (uint64_t)n);
 }
 
 // Enqueues bunch b's retirement: pending kick and re-centring, moments, turn state
@@ -86,7 +107,7 @@ bool on_device(hj_ctx* ctx, const void* p) {
 hj_status enqueue_take(hj_batch* bt, hj_bunch* b, double* z_out, double* dE_out, bool keep) {
   hj_ctx* ctx = bt->ctx;
   const bool direct =
-      !keep && z_out && dE_out && on_device(ctx, z_out) && on_device(ctx, dE_out);
+      !keep && z_out && dE_out && on_device(ctx, z_out, b->n) && on_device(ctx, dE_out, b->n);
   const bool none = !keep && !z_out && !dE_out;
   HJ_TRY(launch_moments(b, 1, direct ? z_out : none ? nullptr : b->z,
                         direct ? dE_out : none ? nullptr : b->dE, true, true));
@@ -374,7 +395,7 @@ static hj_status batch_add_begin(hj_batch* bt, const double* z, const double* dE
   double* de = bt->pool_dE + p.start;
   cudaError_t e = cudaSuccess;
   // from this device's memory the moments' kernel copies the particles as it reads them
-  const bool direct = z && on_device(ctx, z) && on_device(ctx, dE);
+  const bool direct = z && on_device(ctx, z, n) && on_device(ctx, dE, n);
   if (direct) {
   } else if (z) {
     e = cudaMemcpyAsync(dz, z, sizeof(double) * n, cudaMemcpyDefault, bt->stream);

@@ -1,7 +1,7 @@
 // hj_ranges.h -- memory bookkeeping (host only, no CUDA): the free ranges of a
 // batch's particle pool, first fit (admission takes room for a bunch, retirement
-// gives it back and merges it with its free neighbours), and the sizes of cached
-// blocks.
+// gives it back and merges it with its free neighbours), the sizes of cached
+// blocks and the bounds of a caller's.
 #pragma once
 
 #include <algorithm>
@@ -65,6 +65,11 @@ inline size_t size_class(size_t b, size_t kept) {
   const int lg = b > kept ? 14 : 63 - __builtin_clzll((unsigned long long)b);
   const size_t step = size_t(1) << (lg - 2);
   return (b + step - 1) / step * step;
+}
+
+// Whether [p, p + bytes) lies in the allocation of `size` bytes at base.
+inline bool covers(uint64_t base, uint64_t size, uint64_t p, uint64_t bytes) {
+  return p >= base && p - base <= size && bytes <= size - (p - base);
 }
 
 }  // namespace hj_ranges
