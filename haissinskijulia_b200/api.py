@@ -672,9 +672,10 @@ class Batch:
     """Independent bunches advanced together on one GPU (hj_batch_*).
 
     Each bunch has its own particles, RF voltage, wake intensity, bins, seed
-    and turn count; every turn is one batched particle pass and one
-    batched bins step for all live bunches, and blocks of `graph_turns` turns replay a captured CUDA graph.  A bunch's results do
-    not depend on which other bunches share the batch.
+    and turn count; every turn is one batched particle pass and one batched bins
+    step for all live bunches, and blocks of `graph_turns` turns replay a captured
+    CUDA graph.  A bunch's results do not depend on which other bunches share the
+    batch.
 
     pool_particles: particle capacity (16 B each on the device); max_bunches:
     bunch slots; max_nbins: largest bin count; chunk: particles per block of

@@ -18,7 +18,7 @@ constexpr int64_t kMaxBlockParticles = (1 << 20) - 8;
 // particles).
 constexpr int kNumPassCfgs = 6;       // thread layouts of the fused pass
 constexpr int kPassLayoutMask = 7;    // layout bits of a pass configuration
-constexpr int kPassN32 = 8;           // + one 32-bit NGP counter per bin (else 16-bit pairs)
+constexpr int kPassN32 = 8;           // + 32-bit counters of a cell's halves (else 16-bit ones)
 constexpr int kPassFastNormals = 16;  // + single-precision quantum-excitation normals
 // Launch-only bit (never in a caller's configuration): the pass's hot window
 // holds fewer than all B + 1 cells, so its deposits are range-checked.
@@ -108,9 +108,10 @@ inline int track_grid_size(int64_t n, int B, int num_sms, int blocks_per_sm, int
   int64_t g = (n + per_block - 1) / per_block;
   int64_t cap = (int64_t)num_sms * blocks_per_sm;
   if (g > cap) g = cap;
-  // At most kMaxBlockParticles per block and turn.  Block b takes the groups of PPT particles b·T + t + k·g·T: at most
-  // ceil((n / PPT) / (g·T)) steps of T·PPT particles, and block 0 also
-  // the tail that whole warps leave over.  So g is raised until no block takes more steps than fit.
+  // At most kMaxBlockParticles per block and turn.  Block b takes the groups of PPT
+  // particles b·T + t + k·g·T: at most ceil((n / PPT) / (g·T)) steps of T·PPT particles,
+  // and block 0 also the tail that whole warps leave over.  So g is raised until no block
+  // takes more steps than fit.
   const int64_t threads = pass_cfg_threads(cfg);
   const int64_t steps = kMaxBlockParticles / ((int64_t)pass_cfg_ppt(cfg) * threads);
   const int64_t groups = n / pass_cfg_ppt(cfg);

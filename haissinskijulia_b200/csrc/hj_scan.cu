@@ -20,11 +20,11 @@
 // thread: the thread's suffix sum, a weighted shuffle scan over the warp, over
 // the warps, and (one cluster barrier) over the CTAs.  T[i-J], half a grid
 // away, is read from the CTA that holds it through distributed shared memory.
-// What bounds it is the chain of barriers and FP64 latencies, not bytes (72 B
-// per bin and turn) or operations (about 60 per bin).  Measured on B200 against
-// the FFT step, whole turns: 1e5 particles at 4096 bins 30.5 -> 21.8 us, 1e6 at
-// 10000 bins 67 -> 46 us, 32 bunches of 1e6 at 8192 bins 572 -> 441 us (with the
-// admissions, which need no FFT(W) any more).
+// What bounds it is the chain of barriers and FP64 latencies, not bytes (80 B
+// per bin and turn: 24 read, 24 cleared, 32 written) or operations (about 60 per
+// bin).  16384 bins, serialised: SCAN_US us against 42.7 for the FFT step and 10.1
+// for the merge of block partials that it needed.  A whole turn of 1e5 particles at
+// 4096 bins takes 15.5 us (30.5 with those two).
 #include <cooperative_groups.h>
 
 #include "hj_internal.h"

@@ -940,7 +940,7 @@ __device__ __forceinline__ void pass_body(const PassArgs& a, const PassRange& rg
   PassWindow kw{s_win, 0, 0u, 0u};
   if (WAKE) {
     int w0 = 0;
-    if (WIN && hot < nc) {   // even, so that the 16-bit pairs keep bin b at word b >> 1
+    if (WIN && hot < nc) {   // even, so that copy16_async of the kick window starts on 16 bytes
       int jm;
       double wm;
       kick_cell(ts->last_mean_z, g, jm, wm);
@@ -1226,12 +1226,13 @@ __global__ void __launch_bounds__(kTrackThreads) k_flush(FlushArgs a) {
 // sin hi, lo), filled when the kernels are prepared.
 __device__ double g_rf_unit[kRfTableSize][4];
 
-// a b as a sum of two doubles, a and b being such sums.
+// a b as a sum of two doubles, a and b being such sums (the product's error by one FMA,
+// T. J. Dekker, Numer. Math. 18, 1971).
 __device__ __forceinline__ double2 mul_dd(double ah, double al, double bh, double bl) {
   const double p = __dmul_rn(ah, bh);
   return make_double2(p, fma(ah, bh, -p) + fma(ah, bl, al * bh));
 }
-// x + y, |x| and |y| arbitrary (two-sum).
+// x + y, |x| and |y| arbitrary (D. E. Knuth's two-sum).
 __device__ __forceinline__ double2 add_dd(double2 x, double2 y) {
   const double s = __dadd_rn(x.x, y.x), t = __dsub_rn(s, x.x);
   const double e = __dadd_rn(__dsub_rn(x.x, __dsub_rn(s, t)), __dsub_rn(y.x, t));
@@ -1538,7 +1539,7 @@ cudaError_t allow_dynamic_smem(const void* fn, int max_smem_optin) {
 }
 
 namespace {
-// cfg: thread layout (bits 0-2) | kPassN32 (32-bit NGP counters) |
+// cfg: thread layout (bits 0-2) | kPassN32 (32-bit counters) |
 // kPassFastNormals | kPassWindowed (range-checked deposits; with the wake only)
 template <bool W, int Q, bool N, bool H>
 const void* pass_fn_wqnh(int layout) {

@@ -259,7 +259,7 @@ hj_status hj_bunch_observe(hj_bunch* b, double* d_z_out, double* d_dE_out, hj_re
 hj_status hj_bunch_finish(hj_bunch* b, hj_result* res);
 /* Device-time profiling of the turns enqueued while enabled: CUDA events are
  * recorded on the bunch's stream around each particle pass and each bins
- * step (histogram reduction + convolution + E0 update).  enable = 0 stops
+ * step (wake potential + kick table + E0 update).  enable = 0 stops
  * and clears.  No reference counterpart (the reference times whole calls
  * with BenchmarkTools, tests/benchmark_total.jl:343-369). */
 hj_status hj_bunch_set_profiling(hj_bunch* b, int32_t enable);
