@@ -64,12 +64,13 @@ inline int resolve_pass_request(int r, int automatic) {
 // Particles per block of a batch member of n particles, in a batch of `slots`
 // bunches created with `chunk` particles per block.  A chunk of the caller's own is
 // taken as it is.  The default one leaves the size to this rule: member_blocks(slots)
-// blocks of kMinChunk to 2 kDefaultChunk particles.  A block costs about 8 us beside its particles (1
-// us a thousand), so large bunches take large blocks, while a batch of few or
+// blocks of kMinChunk to 2 kDefaultChunk particles.  A block costs about 8 us beside its
+// particles (1 us a thousand), so large bunches take large blocks, while a batch of few or
 // small bunches must not wait for one block each: eight, or what fills the SMs
-// twice when every slot is taken.  Measured, us a turn, against 65536 for
-// all: 256 bunches of 1e4 to 2e6 874 -> 861, 32 bunches of 1e6 312 -> 278, 64 of 1e4
-// to 5e4 62 -> 37, 16 served ones (1.6e6 particles) 86 -> 67 with eight blocks.
+// twice when every slot is taken.  Measured, us a turn, against 65532 for
+// all: 256 bunches of 1e4 to 2e6 870 -> 862, 32 bunches of 1e6 303 -> 262, 64 of 1e4
+// to 5e4 58 -> 32, 16 served ones (1.6e6 particles) 81 -> 45; but 256 of 1e5 272 -> 319,
+// 148 of 1e5 144 -> 185, where a caller does better with blocks of their own.
 // A function of n and of how the batch was created: a bunch's sums do not depend
 // on the bunches that share it.
 constexpr int64_t kDefaultChunk = 65536;

@@ -22,7 +22,7 @@
 // away, is read from the CTA that holds it through distributed shared memory.
 // What bounds it is the chain of barriers and FP64 latencies, not bytes (80 B
 // per bin and turn: 24 read, 24 cleared, 32 written) or operations (about 60 per
-// bin).  16384 bins, serialised: SCAN_US us against 42.7 for the FFT step and 10.1
+// bin).  16384 bins, serialised: 13.9 us against 42.7 for the FFT step and 10.1
 // for the merge of block partials that it needed.  A whole turn of 1e5 particles at
 // 4096 bins takes 15.5 us (30.5 with those two).
 #include <cooperative_groups.h>
@@ -427,10 +427,10 @@ ScanForm plain_scan_form(int B) {
 }
 
 // A batch of bunches of up to max_B bins with `room` SMs for each of its slots: the most
-// CTAs per bunch that fit the SMs at once for all slots, beyond that the fewest that hold the bins (us a turn:
-// 32 bunches of 8192 bins 268 -> 259 with 4 x 512 x 4 instead of 4 x 256 x 8, 64 of
-// 2048 37 -> 31, 16 of up to 8192 48 -> 44; 256 of 4096 877 -> 869 with 1 x 512 x 8
-// instead of 2 x 256 x 8, 886 with 4 x 256 x 4).
+// CTAs per bunch that fit the SMs at once for all slots, beyond that the fewest that hold
+// the bins (us a turn: 32 bunches of 8192 bins 268 -> 259 with 4 x 512 x 4 instead of 4 x
+// 256 x 8, 64 of 2048 37 -> 31, 16 of up to 8192 48 -> 44; 256 of 4096 877 -> 869 with
+// 1 x 512 x 8 instead of 2 x 256 x 8, 886 with 4 x 256 x 4).
 ScanForm batch_scan_form(int max_B, int room) {
   if (max_B <= 512) return batch_form<1, 256, 2>();
   if (max_B <= 1024) return batch_form<1, 512, 2>();

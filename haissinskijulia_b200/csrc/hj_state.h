@@ -112,8 +112,8 @@ struct hj_bunch {
   TurnState* h_ts = nullptr;  // pinned
   // the buffers above are carved from one device block and one pinned block
   // of the context's cache; without uniform centres twP is the context's
-  // shared table and W, lam and Wf point into a block of their own (tables); pot, potd, acc and hist are the first zero_bytes of the
-  // arena's histogram part
+  // shared table and W, lam and Wf point into a block of their own (tables); pot,
+  // potd, acc and hist are the first zero_bytes of the arena's histogram part
   bool passed = false;                    // a pass has been enqueued
   bool batch_member = false;
   int64_t chunk = 0;                      // a member's particles per block of the pass

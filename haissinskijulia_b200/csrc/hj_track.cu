@@ -154,9 +154,9 @@ __device__ __forceinline__ void cic_cell(double z, const GridConst& g, int& idx,
 }
 
 // Cell of the kick table (B + 1 cells): v = z/Δe + 1/2 - e0/Δe (one FMA; where a
-// caller's edges and centres do not fit together, z/Δc + 1 - c1/Δc), j = floor(v) clamped to [0, B], w = v - floor(v).  Cell j >= 1 is the
-// reference's interpolation cell j-1 between centres c[j-1] and c[j]
-// (src/wakefield.jl:64-78); cells 0 and B hold the flat ends pot[0] and pot[B-1]
+// caller's edges and centres do not fit together, z/Δc + 1 - c1/Δc), j = floor(v)
+// clamped to [0, B], w = v - floor(v).  Cell j >= 1 is the reference's interpolation cell
+// j-1 between centres c[j-1] and c[j] (src/wakefield.jl:64-78); cells 0 and B hold the flat ends pot[0] and pot[B-1]
 // that the reference's clamp of z to [c1, cB] gives, so out-of-range particles need
 // no clamp of z.  v agrees with the reference's (z - c1)/Δc to ~1e-15 of the bin
 // count, so the kick agrees to that fraction of a bin-to-bin potential step.
@@ -203,10 +203,11 @@ __device__ __forceinline__ double2 ld_table(const double2* p) {
 //   pot[0] - pot[0] = 0, so a hot cell's (left value, step) from the window
 //   is bit-identical to its global entry.  Cells B-1 and B (whose step or
 //   value the bins step sets differently) are never hot.
-// * Histograms: cells w0 .. w0 + h - 1 have their per-block
-//   counters in shared memory (two counts and a sum per cell).  A deposit
-//   outside goes straight to the bunch's accumulators in global memory (u64: counts [B] | cell counts [B+1]
-//   | cell Σw·2^24 [B+1]); h = B + 1 (w0 = 0) where all cells fit.
+// * Histograms: cells w0 .. w0 + h - 1 have their per-block counters in shared
+//   memory (two counts and a sum per cell), and behind them a spare cell.  A deposit
+//   outside goes straight to the bunch's accumulators in global memory (u64: counts
+//   [B] | cell counts [B+1] | cell Σw·2^24 [B+1]) and to the spare cell; h = B + 1
+//   (w0 = 0) where all cells fit.
 struct PassWindow {
   const double* s_win;
   int w0;
